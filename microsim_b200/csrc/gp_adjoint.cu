@@ -3,23 +3,25 @@
 //
 // Forward: the step of gp_adjoint_cell.cuh (the plain step's model) in the
 // working precision T (float: the chosen form; double: the reference
-// adjoint), two kernels per step like the plain form: Delta-phi on the
-// interior plus one ghost ring, then the mu/phi update.  Every
+// adjoint), one kernel per step: a block stages a tile, computes Delta-phi on
+// the tile and one ring in shared memory, then the mu/phi update.  Every
 // `every`-th state is kept (checkpoints).
 //
-// Reverse of one step n (state x_n, adjoint lambda_{n+1} of x_{n+1}):
-//   1. recompute Delta-phi of x_n on the ring;
-//   2. per interior cell: reverse of its mu/phi update -> its own adjoints
-//      and the adjoints of its flux divergences (gdf, gdj);
-//   3. per face: reverse of the diffusion flux and the antitrapping current
-//      (adjoint = difference of the two cells' gdf, gdj), scattered by atomic
-//      adds into phi, mu and Delta-phi of the cells it reads;
-//   4. per ring cell with a nonzero Delta-phi adjoint: reverse of Delta-phi,
-//      scattered into its 3x3 phi stencil and its mu.
+// Reverse of one step n (state x_n, adjoint lambda_{n+1} of x_{n+1}).  The
+// adjoint of a cell's flux divergences depends on its own phi and lambda_mu
+// alone, so the dense part is a gather; only cells with phi gradients near
+// them (listed when the segment is recomputed, a few percent of a grid) scatter:
+//   1. k_rev_cell, every cell: reverse of its mu/phi update and of the
+//      diffusion flux through its four faces (plain stores, one writer);
+//   2. k_rev_jat, the faces of listed cells: reverse of the antitrapping
+//      current, scattered by atomic adds into phi, mu and Delta-phi;
+//   3. k_rev_dphi, the listed cells: reverse of Delta-phi, eight lanes per
+//      cell, scattered into its 3x3 phi stencil and its mu.
 // Ghost reads are boundary index maps, so their adjoints land on the mapped
-// interior cells.  Parameter gradients are reduced per block in FP64.
+// interior cells.  Parameter gradients accumulate in FP64 per block.
 // Backward: segments of `every` steps, last first: the segment is recomputed
-// from its checkpoint into a buffer of `every` states, then reversed.
+// from its checkpoint into a buffer of `every` states (each with its Delta-phi
+// and its list), then reversed.
 // Memory: ceil(N / every) + every states (every = ceil(sqrt(N)) by default).
 
 #include <math.h>
@@ -62,6 +64,19 @@ __device__ __forceinline__ int64_t ix_ring(const Geo& g, int x, int y, int a) {
   return a * g.rplane + (int64_t)(x + 1) * g.rpitch + (y + 1);
 }
 
+// x / d; when d is a power of two (dx = dy = 1 in most inputs) the product with its exact
+// reciprocal, which has the same bits as the quotient.
+__device__ __forceinline__ float pdiv(float x, float d) {
+  const int b = __float_as_int(d), e = (b >> 23) & 0xFF;
+  if ((b & 0x807FFFFF) == 0 && e > 1 && e < 253) return x * __int_as_float((254 - e) << 23);
+  return x / d;
+}
+__device__ __forceinline__ double pdiv(double x, double d) {
+  const long long b = __double_as_longlong(d), e = (b >> 52) & 0x7FF;
+  if ((b & 0x800FFFFFFFFFFFFFLL) == 0 && e > 1 && e < 2045) return x * __longlong_as_double((2046LL - e) << 52);
+  return x / d;
+}
+
 template <typename T>
 __device__ __forceinline__ void load_P(const T* st, const Geo& g, int x, int y, T (&P)[3][3][2]) {
 #pragma unroll
@@ -72,6 +87,23 @@ __device__ __forceinline__ void load_P(const T* st, const Geo& g, int x, int y, 
       for (int a = 0; a < 2; a++) P[i][j][a] = ld_phi(st, g, x + i - 1, y + j - 1, a);
 }
 
+// The 3x3 block holds one value in [0, 1] per phase: every phi gradient is 0, no phase is active,
+// Delta-phi is 0 whatever mu is, and no antitrapping current crosses the cell's faces.
+template <typename T>
+__device__ __forceinline__ bool flat_P(const T (&P)[3][3][2]) {
+  bool f = true;
+#pragma unroll
+  for (int a = 0; a < 2; a++) {
+    const T c = P[1][1][a];
+    f = f && c >= (T)0 && c <= (T)1;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) f = f && P[i][j][a] == c;
+  }
+  return f;
+}
+
 // Face k of interior cell (x, y): 0 = x+, 1 = x-, 2 = y+, 3 = y-; M[5], D[5]:
 // mu and Delta-phi (phase 0) of the cell and its x-, x+, y-, y+ neighbours.
 template <typename T>
@@ -79,9 +111,9 @@ __device__ __forceinline__ Face<T> cell_face(const AM<T>& m, const Geo& g, int y
                                              const T (&M)[5], const T (&D)[5], int k) {
   Face<T> f;
   const T ty = (T)2 * m.dy;
-  auto cy = [&](int i, int a) { return (P[i][2][a] - P[i][0][a]) / ty; };
+  auto cy = [&](int i, int a) { return pdiv(P[i][2][a] - P[i][0][a], ty); };
   auto cx = [&](int j, int a) {
-    return (T)0.5 * ((P[2][j][a] - P[1][j][a]) / m.dx + (P[1][j][a] - P[0][j][a]) / m.dx);
+    return (T)0.5 * (pdiv(P[2][j][a] - P[1][j][a], m.dx) + pdiv(P[1][j][a] - P[0][j][a], m.dx));
   };
   for (int a = 0; a < 2; a++) {
     if (k == 0) {
@@ -104,48 +136,134 @@ __device__ __forceinline__ Face<T> cell_face(const AM<T>& m, const Geo& g, int y
   return f;
 }
 
+// the diffusion flux of face k alone (fface on the cell's operands, without the antitrapping ones)
 template <typename T>
-__device__ __forceinline__ void load_MD(const T* st, const T* ring, const Geo& g, int x, int y, T (&M)[5],
-                                        T (&D)[5], T (&Dc)[2]) {
-  const int dx[5] = {0, -1, 1, 0, 0}, dy[5] = {0, 0, 0, -1, 1};
-#pragma unroll
-  for (int s = 0; s < 5; s++) {
-    M[s] = ld_mu(st, g, x + dx[s], y + dy[s]);
-    D[s] = ring[ix_ring(g, x + dx[s], y + dy[s], 0)];
-  }
-  Dc[0] = D[0];
-  Dc[1] = ring[ix_ring(g, x, y, 1)];
+__device__ __forceinline__ T cell_flux(const AM<T>& m, T pc0, T pc1, T pn0, T pn1, T muc, T mun, T h) {
+  const T Dc = m.Ds * m.cmu[0] * pc0 + m.Dl * m.cmu[1] * pc1;
+  const T Dn = m.Ds * m.cmu[0] * pn0 + m.Dl * m.cmu[1] * pn1;
+  return (Dn + Dc) * (T)0.5 * pdiv(mun - muc, h);
+}
+
+// Block tile of the dense kernels: a cell per thread, y fastest (a warp per tile row).
+constexpr int TX = 8, TY = 32, NT = TX * TY;
+constexpr int X1 = TX + 2, Y1 = TY + 2, X2 = TX + 4, Y2 = TY + 4;
+
+__device__ __forceinline__ void tile_origin(const Geo& g, int& x0, int& y0) {
+  const int nty = (g.my + TY - 1) / TY;
+  x0 = (int)(blockIdx.x / nty) * TX;
+  y0 = (int)(blockIdx.x % nty) * TY;
+}
+
+// Ring position (x, y) = (x0 - 1 + i, y0 - 1 + j) of the tile belongs to it: one of its cells, or a
+// cell of the grid's ghost ring beside it.
+__device__ __forceinline__ bool owns_ring(const Geo& g, int x, int y, int i, int j) {
+  return x <= g.mx && y <= g.my && ((i >= 1 && i <= TX) || x == -1 || (i == TX + 1 && x == g.mx)) &&
+         ((j >= 1 && j <= TY) || y == -1 || (j == TY + 1 && y == g.my));
 }
 
 // ------------------------------------------------------------------ forward
 
+// One step st -> out (out == nullptr: Delta-phi and the list only).  With ring: Delta-phi is also
+// written there (interior and ghost ring), and the ring cells whose phi block is not flat are
+// appended to list (as ring offsets), their number in *cnt.
+// Bound by latency: a 512^2 FP32 step moves 6 MB within L2, and a block's chain is stage -> flags ->
+// Delta-phi -> update.  Cells with a flat block (all but a few percent) skip the phase-field
+// arithmetic; the others are compacted first, so that a warp of the tile does not wait for the few
+// of its lanes that hold an interface.
 template <typename T>
-__global__ void __launch_bounds__(256) k_fwd_dphi(const AM<T> m, Geo g, const T* __restrict__ st,
-                                                  T* __restrict__ ring) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x - 1, x = blockIdx.y - 1;
-  if (y > g.my) return;
-  T P[3][3][2], dp[2];
-  load_P(st, g, x, y, P);
-  dphi_fwd(m, P, ld_mu(st, g, x, y), dp);
-  ring[ix_ring(g, x, y, 0)] = dp[0];
-  ring[ix_ring(g, x, y, 1)] = dp[1];
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_fwd_update(const AM<T> m, Geo g, const T* __restrict__ st,
-                                                    const T* __restrict__ ring, T* __restrict__ out) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x, x = blockIdx.y;
-  if (y >= g.my) return;
-  T P[3][3][2], M[5], D[5], Dc[2], F[4], J[4];
-  load_P(st, g, x, y, P);
-  load_MD(st, ring, g, x, y, M, D, Dc);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const Face<T> f = cell_face(m, g, y, P, M, D, k);
-    F[k] = fface(m, f);
-    J[k] = jface(m, f);
+__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+                                            T* __restrict__ out, T* __restrict__ ring, int* __restrict__ list,
+                                            int* __restrict__ cnt) {
+  __shared__ T sp[2][X2][Y2], su[X1][Y1], sd[2][X1][Y1];
+  __shared__ int s_list[X1 * Y1], s_own[X1 * Y1], s_n, s_m, s_base;
+  int x0, y0;
+  tile_origin(g, x0, y0);
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) s_n = s_m = 0;
+  for (int e = tid; e < X2 * Y2; e += NT) {
+    const int i = e / Y2, j = e % Y2;
+    const int64_t o = (int64_t)gp_map_any(x0 - 2 + i, g.mx, g.bc.phi_x) * g.pitch + gp_map_any(y0 - 2 + j, g.my, g.bc.phi_y);
+    sp[0][i][j] = st[o];
+    sp[1][i][j] = st[g.plane + o];
   }
+  for (int e = tid; e < X1 * Y1; e += NT) {
+    const int i = e / Y1, j = e % Y1;
+    su[i][j] = st[2 * g.plane + (int64_t)gp_map_any(x0 - 1 + i, g.mx, g.bc.mu_x) * g.pitch +
+                  gp_map_any(y0 - 1 + j, g.my, g.bc.mu_y)];
+  }
+  __syncthreads();
+  auto block3 = [&](int i, int j, T (&P)[3][3][2]) {  // around ring position (i, j)
+#pragma unroll
+    for (int di = 0; di < 3; di++)
+#pragma unroll
+      for (int dj = 0; dj < 3; dj++)
+#pragma unroll
+        for (int a = 0; a < 2; a++) P[di][dj][a] = sp[a][i + di][j + dj];
+  };
+  for (int e0 = 0; e0 < X1 * Y1; e0 += NT) {
+    const int e = e0 + tid;
+    bool act = false, own = false;
+    if (e < X1 * Y1) {
+      const int i = e / Y1, j = e % Y1, x = x0 - 1 + i, y = y0 - 1 + j;
+      sd[0][i][j] = sd[1][i][j] = (T)0;
+      if (x <= g.mx && y <= g.my) {
+        T P[3][3][2];
+        block3(i, j, P);
+        act = !flat_P(P);
+        own = act && ring && owns_ring(g, x, y, i, j);
+      }
+    }
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned bal = __ballot_sync(0xffffffffu, act), balo = __ballot_sync(0xffffffffu, own);
+    int base = 0, baseo = 0;
+    if (lane == 0 && bal) base = atomicAdd(&s_n, __popc(bal));
+    if (lane == 0 && balo) baseo = atomicAdd(&s_m, __popc(balo));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    baseo = __shfl_sync(0xffffffffu, baseo, 0);
+    if (act) s_list[base + __popc(bal & below)] = e;
+    if (own) s_own[baseo + __popc(balo & below)] = e;
+  }
+  __syncthreads();
+  if (ring && tid == 0 && s_m) s_base = atomicAdd(cnt, s_m);
+  for (int q = tid; q < s_n; q += NT) {
+    const int e = s_list[q], i = e / Y1, j = e % Y1;
+    T P[3][3][2], dp[2];
+    block3(i, j, P);
+    dphi_fwd(m, P, su[i][j], dp);
+    sd[0][i][j] = dp[0];
+    sd[1][i][j] = dp[1];
+  }
+  __syncthreads();
+  if (ring) {
+    for (int q = tid; q < s_m; q += NT) {
+      const int e = s_own[q];
+      list[s_base + q] = (int)ix_ring(g, x0 - 1 + e / Y1, y0 - 1 + e % Y1, 0);
+    }
+    for (int e = tid; e < X1 * Y1; e += NT) {
+      const int i = e / Y1, j = e % Y1, x = x0 - 1 + i, y = y0 - 1 + j;
+      if (!owns_ring(g, x, y, i, j)) continue;
+      ring[ix_ring(g, x, y, 0)] = sd[0][i][j];
+      ring[ix_ring(g, x, y, 1)] = sd[1][i][j];
+    }
+  }
+  const int i = tid / TY, j = tid % TY, x = x0 + i, y = y0 + j;
+  if (!out || x >= g.mx || y >= g.my) return;
+  T P[3][3][2], F[4], J[4];
+  block3(i + 1, j + 1, P);
+  const T M[5] = {su[i + 1][j + 1], su[i][j + 1], su[i + 2][j + 1], su[i + 1][j], su[i + 1][j + 2]};
   const T ph[2] = {P[1][1][0], P[1][1][1]};
+  F[0] = cell_flux(m, ph[0], ph[1], P[2][1][0], P[2][1][1], M[0], M[2], m.dx);
+  F[1] = cell_flux(m, P[0][1][0], P[0][1][1], ph[0], ph[1], M[1], M[0], m.dx);
+  F[2] = cell_flux(m, ph[0], ph[1], P[1][2][0], P[1][2][1], M[0], M[4], m.dy);
+  F[3] = cell_flux(m, P[1][0][0], P[1][0][1], ph[0], ph[1], M[3], M[0], m.dy);
+  const T Dc[2] = {sd[0][i + 1][j + 1], sd[1][i + 1][j + 1]};
+#pragma unroll
+  for (int k = 0; k < 4; k++) J[k] = (T)0;
+  if (!flat_P(P)) {
+    const T D[5] = {Dc[0], sd[0][i][j + 1], sd[0][i + 2][j + 1], sd[0][i + 1][j], sd[0][i + 1][j + 2]};
+#pragma unroll
+    for (int k = 0; k < 4; k++) J[k] = jface(m, cell_face(m, g, y, P, M, D, k));
+  }
   const int64_t o = (int64_t)x * g.pitch + y;
   out[2 * g.plane + o] = mu_new(m, ph, M[0], Dc, F, J);
   out[o] = ph[0] + Dc[0];
@@ -154,99 +272,198 @@ __global__ void __launch_bounds__(256) k_fwd_update(const AM<T> m, Geo g, const 
 
 // ------------------------------------------------------------------ reverse
 
-// block sum of the four parameter adjoints into grad (FP64)
-__device__ __forceinline__ void reduce_params(double (&lp)[NPARAM], double* grad) {
-  __shared__ double s[NPARAM][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// Adjoint of a cell's divflux (gdf) over dt: d mu_new / d c times lambda_mu (mu_new_rev); that of
+// divjat is its negative.
+template <typename T>
+__device__ __forceinline__ T cell_ldc(const AM<T>& m, T p0, T p1, T lmn) {
+  if (p0 == (T)1) return (T)2 * m.A[0] * lmn;
+  if (p1 == (T)1) return (T)2 * m.A[1] * lmn;
+  return lmn / (m.cmu[0] * hfun(p0) + m.cmu[1] * hfun(p1));
+}
+
+// Sum of v over the block into *slot (its only writer; launches that share it are ordered).
+__device__ __forceinline__ void block_add(double v, double* slot) {
+  __shared__ double s[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-  for (int p = 0; p < NPARAM; p++) {
-    double v = lp[p];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) s[p][w] = v;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  __syncthreads();  // s of a previous call has been read
+  if (lane == 0) s[w] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int i = 0; i < nw; i++) t += s[i];
+    if (t != 0.0) *slot += t;
+  }
+}
+
+// 1. reverse of the cell update and of the diffusion fluxes: every contribution that reaches a
+// cell's own phi and mu through its update and its four faces, gathered (a boundary cell also takes
+// the ghost cell that maps to it).  Writes lam_out and the cell's Delta-phi adjoint (ldphi; 0 on the
+// ghost ring).  part[block] accumulates the D_liquid gradient, each face counted by its lower cell.
+// Bound by its loads: 6 planes in, 5 out, with one synchronisation.
+template <typename T>
+__global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+                                                 const T* __restrict__ ring, const T* __restrict__ lam_in,
+                                                 T* __restrict__ lam_out, T* __restrict__ ldphi,
+                                                 double* __restrict__ part) {
+  __shared__ T sp[2][X1][Y1], su[X1][Y1], sg[X1][Y1];
+  int x0, y0;
+  tile_origin(g, x0, y0);
+  const int tid = threadIdx.x;
+  const T* const lmu_in = lam_in + 2 * g.plane;
+  for (int e = tid; e < X1 * Y1; e += NT) {
+    const int i = e / Y1, j = e % Y1, x = x0 - 1 + i, y = y0 - 1 + j;
+    const int64_t o = (int64_t)gp_map_any(x, g.mx, g.bc.phi_x) * g.pitch + gp_map_any(y, g.my, g.bc.phi_y);
+    const T p0 = st[o], p1 = st[g.plane + o];
+    sp[0][i][j] = p0;
+    sp[1][i][j] = p1;
+    su[i][j] = st[2 * g.plane + (int64_t)gp_map_any(x, g.mx, g.bc.mu_x) * g.pitch + gp_map_any(y, g.my, g.bc.mu_y)];
+    const bool in = x >= 0 && x < g.mx && y >= 0 && y < g.my;
+    sg[i][j] = in ? cell_ldc(m, p0, p1, lmu_in[(int64_t)x * g.pitch + y]) * m.dt : (T)0;
+    if (!in && owns_ring(g, x, y, i, j)) ldphi[ix_ring(g, x, y, 0)] = ldphi[ix_ring(g, x, y, 1)] = (T)0;
   }
   __syncthreads();
-  if (threadIdx.x < NPARAM) {
-    double v = 0.0;
-    for (int i = 0; i < nw; i++) v += s[threadIdx.x][i];
-    if (v != 0.0) atomicAdd(grad + threadIdx.x, v);
-  }
-}
-
-// 2. reverse of the cell update: lam_out (phi, mu of the cell) is written,
-// ldphi (ring, zeroed before) receives the cell's own Delta-phi adjoint
-template <typename T>
-__global__ void __launch_bounds__(256) k_rev_cell(const AM<T> m, Geo g, const T* __restrict__ st,
-                                                  const T* __restrict__ ring, const T* __restrict__ lam_in,
-                                                  T* __restrict__ lam_out, T* __restrict__ ldphi,
-                                                  T* __restrict__ gdf, T* __restrict__ gdj) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x, x = blockIdx.y;
-  if (y >= g.my) return;
-  const int64_t o = (int64_t)x * g.pitch + y;
-  T P[3][3][2], M[5], D[5], Dc[2], F[4], J[4];
-  load_P(st, g, x, y, P);
-  load_MD(st, ring, g, x, y, M, D, Dc);
+  double dl = 0.0;
+  const int i = tid / TY + 1, j = tid % TY + 1, x = x0 + i - 1, y = y0 + j - 1;
+  if (x < g.mx && y < g.my) {
+    const int64_t o = (int64_t)x * g.pitch + y;
+    const T ph[2] = {sp[0][i][j], sp[1][i][j]};
+    const T M[5] = {su[i][j], su[i - 1][j], su[i + 1][j], su[i][j - 1], su[i][j + 1]};
+    const T lp0 = lam_in[o], lp1 = lam_in[g.plane + o], lmn = lmu_in[o];
+    T lph[2] = {lp0, lp1}, lmu = (T)0, ldp[2] = {lp0, lp1};
+    if (ph[0] == (T)1 || ph[1] == (T)1) {
+      const int b = ph[0] == (T)1 ? 0 : 1;
+      lmu = (T)2 * m.A[b] * lmn * m.cmu[b];
+    } else {
+      T P[3][3][2], F[4], J[4], df, dj;
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const Face<T> f = cell_face(m, g, y, P, M, D, k);
-    F[k] = fface(m, f);
-    J[k] = jface(m, f);
+      for (int di = 0; di < 3; di++)
+#pragma unroll
+        for (int dj2 = 0; dj2 < 3; dj2++)
+#pragma unroll
+          for (int a = 0; a < 2; a++) P[di][dj2][a] = sp[a][i - 1 + di][j - 1 + dj2];
+      T D[5];
+      const T* r = ring + ix_ring(g, x, y, 0);
+      D[0] = r[0];
+      D[1] = r[-g.rpitch];
+      D[2] = r[g.rpitch];
+      D[3] = r[-1];
+      D[4] = r[1];
+      const T Dc[2] = {D[0], r[g.rplane]};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const Face<T> f = cell_face(m, g, y, P, M, D, k);
+        F[k] = fface(m, f);
+        J[k] = jface(m, f);
+      }
+      mu_new_rev(m, ph, M[0], Dc, F, J, lmn, lph, lmu, ldp, df, dj);
+    }
+    ldphi[ix_ring(g, x, y, 0)] = ldp[0];
+    ldphi[ix_ring(g, x, y, 1)] = ldp[1];
+    // the diffusion fluxes: s = +1 where the cell is the face's lower one
+    const T k0 = m.Ds * m.cmu[0], k1 = m.Dl * m.cmu[1];
+    const T Dme = k0 * ph[0] + k1 * ph[1];
+    auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, T h, bool to_phi, bool to_mu) {
+      const T lF = pdiv(g_lo - g_hi, h), gr = pdiv(mu_hi - mu_lo, h), lD = (T)0.5 * gr * lF;
+      if (to_phi) {
+        lph[0] += lD * k0;
+        lph[1] += lD * k1;
+      }
+      if (to_mu) lmu -= s * pdiv(Dsum * (T)0.5 * lF, h);
+      return lD;
+    };
+    const T gme = sg[i][j];
+    auto nb = [&](int a, int ii, int jj) { return sp[a][ii][jj]; };
+    auto Dnb = [&](int ii, int jj) { return k0 * nb(0, ii, jj) + k1 * nb(1, ii, jj); };
+    const T a0 = gather((T)1, gme, sg[i + 1][j], M[0], M[2], Dnb(i + 1, j) + Dme, m.dx, true, true);
+    const T a1 = gather((T)-1, sg[i - 1][j], gme, M[1], M[0], Dme + Dnb(i - 1, j), m.dx, true, true);
+    const T a2 = gather((T)1, gme, sg[i][j + 1], M[0], M[4], Dnb(i, j + 1) + Dme, m.dy, true, true);
+    const T a3 = gather((T)-1, sg[i][j - 1], gme, M[3], M[0], Dme + Dnb(i, j - 1), m.dy, true, true);
+    dl += (double)(a0 * m.cmu[1] * (ph[1] + nb(1, i + 1, j))) + (double)(a2 * m.cmu[1] * (ph[1] + nb(1, i, j + 1)));
+    if (x == 0) dl += (double)(a1 * m.cmu[1] * (nb(1, i - 1, j) + ph[1]));
+    if (y == 0) dl += (double)(a3 * m.cmu[1] * (nb(1, i, j - 1) + ph[1]));
+    // the ghost cell (ghost row -1 or M, against the grid's first or last row `e`) that maps to this one
+    auto ghost = [&](bool along_x, bool low) {
+      const int Mg = along_x ? g.mx : g.my, v = low ? -1 : Mg, e = low ? 0 : Mg - 1, own = along_x ? x : y;
+      const int mp = gp_map(v, Mg, along_x ? g.bc.phi_x : g.bc.phi_y), mm = gp_map(v, Mg, along_x ? g.bc.mu_x : g.bc.mu_y);
+      if (mp != own && mm != own) return;
+      const int ex = along_x ? e : x, ey = along_x ? y : e, vx = along_x ? v : x, vy = along_x ? y : v;
+      const T e0 = ld_phi(st, g, ex, ey, 0), e1 = ld_phi(st, g, ex, ey, 1);
+      const T v0 = ld_phi(st, g, vx, vy, 0), v1 = ld_phi(st, g, vx, vy, 1);
+      const T ge = cell_ldc(m, e0, e1, lmu_in[(int64_t)ex * g.pitch + ey]) * m.dt;
+      const T ue = st[2 * g.plane + (int64_t)ex * g.pitch + ey], uv = ld_mu(st, g, vx, vy);
+      const T Ds2 = (k0 * v0 + k1 * v1) + (k0 * e0 + k1 * e1), h = along_x ? m.dx : m.dy;
+      if (low) gather((T)1, (T)0, ge, uv, ue, Ds2, h, mp == own, mm == own);
+      else gather((T)-1, ge, (T)0, ue, uv, Ds2, h, mp == own, mm == own);
+    };
+    if (x <= 2 || x >= g.mx - 3) {
+      ghost(true, true);
+      ghost(true, false);
+    }
+    if (y <= 2 || y >= g.my - 3) {
+      ghost(false, true);
+      ghost(false, false);
+    }
+    lam_out[o] = lph[0];
+    lam_out[g.plane + o] = lph[1];
+    lam_out[2 * g.plane + o] = lmu;
   }
-  const T ph[2] = {P[1][1][0], P[1][1][1]};
-  const T lp0 = lam_in[o], lp1 = lam_in[g.plane + o], lmn = lam_in[2 * g.plane + o];
-  T lph[2] = {lp0, lp1}, lmu = (T)0, ldp[2] = {lp0, lp1}, df = (T)0, dj = (T)0;
-  mu_new_rev(m, ph, M[0], Dc, F, J, lmn, lph, lmu, ldp, df, dj);
-  lam_out[o] = lph[0];
-  lam_out[g.plane + o] = lph[1];
-  lam_out[2 * g.plane + o] = lmu;
-  ldphi[ix_ring(g, x, y, 0)] += ldp[0];
-  ldphi[ix_ring(g, x, y, 1)] += ldp[1];
-  gdf[o] = df;
-  gdj[o] = dj;
+  block_add(dl, part + blockIdx.x);
 }
 
-// Scatter of one adjoint contribution; a zero one is skipped (most faces of a bulk region carry no
-// antitrapping current, so most of their tangential and Delta-phi adjoints are zero).  The float
-// sums are order-dependent anyway (atomics); skipping a +-0 addend changes at most a zero's sign.
+// Scatter of one adjoint contribution; a zero one is skipped.
 template <typename T>
 __device__ __forceinline__ void add_nz(T* p, T v) {
   if (v != (T)0) atomicAdd(p, v);
 }
 
-// 3. reverse of the face fluxes; thread = one face (lower cell (x, y)):
-// x-faces for x in [-1, mx-1], y in [0, my-1]; y-faces for x in [0, mx-1], y in [-1, my-1]
+// 2. reverse of the antitrapping currents: a thread per face of a listed ring cell (k as in
+// cell_face).  A face between two listed cells belongs to its lower one; one whose lower cell is flat
+// to its upper one.  Faces between two flat cells carry no current and no derivative.
+// Bound by latency (a few thousand threads with one dependent chain of square roots and divisions).
 template <typename T>
-__global__ void __launch_bounds__(256) k_rev_face(const AM<T> m, Geo g, const T* __restrict__ st,
-                                                  const T* __restrict__ ring, const T* __restrict__ gdf,
-                                                  const T* __restrict__ gdj, T* __restrict__ lam_out,
-                                                  T* __restrict__ ldphi, double* __restrict__ grad) {
-  double lpd[NPARAM] = {0, 0, 0, 0};
-  const int dir = blockIdx.z;  // 0: x-faces, 1: y-faces
-  const int x = blockIdx.y - (dir == 0 ? 1 : 0);
-  const int y = blockIdx.x * blockDim.x + threadIdx.x - (dir == 1 ? 1 : 0);
-  const bool valid = dir == 0 ? (y < g.my && x <= g.mx - 1) : (y <= g.my - 1 && x < g.mx);
-  if (valid) {
+__global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+                                                 const T* __restrict__ ring, const T* __restrict__ lam_in,
+                                                 T* __restrict__ lam_out, T* __restrict__ ldphi,
+                                                 const int* __restrict__ list, const int* __restrict__ cnt,
+                                                 double* __restrict__ part) {
+  double dl = 0.0;
+  const int n = 4 * *cnt;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int o = list[q >> 2], k = q & 3, dir = k >> 1;
+    int x = o / g.rpitch - 1, y = o % g.rpitch - 1;  // the listed cell, then the face's lower cell
+    if (k & 1) {
+      if (dir == 0) x--;
+      else y--;
+    }
+    const bool valid = dir == 0 ? (x >= -1 && x < g.mx && y >= 0 && y < g.my) : (y >= -1 && y < g.my && x >= 0 && x < g.mx);
+    if (!valid) continue;
+    if (k & 1) {
+      T P[3][3][2];
+      load_P(st, g, x, y, P);
+      if (!flat_P(P)) continue;
+    }
     const int xn = dir == 0 ? x + 1 : x, yn = dir == 0 ? y : y + 1;
-    const bool cin = x >= 0 && y >= 0, nin = xn < g.mx && yn < g.my;
     const T h = dir == 0 ? m.dx : m.dy;
-    const T lF = ((cin ? gdf[(int64_t)x * g.pitch + y] : (T)0) - (nin ? gdf[(int64_t)xn * g.pitch + yn] : (T)0)) / h;
-    const T lJ = ((cin ? gdj[(int64_t)x * g.pitch + y] : (T)0) - (nin ? gdj[(int64_t)xn * g.pitch + yn] : (T)0)) *
-                 m.jscale / h;
-    // the face's operands, as the cells build them
     Face<T> f;
     const T ty = (T)2 * m.dy;
     for (int a = 0; a < 2; a++) {
       f.pc[a] = ld_phi(st, g, x, y, a);
       f.pn[a] = ld_phi(st, g, xn, yn, a);
       if (dir == 0) {
-        f.tc[a] = (ld_phi(st, g, x, y + 1, a) - ld_phi(st, g, x, y - 1, a)) / ty;
-        f.tn[a] = (ld_phi(st, g, xn, y + 1, a) - ld_phi(st, g, xn, y - 1, a)) / ty;
+        f.tc[a] = pdiv(ld_phi(st, g, x, y + 1, a) - ld_phi(st, g, x, y - 1, a), ty);
+        f.tn[a] = pdiv(ld_phi(st, g, xn, y + 1, a) - ld_phi(st, g, xn, y - 1, a), ty);
       } else {
-        const T c0 = ld_phi(st, g, x, y, a), n0 = ld_phi(st, g, x, yn, a);
-        f.tc[a] = (T)0.5 * ((ld_phi(st, g, x + 1, y, a) - c0) / m.dx + (c0 - ld_phi(st, g, x - 1, y, a)) / m.dx);
-        f.tn[a] = (T)0.5 * ((ld_phi(st, g, x + 1, yn, a) - n0) / m.dx + (n0 - ld_phi(st, g, x - 1, yn, a)) / m.dx);
+        f.tc[a] = (T)0.5 * (pdiv(ld_phi(st, g, x + 1, y, a) - f.pc[a], m.dx) + pdiv(f.pc[a] - ld_phi(st, g, x - 1, y, a), m.dx));
+        f.tn[a] = (T)0.5 * (pdiv(ld_phi(st, g, x + 1, yn, a) - f.pn[a], m.dx) + pdiv(f.pn[a] - ld_phi(st, g, x - 1, yn, a), m.dx));
       }
     }
+    T lc = (T)0, ln = (T)0;  // the two cells' divjat adjoints
+    if (x >= 0 && y >= 0) lc = -cell_ldc(m, f.pc[0], f.pc[1], lam_in[2 * g.plane + (int64_t)x * g.pitch + y]);
+    if (xn < g.mx && yn < g.my) ln = -cell_ldc(m, f.pn[0], f.pn[1], lam_in[2 * g.plane + (int64_t)xn * g.pitch + yn]);
+    const T lJ = pdiv((lc - ln) * m.jscale, h);
+    if (lJ == (T)0) continue;
     f.muc = ld_mu(st, g, x, y);
     f.mun = ld_mu(st, g, xn, yn);
     f.dpc = ring[ix_ring(g, x, y, 0)];
@@ -255,19 +472,19 @@ __global__ void __launch_bounds__(256) k_rev_face(const AM<T> m, Geo g, const T*
     f.skip = dir == 1 && (y + 3 == g.my - 2);
     FaceAdj<T> L = {};
     T lp[NPARAM] = {(T)0, (T)0, (T)0, (T)0};
-    if (lF != (T)0) fface_rev(m, f, lF, L, lp);
-    if (lJ != (T)0) jface_rev(m, f, lJ, L, lp);
-    for (int p = 0; p < NPARAM; p++) lpd[p] = (double)lp[p];
+    jface_rev(m, f, lJ, L, lp);
+    dl += (double)lp[P_DLIQ];
     for (int a = 0; a < 2; a++) {
       add_nz(lam_out + ix_phi(g, x, y, a), L.pc[a]);
       add_nz(lam_out + ix_phi(g, xn, yn, a), L.pn[a]);
       if (dir == 0) {
-        add_nz(lam_out + ix_phi(g, x, y + 1, a), L.tc[a] / ty);
-        add_nz(lam_out + ix_phi(g, x, y - 1, a), -L.tc[a] / ty);
-        add_nz(lam_out + ix_phi(g, xn, y + 1, a), L.tn[a] / ty);
-        add_nz(lam_out + ix_phi(g, xn, y - 1, a), -L.tn[a] / ty);
+        const T hc = pdiv(L.tc[a], ty), hn = pdiv(L.tn[a], ty);
+        add_nz(lam_out + ix_phi(g, x, y + 1, a), hc);
+        add_nz(lam_out + ix_phi(g, x, y - 1, a), -hc);
+        add_nz(lam_out + ix_phi(g, xn, y + 1, a), hn);
+        add_nz(lam_out + ix_phi(g, xn, y - 1, a), -hn);
       } else {
-        const T hc = (T)0.5 * L.tc[a] / m.dx, hn = (T)0.5 * L.tn[a] / m.dx;
+        const T hc = pdiv((T)0.5 * L.tc[a], m.dx), hn = pdiv((T)0.5 * L.tn[a], m.dx);
         add_nz(lam_out + ix_phi(g, x + 1, y, a), hc);
         add_nz(lam_out + ix_phi(g, x - 1, y, a), -hc);
         add_nz(lam_out + ix_phi(g, x + 1, yn, a), hn);
@@ -279,31 +496,221 @@ __global__ void __launch_bounds__(256) k_rev_face(const AM<T> m, Geo g, const T*
     add_nz(ldphi + ix_ring(g, x, y, 0), L.dpc);
     add_nz(ldphi + ix_ring(g, xn, yn, 0), L.dpn);
   }
-  reduce_params(lpd, grad);
+  block_add(dl, part + blockIdx.x);
 }
 
-// 4. reverse of Delta-phi on the ring
+// 3. reverse of Delta-phi (dphi_rev of gp_adjoint_cell.cuh) on the listed ring cells, eight lanes
+// per cell: lane a * 4 + k reverses face k of phase a's gradient-energy term, the terms at the cell's
+// centre and the projection are evaluated by all eight, and lanes 0 and 1 of each phase scatter the
+// centre's contributions with their faces'.  One thread per cell is a chain of twenty a_c(q)
+// evaluations with their reverses on a few thousand threads, far too few to hide it.
 template <typename T>
-__global__ void __launch_bounds__(256) k_rev_dphi(const AM<T> m, Geo g, const T* __restrict__ st,
+__global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
                                                   const T* __restrict__ ldphi, T* __restrict__ lam_out,
-                                                  double* __restrict__ grad) {
-  double lpd[NPARAM] = {0, 0, 0, 0};
-  const int y = blockIdx.x * blockDim.x + threadIdx.x - 1, x = blockIdx.y - 1;
-  if (y <= g.my) {
-    const T ld[2] = {ldphi[ix_ring(g, x, y, 0)], ldphi[ix_ring(g, x, y, 1)]};
-    if (ld[0] != (T)0 || ld[1] != (T)0) {
-      T P[3][3][2], LP[3][3][2] = {}, lmu = (T)0, lp[NPARAM] = {(T)0, (T)0, (T)0, (T)0};
-      load_P(st, g, x, y, P);
-      dphi_rev(m, P, ld_mu(st, g, x, y), ld, LP, lmu, lp);
-      for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++)
-          for (int a = 0; a < 2; a++)
-            if (LP[i][j][a] != (T)0) atomicAdd(lam_out + ix_phi(g, x + i - 1, y + j - 1, a), LP[i][j][a]);
-      if (lmu != (T)0) atomicAdd(lam_out + ix_mu(g, x, y), lmu);
-      for (int p = 0; p < NPARAM; p++) lpd[p] = (double)lp[p];
+                                                  const int* __restrict__ list, const int* __restrict__ cnt,
+                                                  double* __restrict__ part) {
+  constexpr unsigned ALL = 0xffffffffu;
+  double acc[3] = {0.0, 0.0, 0.0};  // mobility, delta, gamma
+  const int lane = threadIdx.x & 31, sub = lane & 7, a = sub >> 2, k = sub & 3, dir = k >> 1;
+  const int n = *cnt, warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const T ty = (T)2 * m.dy, h = dir ? m.dy : m.dx;
+  for (int base = 4 * warp; base < n; base += 4 * warps) {
+    const int q = base + (lane >> 3);
+    const int o = list[q < n ? q : n - 1], x = o / g.rpitch - 1, y = o % g.rpitch - 1;
+    const T ldp[2] = {q < n ? ldphi[o] : (T)0, q < n ? ldphi[o + g.rplane] : (T)0};
+    bool on = ldp[0] != (T)0 || ldp[1] != (T)0;
+    if (!__any_sync(ALL, on)) continue;
+    T P[3][3][2];
+    load_P(st, g, x, y, P);
+    const T ph[2] = {P[1][1][0], P[1][1][1]}, mu = ld_mu(st, g, x, y);
+    // the record at the centre and the active phases
+    T cx[2], cy[2];
+    bool act[2];
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      const T gx = pdiv(P[2][1][p] - P[1][1][p], m.dx), bgx = pdiv(P[1][1][p] - P[0][1][p], m.dx);
+      const T gy = pdiv(P[1][2][p] - P[1][1][p], m.dy), lgy = pdiv(P[1][1][p] - P[1][0][p], m.dy);
+      cx[p] = (T)0.5 * (gx + bgx);
+      cy[p] = pdiv(P[1][2][p] - P[1][0][p], ty);
+      act[p] = fabs(pdiv(gx - bgx, m.dx) + pdiv(gy - lgy, m.dy)) > (T)0;
     }
+    on = on && (act[0] || act[1]);  // no active phase: Delta-phi is 0 whatever the inputs
+    // the lane's face: f[n][t] along its normal (n = 0 lower, 1 upper cell) and tangent (t = 0 .. 2)
+    T s[2], gn[2], tg[2];
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      T f[2][3];
+#pragma unroll
+      for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+        for (int t = 0; t < 3; t++)
+          f[nn][t] = dir == 0 ? (k == 0 ? P[1 + nn][t][p] : P[nn][t][p]) : (k == 2 ? P[t][1 + nn][p] : P[t][nn][p]);
+      s[p] = (T)0.5 * (f[1][1] + f[0][1]);
+      gn[p] = pdiv(f[1][1] - f[0][1], h);
+      T tt[2];
+#pragma unroll
+      for (int nn = 0; nn < 2; nn++)
+        tt[nn] = dir == 0 ? pdiv(f[nn][2] - f[nn][0], ty)
+                          : (T)0.5 * (pdiv(f[nn][2] - f[nn][1], m.dx) + pdiv(f[nn][1] - f[nn][0], m.dx));
+      tg[p] = tt[0] + tt[1];
+    }
+    const T sa = a ? s[1] : s[0], sb = a ? s[0] : s[1], ga = a ? gn[1] : gn[0], gb = a ? gn[0] : gn[1];
+    const T ta = a ? tg[1] : tg[0], tb = a ? tg[0] : tg[1];
+    const T pa = a ? ph[1] : ph[0], pb = a ? ph[0] : ph[1], cxa = a ? cx[1] : cx[0], cxb = a ? cx[0] : cx[1];
+    const T cya = a ? cy[1] : cy[0], cyb = a ? cy[0] : cy[1];
+    const bool act_a = a ? act[1] : act[0];
+    const T Qn = sa * gb - sb * ga, Qt = (T)0.5 * (sa * tb - sb * ta);
+    const T Qx = dir ? Qt : Qn, Qy = dir ? Qn : Qt;
+    const T sg = (k & 1) ? (T)-1 : (T)1;
+    T sum4 = sg * pdiv(face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir), h);
+    sum4 += __shfl_xor_sync(ALL, sum4, 1);
+    sum4 += __shfl_xor_sync(ALL, sum4, 2);
+    // the centre term (tterm)
+    const T v0 = pa * cxb - pb * cxa, v1 = pa * cyb - pb * cya;
+    T q0, q1, r0, r1;
+    mv(m.R[a], v0, v1, q0, q1);
+    mv(m.R[a], cxb, cyb, r0, r1);
+    const Aniso<T> A = aniso(m.dab, q0, q1);
+    const T q2 = q0 * q0 + q1 * q1;
+    const T qr = q0 * r0 + q1 * r1, dr = A.d0 * r0 + A.d1 * r1;
+    const T dA = (T)2 * m.gam * (A.ac * A.ac * qr + A.ac * q2 * dr);
+    const T psi = psi_of(m, a, mu);
+    const T lam = act_a ? m.eps * (-dA + (T)2 * m.gam * sum4) - m.inv_eps * wfun(m, ph, act, a) - psi * dhfun(pa) : (T)0;
+    const T lam_o = __shfl_xor_sync(ALL, lam, 4);
+    const T l0 = a ? lam_o : lam, l1 = a ? lam : lam_o;
+    const int na = (act[0] ? 1 : 0) + (act[1] ? 1 : 0);
+    const T nact = (T)(na ? na : 1), mean = (l0 + l1) / nact;
+    const T kk = m.dt * mob_eff(m, ph) / m.eps;
+    T dp[2] = {act[0] ? kk * (l0 - mean) : (T)0, act[1] ? kk * (l1 - mean) : (T)0};
+    Proj pr;
+    T Dsum, sphi;
+    proj_fwd(ph, act, dp, pr, Dsum, sphi);
+    T ld[2] = {ldp[0], ldp[1]}, lph[2] = {(T)0, (T)0};
+    proj_rev(ph, act, pr, Dsum, sphi, ld, lph);
+    const T m0 = act[0] ? kk * ld[0] : (T)0, m1 = act[1] ? kk * ld[1] : (T)0;
+    const T la = act_a && on ? (a ? m1 : m0) - (m0 + m1) / nact : (T)0;
+    if (on && sub == 0)
+      acc[0] += (double)((act[0] ? ld[0] * (l0 - mean) : (T)0) * kk / m.mob +
+                         (act[1] ? ld[1] * (l1 - mean) : (T)0) * kk / m.mob);
+    if (!on || sub != 0) lph[0] = lph[1] = (T)0;  // the projection's own adjoint once per cell
+    T lpa = a ? lph[1] : lph[0], lpb = a ? lph[0] : lph[1];
+    // the face's reverse
+    const T lt = m.eps * la;
+    T lQx = (T)0, lQy = (T)0, lS = (T)0, ldab = (T)0, lgam = (T)0, lmu = (T)0;
+    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir, pdiv((T)2 * m.gam * sg, h) * lt, lQx, lQy, lS, ldab);
+    const T lQn = dir ? lQy : lQx, lQt = dir ? lQx : lQy;
+    const T lsa = lQn * gb + (T)0.5 * lQt * tb, lsb = -lQn * ga - (T)0.5 * lQt * ta + lS;
+    const T lga = -lQn * sb, lgb = lQn * sa, lta = -(T)0.5 * lQt * sb, ltb = (T)0.5 * lQt * sa;
+    // the centre's reverse (every lane of the phase evaluates it; lanes k = 0 and 1 use it)
+    T lcxa, lcya, lcxb = (T)0, lcyb = (T)0;
+    {
+      const T ldA = -lt, L = (T)2 * m.gam * ldA;
+      const T lac = L * ((T)2 * A.ac * qr + q2 * dr);
+      const T lqr = L * A.ac * A.ac, lq2 = L * A.ac * dr, ldr = L * A.ac * q2;
+      const T ld0 = ldr * r0, ld1 = ldr * r1;
+      const T lr0 = lqr * q0 + ldr * A.d0, lr1 = lqr * q1 + ldr * A.d1;
+      const T c = (T)16 * m.dab;
+      const T lq0 = lqr * r0 + c * (ld0 * A.J[0][0] + ld1 * A.J[1][0]) + lac * A.d0 + (T)2 * q0 * lq2;
+      const T lq1 = lqr * r1 + c * (ld0 * A.J[0][1] + ld1 * A.J[1][1]) + lac * A.d1 + (T)2 * q1 * lq2;
+      T lv0 = (T)0, lv1 = (T)0;
+      mv_rev(m.R[a], lr0, lr1, lcxb, lcyb);
+      mv_rev(m.R[a], lq0, lq1, lv0, lv1);
+      lcxb += lv0 * pa;
+      lcyb += lv1 * pa;
+      lcxa = -lv0 * pb;
+      lcya = -lv1 * pb;
+      if (k == 0) {
+        ldab += (T)16 * (ld0 * A.u0 + ld1 * A.u1) + lac * A.g;
+        lgam += (T)2 * sum4 * lt + (T)2 * (A.ac * A.ac * qr + A.ac * q2 * dr) * ldA;
+        lpa += lv0 * cxb + lv1 * cyb;
+        lpb += -lv0 * cxa - lv1 * cya;
+        const T lw = -m.inv_eps * la;
+        if (a ? act[0] : act[1]) {
+          if (m.obstacle) {
+            const T sgn = (pa * pb >= (T)0) ? (T)1 : (T)-1;
+            lpb += m.wobs * sgn * m.gam * lw;
+            lgam += m.wobs * sgn * pb * lw;
+          } else {
+            lpb += (T)36 * m.gam * pb * pa * lw;
+            lpa += (T)18 * m.gam * pb * pb * lw;
+            lgam += (T)18 * pb * pb * pa * lw;
+          }
+        }
+        lmu = -dpsi_dmu(m, a, mu) * dhfun(pa) * la;
+        lpa -= psi * d2hfun(pa) * la;
+      }
+    }
+    if (!on) {  // the other cells of the warp: nothing (their operands may have overflowed)
+      ldab = lgam = lmu = (T)0;
+      lpa = lpb = (T)0;
+    }
+    acc[1] += (double)ldab;
+    acc[2] += (double)lgam;
+    lmu += __shfl_xor_sync(ALL, lmu, 4);
+    if (on && sub == 0) add_nz(lam_out + ix_mu(g, x, y), lmu);
+    // the six cells of the face, both phases of the pair; the partner lane (the other phase) holds
+    // the same cells' other half, exchanged so that a lane adds one phase's values
+    T mine[2][3], other[2][3];
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+      const T lg = pdiv(w ? lgb : lga, h), ls = (T)0.5 * (w ? lsb : lsa), lT = w ? ltb : lta;
+      const T tv = dir == 0 ? pdiv(lT, ty) : pdiv((T)0.5 * lT, m.dx);
+      T v[2][3] = {{-tv, ls - lg, tv}, {-tv, ls + lg, tv}};
+      const T hx = pdiv((T)0.5 * (w ? lcxb : lcxa), m.dx), hy = pdiv(w ? lcyb : lcya, ty);
+      if (k == 0) {  // rows x, x + 1: the centre and its x+, y-, y+ neighbours
+        v[0][1] += w ? lpb : lpa;
+        v[1][1] += hx;
+        v[0][0] -= hy;
+        v[0][2] += hy;
+      } else if (k == 1) {  // row x - 1
+        v[0][1] -= hx;
+      }
+#pragma unroll
+      for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+        for (int t = 0; t < 3; t++) (w ? other : mine)[nn][t] = on ? v[nn][t] : (T)0;
+    }
+#pragma unroll
+    for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+      for (int t = 0; t < 3; t++) {
+        const T v = mine[nn][t] + __shfl_xor_sync(ALL, other[nn][t], 4);
+        if (!on) continue;
+        const int dn = nn - (k & 1), dt = t - 1;
+        add_nz(lam_out + ix_phi(g, dir ? x + dt : x + dn, dir ? y + dn : y + dt, a), v);
+      }
   }
-  reduce_params(lpd, grad);
+#pragma unroll
+  for (int p = 0; p < 3; p++) block_add(acc[p], part + 3 * blockIdx.x + p);
+}
+
+// The parameter gradients from the blocks' sums: thread block p, a fixed order.
+__global__ void __launch_bounds__(256) k_grad(const double* __restrict__ cell, int ncell,
+                                              const double* __restrict__ jat, int njat,
+                                              const double* __restrict__ dphi, int ndphi, double* __restrict__ grad) {
+  const int p = blockIdx.x;
+  double v = 0.0;
+  if (p == P_DLIQ) {
+    for (int i = threadIdx.x; i < ncell; i += blockDim.x) v += cell[i];
+    for (int i = threadIdx.x; i < njat; i += blockDim.x) v += jat[i];
+  } else {
+    for (int i = threadIdx.x; i < ndphi; i += blockDim.x) v += dphi[3 * i + p];
+  }
+  if (threadIdx.x == 0) grad[p] = 0.0;
+  block_add(v, grad + p);
+}
+
+// Values start .. start + n - 1 of dense FP64 host planes, staged on the device, <-> the planes at st.
+template <typename T>
+__global__ void __launch_bounds__(256) k_fields(T* __restrict__ st, double* __restrict__ stage, Geo g, int64_t start,
+                                                int64_t n, int up) {
+  const int64_t cells = (int64_t)g.mx * g.my;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = (start + i) / cells, r = (start + i) % cells;
+    const int64_t o = p * g.plane + (r / g.my) * g.pitch + r % g.my;
+    if (up) st[o] = (T)stage[i];
+    else stage[i] = (double)st[o];
+  }
 }
 
 // ------------------------------------------------------------------ host side
@@ -366,9 +773,17 @@ struct Adj : AdjBase {
   AM<T> m;
   Geo g;
   cudaStream_t s = nullptr;
-  T *ckpt = nullptr, *seg = nullptr, *cur = nullptr, *nxt = nullptr, *ring = nullptr;
-  T *lam[2] = {nullptr, nullptr}, *ldphi = nullptr, *gdf = nullptr, *gdj = nullptr;
-  double* dgrad = nullptr;
+  T *ckpt = nullptr, *seg = nullptr, *cur = nullptr, *nxt = nullptr;
+  int64_t ckpt_states = 0, seg_states = 0;  // capacities, kept between calls
+  // Delta-phi, list of the cells that are not flat and its length: of every state of a segment
+  // (slots == seg_states), or of one state at a time, recomputed before its reverse, where that
+  // does not fit (slots == 1)
+  T* ring = nullptr;
+  int *list = nullptr, *cnt = nullptr;
+  int64_t slots = 0;
+  T *lam[2] = {nullptr, nullptr}, *ldphi = nullptr;
+  double *part = nullptr, *dgrad = nullptr, *stage = nullptr;
+  int ntile = 0, nlist = 0;  // blocks of the dense kernels and of the list kernels
   int64_t nsteps = 0, every = 0, nck = 0;
   bool have = false;
 
@@ -381,12 +796,14 @@ struct Adj : AdjBase {
     cudaFree(cur);
     cudaFree(nxt);
     cudaFree(ring);
+    cudaFree(list);
+    cudaFree(cnt);
     cudaFree(lam[0]);
     cudaFree(lam[1]);
     cudaFree(ldphi);
-    cudaFree(gdf);
-    cudaFree(gdj);
+    cudaFree(part);
     cudaFree(dgrad);
+    cudaFree(stage);
     if (s) cudaStreamDestroy(s);
   }
 
@@ -400,65 +817,107 @@ struct Adj : AdjBase {
     g.rpitch = (int)gp_round_up(g.my + 2, 32);
     g.rplane = (int64_t)g.rpitch * (g.mx + 2);
     g.bc = gp_bc_of(model);
+    if (g.rplane > INT32_MAX) {
+      gp_set_error("adjoint: %d x %d cells do not fit", g.mx, g.my);
+      return GP_E_NOMEM;
+    }
+    int dev = 0, sms = 0;
+    ADJ_CUDA(cudaGetDevice(&dev));
+    ADJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    ntile = ((g.mx + TX - 1) / TX) * ((g.my + TY - 1) / TY);
+    nlist = 4 * sms;
     ADJ_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     ADJ_CUDA(cudaMalloc(&cur, sizeof(T) * state()));
     ADJ_CUDA(cudaMalloc(&nxt, sizeof(T) * state()));
-    ADJ_CUDA(cudaMalloc(&ring, sizeof(T) * 2 * g.rplane));
     ADJ_CUDA(cudaMalloc(&lam[0], sizeof(T) * state()));
     ADJ_CUDA(cudaMalloc(&lam[1], sizeof(T) * state()));
     ADJ_CUDA(cudaMalloc(&ldphi, sizeof(T) * 2 * g.rplane));
-    ADJ_CUDA(cudaMalloc(&gdf, sizeof(T) * g.plane));
-    ADJ_CUDA(cudaMalloc(&gdj, sizeof(T) * g.plane));
+    ADJ_CUDA(cudaMalloc(&part, sizeof(double) * ((int64_t)ntile + 4 * nlist)));
     ADJ_CUDA(cudaMalloc(&dgrad, sizeof(double) * NPARAM));
     ADJ_CUDA(cudaMemsetAsync(cur, 0, sizeof(T) * state(), s));
     ADJ_CUDA(cudaMemsetAsync(nxt, 0, sizeof(T) * state(), s));
     return GP_OK;
   }
 
-  cudaError_t step(const T* in, T* out) {
-    const dim3 b(256), gr((g.my + 2 + 255) / 256, g.mx + 2), gu((g.my + 255) / 256, g.mx);
-    k_fwd_dphi<T><<<gr, b, 0, s>>>(m, g, in, ring);
-    k_fwd_update<T><<<gu, b, 0, s>>>(m, g, in, ring, out);
+  cudaError_t step(const T* in, T* out, T* r = nullptr, int* l = nullptr, int* c = nullptr) {
+    k_fwd<T><<<ntile, NT, 0, s>>>(m, g, in, out, r, l, c);
     return cudaGetLastError();
   }
 
-  // lam_in = adjoint of the state after x, lam_out = adjoint of x
-  cudaError_t rev_step(const T* x, const T* lin, T* lout) {
-    const dim3 b(256), gr((g.my + 2 + 255) / 256, g.mx + 2), gu((g.my + 255) / 256, g.mx);
-    k_fwd_dphi<T><<<gr, b, 0, s>>>(m, g, x, ring);
-    cudaError_t e = cudaMemsetAsync(ldphi, 0, sizeof(T) * 2 * g.rplane, s);
-    if (e != cudaSuccess) return e;
-    k_rev_cell<T><<<gu, b, 0, s>>>(m, g, x, ring, lin, lout, ldphi, gdf, gdj);
-    const dim3 gf((g.my + 1 + 255) / 256, g.mx + 1, 2);
-    k_rev_face<T><<<gf, b, 0, s>>>(m, g, x, ring, gdf, gdj, lout, ldphi, dgrad);
-    k_rev_dphi<T><<<gr, b, 0, s>>>(m, g, x, ldphi, lout, dgrad);
+  // lin = adjoint of the state after x, lout = adjoint of x; r, l, c: x's Delta-phi, list and its length
+  cudaError_t rev_step(const T* x, const T* r, const int* l, const int* c, const T* lin, T* lout) {
+    k_rev_cell<T><<<ntile, NT, 0, s>>>(m, g, x, r, lin, lout, ldphi, part);
+    k_rev_jat<T><<<nlist, 128, 0, s>>>(m, g, x, r, lin, lout, ldphi, l, c, part + ntile);
+    k_rev_dphi<T><<<nlist, 128, 0, s>>>(m, g, x, ldphi, lout, l, c, part + ntile + nlist);
     return cudaGetLastError();
   }
 
-  // host [planes][mx][my] doubles <-> device [planes][mx][pitch] T
+  // Host [planes][mx][my] doubles <-> device [planes][mx][pitch] T, converted on the device through a
+  // staging buffer of at most kStage doubles (the conversion of a 512^2 state on a host core took
+  // longer than its 100 steps).  An upload without a host array is zeros.
+  static constexpr int64_t kStage = 4 << 20;
+  int move(T* planes, int nplanes, double* host, bool up) {
+    const int64_t all = (int64_t)nplanes * g.mx * g.my;
+    if (!host) {
+      if (up) ADJ_CUDA(cudaMemsetAsync(planes, 0, sizeof(T) * nplanes * g.plane, s));
+      return GP_OK;
+    }
+    const int64_t room = 3ll * g.mx * g.my < kStage ? 3ll * g.mx * g.my : kStage;
+    if (!stage) ADJ_CUDA(cudaMalloc(&stage, sizeof(double) * room));
+    for (int64_t at = 0; at < all; at += room) {
+      const int64_t n = all - at < room ? all - at : room;
+      if (up) ADJ_CUDA(cudaMemcpyAsync(stage, host + at, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+      k_fields<T><<<592, 256, 0, s>>>(planes, stage, g, at, n, up ? 1 : 0);
+      ADJ_CUDA(cudaGetLastError());
+      if (!up) ADJ_CUDA(cudaMemcpyAsync(host + at, stage, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+    }
+    return GP_OK;
+  }
   int upload(T* dst, const double* phi, const double* mu) {
-    std::vector<T> h(state(), (T)0);
-    for (int a = 0; a < 3; a++) {
-      const double* src = a < 2 ? (phi ? phi + (int64_t)a * g.mx * g.my : nullptr) : mu;
-      if (!src) continue;
-      for (int x = 0; x < g.mx; x++)
-        for (int y = 0; y < g.my; y++) h[a * g.plane + (int64_t)x * g.pitch + y] = (T)src[(int64_t)x * g.my + y];
-    }
-    ADJ_CUDA(cudaMemcpyAsync(dst, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, s));
-    ADJ_CUDA(cudaStreamSynchronize(s));
-    return GP_OK;
+    int rc = move(dst, 2, const_cast<double*>(phi), true);
+    return rc == GP_OK ? move(dst + 2 * g.plane, 1, const_cast<double*>(mu), true) : rc;
   }
-  int download(const T* src, double* phi, double* mu) {
-    std::vector<T> h(state());
-    ADJ_CUDA(cudaMemcpyAsync(h.data(), src, sizeof(T) * h.size(), cudaMemcpyDeviceToHost, s));
-    ADJ_CUDA(cudaStreamSynchronize(s));
-    for (int a = 0; a < 3; a++) {
-      double* dst = a < 2 ? (phi ? phi + (int64_t)a * g.mx * g.my : nullptr) : mu;
-      if (!dst) continue;
-      for (int x = 0; x < g.mx; x++)
-        for (int y = 0; y < g.my; y++) dst[(int64_t)x * g.my + y] = (double)h[a * g.plane + (int64_t)x * g.pitch + y];
+  int download(T* src, double* phi, double* mu) {
+    int rc = move(src, 2, phi, false);
+    if (rc == GP_OK) rc = move(src + 2 * g.plane, 1, mu, false);
+    if (rc == GP_OK) ADJ_CUDA(cudaStreamSynchronize(s));
+    return rc;
+  }
+
+  // at least `need` states in *p, the old ones released first when there are too few
+  bool reserve(T** p, int64_t* have_states, int64_t need) {
+    if (*have_states >= need) return true;
+    cudaFree(*p);
+    *p = nullptr;
+    *have_states = 0;
+    if (cudaMalloc(p, sizeof(T) * state() * need) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return false;
     }
-    return GP_OK;
+    *have_states = need;
+    return true;
+  }
+
+  // Delta-phi, list and count slots for `need` states, or for one where they do not fit
+  bool reserve_slots(int64_t need) {
+    if (slots >= need) return true;
+    for (int64_t n = need;; n = 1) {
+      cudaFree(ring);
+      cudaFree(list);
+      cudaFree(cnt);
+      ring = nullptr;
+      list = cnt = nullptr;
+      slots = 0;
+      if (cudaMalloc(&ring, sizeof(T) * 2 * g.rplane * n) == cudaSuccess &&
+          cudaMalloc(&list, sizeof(int) * g.rplane * n) == cudaSuccess &&
+          cudaMalloc(&cnt, sizeof(int) * n) == cudaSuccess) {
+        slots = n;
+        return true;
+      }
+      cudaGetLastError();
+      if (n == 1) return false;
+    }
   }
 
   int forward(const double* phi0, const double* mu0, int64_t n, int64_t ev, double* phi_out,
@@ -467,13 +926,23 @@ struct Adj : AdjBase {
     if (ev <= 0) ev = (int64_t)ceil(sqrt((double)n));
     if (ev > n) ev = n;
     const int64_t nc = (n + ev - 1) / ev;
-    cudaFree(ckpt);
-    cudaFree(seg);
-    ckpt = seg = nullptr;
     have = false;
-    if (cudaMalloc(&ckpt, sizeof(T) * state() * nc) != cudaSuccess ||
-        cudaMalloc(&seg, sizeof(T) * state() * ev) != cudaSuccess) {
-      cudaGetLastError();
+    ADJ_CUDA(cudaStreamSynchronize(s));  // buffers are released below only when too small
+    bool ok = reserve(&ckpt, &ckpt_states, nc) && reserve(&seg, &seg_states, ev) && reserve_slots(ev);
+    if (!ok) {  // what an earlier, other split keeps may stand in the way: start over
+      cudaFree(ckpt);
+      cudaFree(seg);
+      ckpt = seg = nullptr;
+      ckpt_states = seg_states = 0;
+      cudaFree(ring);
+      cudaFree(list);
+      cudaFree(cnt);
+      ring = nullptr;
+      list = cnt = nullptr;
+      slots = 0;
+      ok = reserve(&ckpt, &ckpt_states, nc) && reserve(&seg, &seg_states, ev) && reserve_slots(ev);
+    }
+    if (!ok) {
       gp_set_error("adjoint: %lld checkpoints + %lld segment states do not fit", (long long)nc, (long long)ev);
       return GP_E_NOMEM;
     }
@@ -503,17 +972,29 @@ struct Adj : AdjBase {
     if (!grad) return GP_E_ARG;
     int rc = upload(lam[0], lphi, lmu);
     if (rc != GP_OK) return rc;
-    ADJ_CUDA(cudaMemsetAsync(dgrad, 0, sizeof(double) * NPARAM, s));
+    ADJ_CUDA(cudaMemsetAsync(part, 0, sizeof(double) * ((int64_t)ntile + 4 * nlist), s));
+    const bool all = slots >= every;  // every state of a segment has its slot
     int li = 0;
     for (int64_t k = nck - 1; k >= 0; k--) {
       const int64_t start = k * every, len = (nsteps - start < every) ? nsteps - start : every;
-      ADJ_CUDA(cudaMemcpyAsync(seg, ckpt + k * state(), sizeof(T) * state(), cudaMemcpyDeviceToDevice, s));
-      for (int64_t i = 1; i < len; i++) ADJ_CUDA(step(seg + (i - 1) * state(), seg + i * state()));
+      const T* const first = ckpt + k * state();
+      auto at = [&](int64_t i) { return i ? seg + i * state() : first; };
+      if (all) ADJ_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * len, s));
+      for (int64_t i = 1; i < len; i++)
+        ADJ_CUDA(all ? step(at(i - 1), seg + i * state(), ring + (i - 1) * 2 * g.rplane, list + (i - 1) * g.rplane, cnt + (i - 1))
+                     : step(at(i - 1), seg + i * state()));
       for (int64_t i = len - 1; i >= 0; i--) {
-        ADJ_CUDA(rev_step(seg + i * state(), lam[li], lam[li ^ 1]));
+        const int64_t q = all ? i : 0;
+        T* const r = ring + q * 2 * g.rplane;
+        int* const l = list + q * g.rplane;
+        if (!all) ADJ_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
+        if (!all || i == len - 1) ADJ_CUDA(step(at(i), nullptr, r, l, cnt + q));
+        ADJ_CUDA(rev_step(at(i), r, l, cnt + q, lam[li], lam[li ^ 1]));
         li ^= 1;
       }
     }
+    k_grad<<<NPARAM, 256, 0, s>>>(part, ntile, part + ntile, nlist, part + ntile + nlist, nlist, dgrad);
+    ADJ_CUDA(cudaGetLastError());
     ADJ_CUDA(cudaMemcpyAsync(grad, dgrad, sizeof(double) * NPARAM, cudaMemcpyDeviceToHost, s));
     ADJ_CUDA(cudaStreamSynchronize(s));
     if (lphi0 || lmu0) return download(lam[li], lphi0, lmu0);

@@ -1,0 +1,85 @@
+"""The adjoint's tiled kernels at the sizes where they can go wrong: grids smaller than a tile, exact
+multiples of the 8 x 32 tile and one cell either way, interfaces crossing every border, each boundary
+type per axis, and segments whose Delta-phi is recomputed state by state.
+
+The yardstick is a directional central difference of the FP64 forward (the initial-state adjoint and the
+mobility/diffusivity gradients in one number each): with h = 1e-6 its own error is about 1e-9 relative from
+rounding plus h^2 from the third derivative, far below the 1e-4 asked for."""
+import numpy as np
+import pytest
+
+import microsim_b200 as mb
+from microsim_b200 import adjoint, configs
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(4, 4), (7, 31), (8, 32), (9, 33), (16, 64), (17, 65), (23, 5), (5, 70)]
+
+
+def _case(mx, my, bc, well):
+    c = configs.binary_case(mx, my, gap=1.0, supersat=0.5, eps=3.0, delta=0.03, theta=12.0, dt=0.05, tau=1.3332,
+                            function_w=2 if well else 1, seed=(0, 0, 0.4 * max(mx, my)), bc=bc)
+    return mb.load_case(c)
+
+
+@pytest.mark.parametrize("well", [0, 1])
+@pytest.mark.parametrize("bc", [(1, 1, 1, 1), (3, 3, 1, 1), (1, 1, 3, 3), (3, 3, 3, 3)])
+@pytest.mark.parametrize("size", SIZES)
+def test_adjoint_matches_directional_differences(size, bc, well):
+    m, phi, mu = _case(*size, bc, well)
+    rng = np.random.default_rng(1)
+    with mb.Context(m, mb.GP_FP64) as c:  # a state with a developed interface, off the projection's corners
+        c.upload(phi, mu)
+        c.step(60)
+        phi, mu = c.download()
+    steps = 5
+    wp, wu = rng.standard_normal(phi.shape), rng.standard_normal(mu.shape)
+    inside = (phi > 1e-3) & (phi < 1 - 1e-3)
+    dphi, dmu = rng.standard_normal(phi.shape) * inside, rng.standard_normal(mu.shape)
+    dp = np.array([0.3, 0.0, 0.2, 0.3])
+    p = adjoint.params_of(m)
+
+    def forward(h, every=0, back=False):
+        with adjoint.Adjoint(adjoint.with_params(m, p + h * dp), mb.GP_FP64) as a:
+            q, u = a.forward(phi + h * dphi, mu + h * dmu, steps, every)
+            if back:
+                return a.backward(wp, wu, initial=True)
+            return float((wp * q).sum() + (wu * u).sum())
+
+    g, lphi, lmu = forward(0.0, back=True)
+    an = float((lphi * dphi).sum() + (lmu * dmu).sum() + g @ dp)
+    h = 1e-6
+    fd = (forward(h) - forward(-h)) / (2 * h)
+    scale = np.abs(lphi * dphi).sum() + np.abs(lmu * dmu).sum() + np.abs(g * dp).sum()
+    assert abs(an - fd) <= 1e-4 * scale, (an, fd, scale)
+    for every in (1, 2, steps):
+        g2, lphi2, lmu2 = forward(0.0, every, True)
+        np.testing.assert_allclose(g2, g, rtol=1e-9, atol=1e-12 * np.abs(g).max())
+        np.testing.assert_allclose(lphi2, lphi, rtol=1e-9, atol=1e-11 * np.abs(lphi).max())
+
+
+def test_forward_is_the_plain_step_at_every_size():
+    for size in SIZES:
+        m, phi, mu = _case(*size, (3, 3, 1, 1), 0)
+        with adjoint.Adjoint(m, mb.GP_FP64) as a:
+            pa, ua = a.forward(phi, mu, 40)
+        with mb.Context(m, mb.GP_FP64) as c:
+            c.upload(phi, mu)
+            c.step(40)
+            pp, up = c.download()
+        assert np.abs(pa - pp).max() <= 1e-10 and np.abs(ua - up).max() <= 1e-10, size
+
+
+def test_runs_of_different_lengths_on_one_object():
+    """The kept workspaces serve shorter, longer and shorter runs again, each as a fresh object's."""
+    m, phi, mu = _case(33, 40, (1, 1, 1, 1), 0)
+    w = np.random.default_rng(2).standard_normal(phi.shape)
+    with adjoint.Adjoint(m, mb.GP_FP64) as a:
+        for steps, every in ((9, 0), (50, 0), (4, 1), (50, 25), (1, 0)):
+            q, u = a.forward(phi, mu, steps, every)
+            g = a.backward(w)
+            with adjoint.Adjoint(m, mb.GP_FP64) as b:
+                q2, u2 = b.forward(phi, mu, steps, every)
+                g2 = b.backward(w)
+            assert np.array_equal(q, q2) and np.array_equal(u, u2)
+            np.testing.assert_allclose(g, g2, rtol=1e-10)
