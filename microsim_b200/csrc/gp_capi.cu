@@ -21,6 +21,15 @@ extern "C" void gp_set_error(const char* fmt, ...);
 cudaError_t gp_f64_step(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane, const double* phi,
                         const double* mu, double* dphi, double* phi_out, double* mu_out, cudaStream_t s, bool smooth = false, const double* ghost_rows = nullptr,
                         const gp_temp_step* temp = nullptr);
+struct gp_f64_tiles;
+cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out);
+void gp_f64_tiles_destroy(gp_f64_tiles* t);
+cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s);
+cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
+                              const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
+                              const gp_temp_step* temp);
+cudaError_t gp_f64_dphi(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane, const double* phi,
+                        const double* mu, double* dphi, cudaStream_t s, const gp_temp_step* temp);
 struct gp_f32_batch;
 int gp_f32_supported(const gp_model& m);
 cudaError_t gp_f32_batch_create(const gp_model* models, int n, gp_f32_batch** out);
@@ -104,6 +113,9 @@ struct gp_ctx {
   void* phi[2];
   void* mu[2];
   double* dphi;    // FP64 form: Delta-phi of the last phase-field half step
+  gp_f64_tiles* tiles;    // FP64 form: the tile kernels' tables (nullptr: every step through dphi)
+  int dphi_stale;         // the tile kernels took the last step: dphi follows from buffer 1-cur when asked for
+  gp_temp_step last_temp; // the temperature that step ran at
   double* gov;     // FP64 form: the ghost rows a moving-frame shift leaves ([N+K1][mx][6])
   int gov_pending; // the next phase-field half step reads gov
   gp_f32_batch* f32;  // FP32 form: a batch of one instance over phi/mu
@@ -188,7 +200,8 @@ extern "C" int gp_create(const gp_model* m, int precision, gp_ctx** out) {
   }
   if (ok && precision == GP_FP64) {
     ok = cudaMalloc(&c->dphi, (size_t)m->N * c->rplane * sizeof(double)) == cudaSuccess &&
-         cudaMemset(c->dphi, 0, (size_t)m->N * c->rplane * sizeof(double)) == cudaSuccess;
+         cudaMemset(c->dphi, 0, (size_t)m->N * c->rplane * sizeof(double)) == cudaSuccess &&
+         gp_f64_tiles_create(*m, &c->tiles) == cudaSuccess;
   }
   if (ok) ok = cudaMalloc(&c->partials, (size_t)c->red_blocks * 64 * sizeof(double)) == cudaSuccess &&
                cudaMalloc(&c->reduced, 64 * sizeof(double)) == cudaSuccess;
@@ -223,6 +236,7 @@ extern "C" int gp_destroy(gp_ctx* c) {
     if (c->g64[i]) cudaGraphExecDestroy(c->g64[i]);
   if (c->dphi) cudaFree(c->dphi);
   if (c->gov) cudaFree(c->gov);
+  gp_f64_tiles_destroy(c->tiles);
   if (c->f32) gp_f32_batch_destroy(c->f32);
   if (c->partials) cudaFree(c->partials);
   if (c->stage) cudaFree(c->stage);
@@ -318,6 +332,7 @@ extern "C" int gp_upload(gp_ctx* c, const double* phi, const double* mu) {
   int rc = copy_planes(c, phi, c->phi[c->cur], c->m.N, true);
   if (rc == GP_OK) rc = copy_planes(c, mu, c->mu[c->cur], c->m.K1, true);
   if (rc == GP_OK && c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
+  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
   if (rc == GP_OK) GP_CUDA(cudaStreamSynchronize(c->stream));
   c->have_prev = 0;
   return rc;
@@ -331,15 +346,45 @@ extern "C" int gp_download(gp_ctx* c, double* phi, double* mu) {
   return rc;
 }
 
+// Delta-phi of the last half step into c->dphi, when the tile kernels took that step: buffer 1-cur
+// still holds the state it started from.
+static int dphi_ready(gp_ctx* c) {
+  if (!c->dphi_stale) return GP_OK;
+  GP_CUDA(gp_f64_dphi(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[1 - c->cur],
+                      (const double*)c->mu[1 - c->cur], c->dphi, c->stream, &c->last_temp));
+  c->launches++;
+  c->dphi_stale = 0;
+  return GP_OK;
+}
+
 extern "C" int gp_download_dphi(gp_ctx* c, double* dphi) {
   if (!c || !dphi) return GP_E_ARG;
   if (c->precision != GP_FP64) return GP_E_UNSUPPORTED;
+  const int rc = dphi_ready(c);
+  if (rc != GP_OK) return rc;
   const int64_t rx = c->m.mesh_x + 2, ry = c->m.mesh_y + 2;
   for (int a = 0; a < c->m.N; a++)
     GP_CUDA(cudaMemcpy2DAsync(dphi + a * rx * ry, ry * sizeof(double), c->dphi + a * c->rplane,
                               c->rpitch * sizeof(double), ry * sizeof(double), rx, cudaMemcpyDeviceToHost, c->stream));
   GP_CUDA(cudaStreamSynchronize(c->stream));
   return GP_OK;
+}
+
+// One FP64 step from the current buffer into the other, queued: the tile kernels, or the ring-array
+// path for the step after a moving-frame shift (its explicit ghost rows) and for models the tile
+// kernels do not take.  Returns the launches it took, or a negative error.
+static int f64_launch(gp_ctx* c, int p, const gp_temp_step& ts, const double* gov) {
+  if (c->tiles && !gov) {
+    GP_CUDA(gp_f64_step_tiled(c->m, c->tiles, p, c->pitch, c->plane, (const double*)c->phi[p], (const double*)c->mu[p],
+                              (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream, &ts));
+    c->dphi_stale = 1;
+    return 2;
+  }
+  GP_CUDA(gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[p], (const double*)c->mu[p],
+                      c->dphi, (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream, false, gov, &ts));
+  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+  c->dphi_stale = 0;
+  return 2;
 }
 
 // An isothermal FP64 step is the same two launches every time (no per-step temperature), so
@@ -354,11 +399,9 @@ static int f64_graph(gp_ctx* c, cudaGraphExec_t* out) {
     const gp_temp_step ts = gp_temp_after(c->m, 0);  // not read by an isothermal step
     cudaGraph_t g = nullptr;
     GP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    for (int t = 0, p = c->cur; t < kF64GraphSteps && e == cudaSuccess; t++, p ^= 1)
-      e = gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[p],
-                      (const double*)c->mu[p], c->dphi, (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream,
-                      false, nullptr, &ts);
+    int rc = 0;
+    for (int t = 0, p = c->cur; t < kF64GraphSteps && rc >= 0; t++, p ^= 1) rc = f64_launch(c, p, ts, nullptr);
+    cudaError_t e = rc < 0 ? cudaErrorUnknown : cudaSuccess;
     const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&ge, g, 0);
@@ -379,6 +422,7 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
       if (rc != GP_OK) return rc;
       GP_CUDA(cudaGraphLaunch(ge, c->stream));
       c->launches += 2 * kF64GraphSteps;
+      c->dphi_stale = c->tiles != nullptr;
       c->have_prev = 1;
       c->tstep += kF64GraphSteps;
       t += kF64GraphSteps - 1;
@@ -387,11 +431,11 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
     const int nxt = 1 - c->cur;
     if (c->precision == GP_FP64) {
       const gp_temp_step ts = gp_temp_after(c->m, c->tstep);  // T reset after the previous step
-      GP_CUDA(gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[c->cur],
-                          (const double*)c->mu[c->cur], c->dphi, (double*)c->phi[nxt], (double*)c->mu[nxt],
-                          c->stream, false, c->gov_pending ? c->gov : nullptr, &ts));
+      const int n = f64_launch(c, c->cur, ts, c->gov_pending ? c->gov : nullptr);
+      if (n < 0) return n;
       c->gov_pending = 0;
-      c->launches += 2;
+      c->launches += n;
+      c->last_temp = ts;
     } else {
       GP_CUDA(gp_f32_batch_launch(c->f32, c->cur, c->stream));
       c->launches += gp_f32_batch_launches_per_step(c->f32);
@@ -438,6 +482,8 @@ extern "C" int gp_smooth(gp_ctx* c, int64_t nsteps) {
       c->launches += 2;
       c->cur = nxt;
     }
+    GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+    c->dphi_stale = 0;
     c->have_prev = 0;
     return GP_OK;
   }
@@ -540,6 +586,8 @@ extern "C" int gp_interface_y(gp_ctx* c, int64_t* pos) {
 extern "C" int gp_shift_y(gp_ctx* c, int64_t d) {
   if (!c || d < 0) return GP_E_ARG;
   if (d == 0) return GP_OK;
+  const int rc = dphi_ready(c);  // the shift overwrites the state Delta-phi would follow from
+  if (rc != GP_OK) return rc;
   const int mx = (int)c->m.mesh_x, my = (int)c->m.mesh_y, nxt = 1 - c->cur;
   const dim3 b(256), g((my + 255) / 256, mx);
   const gp_bc bc = gp_bc_of(c->m);
@@ -566,6 +614,7 @@ extern "C" int gp_shift_y(gp_ctx* c, int64_t d) {
   c->cur = nxt;
   c->have_prev = 0;
   if (c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
+  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
   return GP_OK;
 }
 
@@ -604,6 +653,7 @@ extern "C" int gp_state_changed(gp_ctx* c) {
   if (!c) return GP_E_ARG;
   c->have_prev = 0;
   if (c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
+  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
   return GP_OK;
 }
 extern "C" int64_t gp_launch_count(const gp_ctx* c) { return c ? c->launches : 0; }

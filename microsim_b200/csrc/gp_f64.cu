@@ -5,21 +5,30 @@
 // FMA, and every expression keeps the reference's operation order, so the
 // doubles produced here equal the reference solver's.
 //
-// Two kernels per step, the reference's two half steps
-// (microsim_gp.c:103-106), both pure functions of the pre-step state (the
-// reference's sweeps are Jacobi: every stencil read sees old values):
-//   k_dphi   -- Delta-phi on the interior plus one ghost ring
-//               (solverloop/calculate_divergence_phasefield.h:4-62), written to
-//               a scratch ring array (the reference keeps it in the grid cells);
-//   k_update -- antitrapping currents, mu update and phi += Delta-phi on the
-//               interior (calculate_fluxes_concentration.h:4-145,
+// Both half steps of the reference (microsim_gp.c:103-106) are pure functions of
+// the pre-step state (its sweeps are Jacobi: every stencil read sees old values):
+//   Delta-phi on the interior plus one ghost ring
+//               (solverloop/calculate_divergence_phasefield.h:4-62);
+//   antitrapping currents, mu update and phi += Delta-phi on the interior
+//               (calculate_fluxes_concentration.h:4-145,
 //               calculate_divergence_concentration.h:4-153), into the other
 //               buffer of a double-buffered state.
+// k_lean64 steps the tiles far from every interface, k_step64 the others, both half
+// steps of a tile in shared memory.  k_dphi and k_update do them one after the other through a ring array in device memory: the smoothing
+// pre-steps, the step after a moving-frame shift (explicit ghost rows), models with
+// spacings that are no powers of two or pair constants that are not symmetric, and the
+// allocation-free entry.
 // Ghost cells are read through gp_map (boundary copies as index maps).
 //
 // Reference paths are relative to Grand_potential_Finite_difference_2D_serial/.
 
+#include <math.h>
+#include <string.h>
+
+#include <vector>
+
 #include "gp_common.cuh"
+#include "gp_tiles.cuh"
 
 namespace {
 
@@ -128,12 +137,12 @@ __device__ __forceinline__ double hphi(const double* phi, int a) {
   return sum + sum1;
 }
 
-// dh_b/dphi_a, functions/functionH.h:1-23
+// dh_b/dphi_a, functions/functionH.h:1-23 (pa, pb: phi_a, phi_b)
 template <int N>
-__device__ __forceinline__ double dhphi(const double* phi, int b, int a) {
+__device__ __forceinline__ double dhphi(const double* phi, double pb, double pa, int b, int a) {
   double sum = 0.0;
   if (a == b) {
-    sum = 6.0 * phi[a] * (1.0 - phi[a]);
+    sum = 6.0 * pa * (1.0 - pa);
 #pragma unroll
     for (int e = 0; e < N; e++)
 #pragma unroll
@@ -143,9 +152,13 @@ __device__ __forceinline__ double dhphi(const double* phi, int b, int a) {
 #pragma unroll
     for (int e = 0; e < N; e++)
       if (e != b && e != a) sum += 2.0 * phi[e];
-    sum *= phi[b];
+    sum *= pb;
   }
   return sum;
+}
+template <int N>
+__device__ __forceinline__ double dhphi(const double* phi, int b, int a) {
+  return dhphi<N>(phi, phi[b], phi[a], b, a);
 }
 
 // c_a,i(mu, T), functions/functionF_01.h:30-37
@@ -192,6 +205,20 @@ __device__ __forceinline__ double gp_ddiv(double x, double d) {
   if ((bits & 0x000FFFFFFFFFFFFFLL) == 0 && ex > 1 && ex < 2046 && bits > 0)
     return x * __longlong_as_double((2046LL << 52) - bits);
   return x / d;
+}
+
+// a / b (IEEE, the bits of the division) from y = 1.0 / b: two residual corrections of a * y with fused
+// multiply-adds, the last of which rounds correctly (P. Markstein, IBM J. Res. Develop. 34(1), 1990:
+// with y the correctly rounded reciprocal and q within one unit in the last place, q + y (a - b q)
+// rounds to the quotient).  Several quotients by one b then cost one division, without a branch each;
+// operands near the ends of the exponent range, where a residual could leave it, and zeros divide.
+__device__ __forceinline__ double quot(double a, double b, double y) {
+  double q = __dmul_rn(a, y);
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  const double ma = fabs(a), mb = fabs(b);
+  if (ma > 1.0e-200 && ma < 1.0e100 && mb > 1.0e-100 && mb < 1.0e100) return q;
+  return a == 0.0 && b > 0.0 && mb < 1.0e300 ? a : a / b;
 }
 
 template <int N, int K1>
@@ -248,6 +275,26 @@ __device__ __forceinline__ void aniso_dadq(double dab, double q0, double q1, dou
   } else {
     d0 = 0.0;
     d1 = 0.0;
+  }
+}
+
+// aniso_ac and aniso_dadq of one q: five quotients by |q|^4 and |q|^6
+__device__ __forceinline__ void aniso_both(double dab, double q0, double q1, double& ac, double& d0, double& d1) {
+  const double qx2 = q0 * q0, qx4 = qx2 * qx2;
+  const double qy2 = q1 * q1, qy4 = qy2 * qy2;
+  const double q2 = qx2 + qy2;
+  ac = 1.0;
+  d0 = d1 = 0.0;
+  if (fabs(q2) > 1.0e-15) {
+    const double qx3 = q0 * q0 * q0;
+    const double qy3 = q1 * q1 * q1;
+    const double q22 = q2 * q2;
+    const double q23 = q2 * q2 * q2;
+    const double q4 = qx3 * q0 + qy3 * q1;
+    const double y2 = 1.0 / q22, y3 = 1.0 / q23;
+    ac = 1.0 - dab * (3.0 - quot(4.0 * (qx4 + qy4), q22, y2));
+    d0 = 16.0 * dab * (quot(qx3, q22, y2) - quot(q0 * q4, q23, y3));
+    d1 = 16.0 * dab * (quot(qy3, q22, y2) - quot(q1 * q4, q23, y3));
   }
 }
 
@@ -392,15 +439,15 @@ __device__ __forceinline__ double grad_energy_term(const gp_model& m, const doub
   return -dA + divA;
 }
 
-// dw/dphi_a: obstacle functions/functionW_01.h:6-39, well functionW_02.h:4-33
+// dw/dphi_a (pa = phi_a): obstacle functions/functionW_01.h:6-39, well functionW_02.h:4-33
 template <int N>
-__device__ __forceinline__ double dwdphi(const gp_model& m, const double* phi, const double* divphi, int a) {
+__device__ __forceinline__ double dwdphi(const gp_model& m, const double* phi, const double* divphi, double pa, int a) {
   double sum = 0.0;
   if (m.obstacle) {
 #pragma unroll
     for (int b = 0; b < N; b++) {
       if (b == a || !(fabs(divphi[b]) > 0.0)) continue;
-      if ((phi[a] * phi[b]) >= 0.00000) sum += m.Gamma[a][b] * (phi[b]);
+      if ((pa * phi[b]) >= 0.00000) sum += m.Gamma[a][b] * (phi[b]);
       else sum += -m.Gamma[a][b] * (phi[b]);
     }
     sum *= m.w_obstacle;
@@ -408,7 +455,7 @@ __device__ __forceinline__ double dwdphi(const gp_model& m, const double* phi, c
 #pragma unroll
     for (int b = 0; b < N; b++) {
       if (b == a || !(fabs(divphi[b]) > 0.0)) continue;
-      sum += 2.0 * m.Gamma[a][b] * (phi[b] * phi[b] * phi[a]);
+      sum += 2.0 * m.Gamma[a][b] * (phi[b] * phi[b] * pa);
     }
     sum *= 9.0;
   }
@@ -419,11 +466,15 @@ __device__ __forceinline__ double dwdphi(const gp_model& m, const double* phi, c
       if (b == a || c == a) continue;
       if (fabs(divphi[b]) > 0.0 && fabs(divphi[c]) > 0.0) {
         const double pbc = phi[b] * phi[c];
-        if (phi[a] * pbc >= 0.00000) sum += m.Gamma_abc[a][b][c] * pbc;
+        if (pa * pbc >= 0.00000) sum += m.Gamma_abc[a][b][c] * pbc;
         else sum += -m.Gamma_abc[a][b][c] * pbc;
       }
     }
   return sum;
+}
+template <int N>
+__device__ __forceinline__ double dwdphi(const gp_model& m, const double* phi, const double* divphi, int a) {
+  return dwdphi<N>(m, phi, divphi, phi[a], a);
 }
 
 // dw/dphi of the smoothing pre-steps with anisotropy: functionW_01.h:41-62,
@@ -763,6 +814,155 @@ __device__ __forceinline__ void lu_inverse(double (&mm)[K][K], double (&inv)[K][
       }
 }
 
+// Division by the grid spacings: IEEE quotients, or products with their exact reciprocals where the
+// spacings are powers of two (the same bits; gp_ddiv).
+struct DivSpacing {
+  double hx, hy;
+  __device__ __forceinline__ double dx(double v) const { return gp_ddiv(v, hx); }
+  __device__ __forceinline__ double dy(double v) const { return gp_ddiv(v, hy); }
+};
+struct MulSpacing {
+  double ix, iy;
+  __device__ __forceinline__ double dx(double v) const { return v * ix; }
+  __device__ __forceinline__ double dy(double v) const { return v * iy; }
+};
+
+// New mu of a cell from its own and its four neighbours' phi and mu, its Delta-phi and the currents
+// of its four faces.  SMOOTH: the smoothing pre-step (no current, no dh/dt source, the LU inverse).
+template <int N, int K1, bool SMOOTH, typename S>
+__device__ __forceinline__ void cell_update(const gp_model& m, const S& sp, Th thc, const double* ph, const double* phb,
+                                            const double* phf, const double* phl, const double* phr,
+                                            const double* Mc, const double* Mb, const double* Mf, const double* Ml,
+                                            const double* Mr, const double* Dc, const double* jx_c,
+                                            const double* jx_b, const double* jy_c, const double* jy_l,
+                                            double (&mnew)[K1]) {
+  double sum[K1], divflux[K1], divjat[K1], deltac[K1], dcdmu[K1][K1];
+#pragma unroll
+  for (int k = 0; k < K1; k++) {
+    sum[k] = 0.0;
+#pragma unroll
+    for (int l = 0; l < K1; l++) dcdmu[k][l] = 0.0;
+  }
+#pragma unroll
+  for (int a = 0; a < N; a++) {
+    double sdh = 0.0;
+#pragma unroll
+    for (int b = 0; b < N; b++) sdh += dhphi<N>(ph, a, b) * Dc[b];
+#pragma unroll
+    for (int k = 0; k < K1; k++) sum[k] += c_mu<K1>(m, thc, Mc, a, k) * sdh;
+  }
+  const double jscale = m.obstacle ? m.jat_obst : m.jat_well;
+#pragma unroll
+  for (int k = 0; k < K1; k++) {
+    divflux[k] = 0.0;
+#pragma unroll
+    for (int l = 0; l < K1; l++) {
+      const double Dcc = Dcell<N, K1>(m, ph, k, l);
+      const double Dx = (Dcell<N, K1>(m, phf, k, l) + Dcc) * 0.5;
+      const double Dxb = (Dcc + Dcell<N, K1>(m, phb, k, l)) * 0.5;
+      const double Dy = (Dcell<N, K1>(m, phr, k, l) + Dcc) * 0.5;
+      const double Dyl = (Dcc + Dcell<N, K1>(m, phl, k, l)) * 0.5;
+      const double gmx = sp.dx((Mf[l] - Mc[l]));
+      const double gmxb = sp.dx((Mc[l] - Mb[l]));
+      const double gmy = sp.dy((Mr[l] - Mc[l]));
+      const double gmyl = sp.dy((Mc[l] - Ml[l]));
+      divflux[k] += sp.dx((Dx * gmx - Dxb * gmxb));
+      divflux[k] += sp.dy((Dy * gmy - Dyl * gmyl));
+    }
+    if (!SMOOTH) {
+      divjat[k] = sp.dx((jx_c[k] - jx_b[k]) * (jscale));
+      divjat[k] += sp.dy((jy_c[k] - jy_l[k]) * (jscale));
+    }
+  }
+  int bulk = -1;
+#pragma unroll
+  for (int a = 0; a < N; a++)
+    if (bulk < 0 && ph[a] == 1.0) bulk = a;
+  if (bulk >= 0) {
+    double cnew[K1];
+#pragma unroll
+    for (int k = 0; k < K1; k++) {
+      double co = 0.0;
+#pragma unroll
+      for (int a = 0; a < N; a++)
+        if (a == bulk) co = c_mu<K1>(m, thc, Mc, a, k);
+      cnew[k] = SMOOTH ? co + m.dt * (divflux[k]) : co + m.dt * (divflux[k]) - divjat[k];
+    }
+#pragma unroll
+    for (int k = 0; k < K1; k++) {
+      double v = 0.0;
+#pragma unroll
+      for (int a = 0; a < N; a++)
+        if (a == bulk) v = Mu<K1>(m, thc, cnew, a, k);
+      mnew[k] = v;
+    }
+  } else if (SMOOTH) {
+#pragma unroll
+    for (int k = 0; k < K1; k++) {
+      deltac[k] = m.dt * (divflux[k]);
+#pragma unroll
+      for (int l = 0; l < K1; l++)
+#pragma unroll
+        for (int a = 0; a < N; a++) dcdmu[k][l] += m.cmu[a][k][l] * hphi<N>(ph, a);
+    }
+    double inv[K1][K1];
+    lu_inverse<K1>(dcdmu, inv);
+#pragma unroll
+    for (int k = 0; k < K1; k++) {
+      double s = 0;
+#pragma unroll
+      for (int l = 0; l < K1; l++) s = s + inv[k][l] * deltac[l];
+      mnew[k] = s + Mc[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K1; k++) {
+      deltac[k] = m.dt * (divflux[k]) - divjat[k] - sum[k];
+#pragma unroll
+      for (int l = 0; l < K1; l++)
+#pragma unroll
+        for (int a = 0; a < N; a++) dcdmu[k][l] += m.cmu[a][k][l] * hphi<N>(ph, a);
+    }
+#pragma unroll
+    for (int k = 0; k < K1; k++) mnew[k] = Mc[k];
+    if (m.mu_solver == GP_MU_BINARY) {
+      const double iv = 1.0 / dcdmu[0][0];
+      mnew[0] = Mc[0] + deltac[0] * iv;
+    } else if (m.mu_solver == GP_MU_TERNARY && K1 == 2) {
+      const double DET = dcdmu[0][0] * dcdmu[K1 - 1][K1 - 1] - dcdmu[0][K1 - 1] * dcdmu[K1 - 1][0];
+      double inv[2][2];
+      const double yd = 1.0 / DET;
+      inv[0][0] = quot(dcdmu[K1 - 1][K1 - 1], DET, yd);
+      inv[1][1] = quot(dcdmu[0][0], DET, yd);
+      inv[0][1] = quot(-dcdmu[0][K1 - 1], DET, yd);
+      inv[1][0] = quot(-dcdmu[K1 - 1][0], DET, yd);
+#pragma unroll
+      for (int k = 0; k < K1; k++) {
+        double dm = 0.0;
+#pragma unroll
+        for (int l = 0; l < K1; l++) dm += inv[k & 1][l & 1] * deltac[l];
+        mnew[k] = dm + Mc[k];
+      }
+    } else if (m.mu_solver == GP_MU_DILUTE) {
+#pragma unroll
+      for (int k = 0; k < K1; k++) {
+        const double iv = 1.0 / dcdmu[k][k];
+        mnew[k] = Mc[k] + deltac[k] * iv;
+      }
+    } else {
+      double inv[K1][K1];
+      lu_inverse<K1>(dcdmu, inv);
+#pragma unroll
+      for (int k = 0; k < K1; k++) {
+        double s = 0;
+#pragma unroll
+        for (int l = 0; l < K1; l++) s = s + inv[k][l] * deltac[l];
+        mnew[k] = s + Mc[k];
+      }
+    }
+  }
+}
+
 // mu and phi update of the interior.  SMOOTH: the smoothing pre-step
 // (calculate_divergence_concentration.h:154-253): no antitrapping current, no
 // dh/dt source, the LU inverse (matinvnew) for every mu solve.
@@ -840,136 +1040,608 @@ __global__ void __launch_bounds__(256, GP_F64_BLOCKS(N, K1)) k_update(const __gr
   }
 
   const double* ph = P[1][1];
-  double sum[K1], divflux[K1], divjat[K1], deltac[K1], dcdmu[K1][K1];
-#pragma unroll
-  for (int k = 0; k < K1; k++) {
-    sum[k] = 0.0;
-#pragma unroll
-    for (int l = 0; l < K1; l++) dcdmu[k][l] = 0.0;
-  }
-#pragma unroll
-  for (int a = 0; a < N; a++) {
-    double sdh = 0.0;
-#pragma unroll
-    for (int b = 0; b < N; b++) sdh += dhphi<N>(ph, a, b) * Dc[b];
-#pragma unroll
-    for (int k = 0; k < K1; k++) sum[k] += c_mu<K1>(m, thc, Mc, a, k) * sdh;
-  }
-  const double jscale = m.obstacle ? m.jat_obst : m.jat_well;
-#pragma unroll
-  for (int k = 0; k < K1; k++) {
-    divflux[k] = 0.0;
-#pragma unroll
-    for (int l = 0; l < K1; l++) {
-      const double Dcc = Dcell<N, K1>(m, ph, k, l);
-      const double Dx = (Dcell<N, K1>(m, P[2][1], k, l) + Dcc) * 0.5;
-      const double Dxb = (Dcc + Dcell<N, K1>(m, P[0][1], k, l)) * 0.5;
-      const double Dy = (Dcell<N, K1>(m, P[1][2], k, l) + Dcc) * 0.5;
-      const double Dyl = (Dcc + Dcell<N, K1>(m, P[1][0], k, l)) * 0.5;
-      const double gmx = gp_ddiv((Mf[l] - Mc[l]), m.dx);
-      const double gmxb = gp_ddiv((Mc[l] - Mb[l]), m.dx);
-      const double gmy = gp_ddiv((Mr[l] - Mc[l]), m.dy);
-      const double gmyl = gp_ddiv((Mc[l] - Ml[l]), m.dy);
-      divflux[k] += gp_ddiv((Dx * gmx - Dxb * gmxb), m.dx);
-      divflux[k] += gp_ddiv((Dy * gmy - Dyl * gmyl), m.dy);
-    }
-    if (!SMOOTH) {
-      divjat[k] = gp_ddiv((jx_c[k] - jx_b[k]) * (jscale), m.dx);
-      divjat[k] += gp_ddiv((jy_c[k] - jy_l[k]) * (jscale), m.dy);
-    }
-  }
-  int bulk = -1;
-#pragma unroll
-  for (int a = 0; a < N; a++)
-    if (bulk < 0 && ph[a] == 1.0) bulk = a;
   double mnew[K1];
-  if (bulk >= 0) {
-    double cnew[K1];
-#pragma unroll
-    for (int k = 0; k < K1; k++) {
-      double co = 0.0;
-#pragma unroll
-      for (int a = 0; a < N; a++)
-        if (a == bulk) co = c_mu<K1>(m, thc, Mc, a, k);
-      cnew[k] = SMOOTH ? co + m.dt * (divflux[k]) : co + m.dt * (divflux[k]) - divjat[k];
-    }
-#pragma unroll
-    for (int k = 0; k < K1; k++) {
-      double v = 0.0;
-#pragma unroll
-      for (int a = 0; a < N; a++)
-        if (a == bulk) v = Mu<K1>(m, thc, cnew, a, k);
-      mnew[k] = v;
-    }
-  } else if (SMOOTH) {
-#pragma unroll
-    for (int k = 0; k < K1; k++) {
-      deltac[k] = m.dt * (divflux[k]);
-#pragma unroll
-      for (int l = 0; l < K1; l++)
-#pragma unroll
-        for (int a = 0; a < N; a++) dcdmu[k][l] += m.cmu[a][k][l] * hphi<N>(ph, a);
-    }
-    double inv[K1][K1];
-    lu_inverse<K1>(dcdmu, inv);
-#pragma unroll
-    for (int k = 0; k < K1; k++) {
-      double s = 0;
-#pragma unroll
-      for (int l = 0; l < K1; l++) s = s + inv[k][l] * deltac[l];
-      mnew[k] = s + Mc[k];
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < K1; k++) {
-      deltac[k] = m.dt * (divflux[k]) - divjat[k] - sum[k];
-#pragma unroll
-      for (int l = 0; l < K1; l++)
-#pragma unroll
-        for (int a = 0; a < N; a++) dcdmu[k][l] += m.cmu[a][k][l] * hphi<N>(ph, a);
-    }
-#pragma unroll
-    for (int k = 0; k < K1; k++) mnew[k] = Mc[k];
-    if (m.mu_solver == GP_MU_BINARY) {
-      const double iv = 1.0 / dcdmu[0][0];
-      mnew[0] = Mc[0] + deltac[0] * iv;
-    } else if (m.mu_solver == GP_MU_TERNARY && K1 == 2) {
-      const double DET = dcdmu[0][0] * dcdmu[K1 - 1][K1 - 1] - dcdmu[0][K1 - 1] * dcdmu[K1 - 1][0];
-      double inv[2][2];
-      inv[0][0] = dcdmu[K1 - 1][K1 - 1] / DET;
-      inv[1][1] = dcdmu[0][0] / DET;
-      inv[0][1] = -dcdmu[0][K1 - 1] / DET;
-      inv[1][0] = -dcdmu[K1 - 1][0] / DET;
-#pragma unroll
-      for (int k = 0; k < K1; k++) {
-        double dm = 0.0;
-#pragma unroll
-        for (int l = 0; l < K1; l++) dm += inv[k & 1][l & 1] * deltac[l];
-        mnew[k] = dm + Mc[k];
-      }
-    } else if (m.mu_solver == GP_MU_DILUTE) {
-#pragma unroll
-      for (int k = 0; k < K1; k++) {
-        const double iv = 1.0 / dcdmu[k][k];
-        mnew[k] = Mc[k] + deltac[k] * iv;
-      }
-    } else {
-      double inv[K1][K1];
-      lu_inverse<K1>(dcdmu, inv);
-#pragma unroll
-      for (int k = 0; k < K1; k++) {
-        double s = 0;
-#pragma unroll
-        for (int l = 0; l < K1; l++) s = s + inv[k][l] * deltac[l];
-        mnew[k] = s + Mc[k];
-      }
-    }
-  }
+  cell_update<N, K1, SMOOTH>(m, DivSpacing{m.dx, m.dy}, thc, ph, P[0][1], P[2][1], P[1][0], P[1][2], Mc, Mb, Mf, Ml, Mr, Dc, jx_c, jx_b, jy_c,
+                             jy_l, mnew);
   const int64_t o = (int64_t)x * g.pitch + y;
 #pragma unroll
   for (int k = 0; k < K1; k++) mu_out[o + k * g.plane] = mnew[k];
 #pragma unroll
   for (int a = 0; a < N; a++) phi_out[o + a * g.plane] = ph[a] + Dc[a];
+}
+
+// ---------------------------------------------------------------- the tile kernel
+
+// Constants of the tile kernel folded on the host (IEEE, the kernels' operation order).
+struct C64 {
+  double ix, iy, i2y;                       // exact reciprocals of dx, dy, 2 dy (powers of two)
+  double atf[GP_MAX_PHASES][GP_MAX_K1];     // 1 - Diff_a / Diff_liquid
+  double Dp[GP_MAX_PHASES][GP_MAX_K1][GP_MAX_K1];  // mobility of the pure phase (Dcell of its one-hot phi)
+};
+
+// A tile of 8 x 16 cells, two threads per cell.  Shared memory, in doubles.
+template <int N, int K1>
+struct T64 {
+  static constexpr int TX = 8, TY = 16, NT = 2 * TX * TY;
+  static constexpr int X1 = TX + 2, Y1 = TY + 2, X2 = TX + 4, Y2 = TY + 4;  // tile +- 1 (ring), +- 2
+  static constexpr int P = N * (N - 1) / 2;
+  static constexpr int FX = (TX + 3) * Y1, NF = FX + X1 * (TY + 3);   // x-, all faces of the ring's cells
+  static constexpr int JX = (TX + 1) * TY, NJ = JX + TX * (TY + 1);   // x-, all faces of the tile's cells
+  static constexpr int o_phi = 0;                    // [N][X2][Y2]
+  static constexpr int o_mu = o_phi + N * X2 * Y2;   // [K1][X1][Y1]
+  static constexpr int o_dp = o_mu + K1 * X1 * Y1;   // [N][X1][Y1] lambda, then Delta-phi
+  static constexpr int o_face = o_dp + N * X1 * Y1;  // [P][2][NF] gradient-energy face terms, then
+  static constexpr int n_cur = K1 * NJ + (N - 1) * X1 * Y1;  // antitrapping currents [K1][NJ], s(phi) [N-1][X1][Y1]
+  static constexpr int total = o_face + (2 * P * NF > n_cur ? 2 * P * NF : n_cur);
+  static constexpr size_t bytes = total * sizeof(double);
+  static constexpr int unroll = N <= 4 ? N : 1;
+  static constexpr int blocks = N <= 4 ? 2 : 1;  // resident blocks per SM asked of the compiler
+};
+
+// asynchronous 8-byte copy to shared memory (cp.async), complete after cp.async.wait_all
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void pair_of(int p, int& a, int& b) {  // pairs a < b in the order (0,1), (0,2), ...
+  a = 0;
+  while (p >= N - 1 - a) p -= N - 1 - a++;
+  b = a + 1 + p;
+}
+template <int N>
+__device__ __forceinline__ int pair_index(int a, int b) { return a * N - a * (a + 1) / 2 + (b - a - 1); }
+
+// New mu of a bulk cell of phase b all of whose neighbours hold the one-hot phi of b: what cell_update
+// yields there (no current, face mobility (D + D) / 2).  u: centre, x-, x+, y-, y+.
+template <int N, int K1>
+__device__ __forceinline__ void pure_cell(const gp_model& m, const C64& c64, Th th, int b, const double (&u)[5][K1],
+                                          double (&mnew)[K1]) {
+  const double ix = c64.ix, iy = c64.iy, jscale = m.obstacle ? m.jat_obst : m.jat_well;
+  double cnew[K1];
+#pragma unroll
+  for (int k = 0; k < K1; k++) {
+    double divflux = 0.0;
+#pragma unroll
+    for (int l = 0; l < K1; l++) {
+      const double D = c64.Dp[b][k][l], Dx = (D + D) * 0.5;
+      const double gmx = (u[2][l] - u[0][l]) * ix, gmxb = (u[0][l] - u[1][l]) * ix;
+      const double gmy = (u[4][l] - u[0][l]) * iy, gmyl = (u[0][l] - u[3][l]) * iy;
+      divflux += (Dx * gmx - Dx * gmxb) * ix;
+      divflux += (Dx * gmy - Dx * gmyl) * iy;
+    }
+    double divjat = ((0.0 - 0.0) * (jscale)) * ix;
+    divjat += ((0.0 - 0.0) * (jscale)) * iy;
+    cnew[k] = c_mu<K1>(m, th, u[0], b, k) + m.dt * (divflux)-divjat;
+  }
+#pragma unroll
+  for (int k = 0; k < K1; k++) mnew[k] = Mu<K1>(m, th, cnew, b, k);
+}
+
+// The step of the tiles that lean_phase accepts: they hold the one-hot field of one phase on their
+// cells and the two rings a step reads, so Delta-phi is +0, no face carries an antitrapping current
+// and every cell is bulk: mu alone moves, and phi is written only where the output buffer does not
+// hold that field yet (its purity word says so).  The other tiles are listed for k_step64.
+// A warp per tile, two cells of two rows per lane (16-byte loads).  win, wout: purity words of the
+// input and the output buffer (gp_tiles.cuh); cnt[0] counts the list.
+// Bound by latency: tile facts, nine words and mu are a chain of three loads, and one wave of blocks
+// covers a 1024^2 grid.
+template <int N, int K1>
+__global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64,
+                                                Geo g, const uint32_t* __restrict__ geo,
+                                                const uint32_t* __restrict__ win, uint32_t* __restrict__ wout,
+                                                int ntile, const double* __restrict__ mu, double* __restrict__ phi_out,
+                                                double* __restrict__ mu_out, int* __restrict__ list,
+                                                int* __restrict__ cnt) {
+  constexpr int TX = T64<N, K1>::TX, TY = T64<N, K1>::TY;
+  // the list's reader may be scheduled now; it waits for this kernel's end.  This kernel itself was
+  // scheduled while the previous step ran and reads nothing before that has ended.
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= ntile) return;
+  const uint32_t tg = geo[t];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const int b = lean_phase(win, tg, t);
+  if (b < 0) {
+    if (lane == 0) list[atomicAdd(cnt, 1)] = t;
+    return;
+  }
+  const bool write_phi = pf(wout[t], PF_CORE) != 1 + b;
+  const int nty = (g.my + TY - 1) / TY, x0 = (t / nty) * TX, y0 = (t % nty) * TY;
+  const int xr = x0 + (lane >> 3), y = y0 + 2 * (lane & 7);
+  if (x0 > 0 && x0 + TX < g.mx && y0 > 0 && y0 + TY < g.my) {
+    double2 u[2][3][K1];
+    double ul[2][K1], ur[2][K1];
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int k = 0; k < K1; k++) {
+        const double* p = mu + k * g.plane + (int64_t)(xr + 4 * r) * g.pitch + y;
+        u[r][0][k] = __ldg(reinterpret_cast<const double2*>(p));
+        u[r][1][k] = __ldg(reinterpret_cast<const double2*>(p - g.pitch));
+        u[r][2][k] = __ldg(reinterpret_cast<const double2*>(p + g.pitch));
+        ul[r][k] = __ldg(p - 1);
+        ur[r][k] = __ldg(p + 2);
+      }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      double c0[5][K1], c1[5][K1], m0[K1], m1[K1];
+#pragma unroll
+      for (int k = 0; k < K1; k++) {
+        c0[0][k] = u[r][0][k].x; c0[1][k] = u[r][1][k].x; c0[2][k] = u[r][2][k].x; c0[3][k] = ul[r][k]; c0[4][k] = u[r][0][k].y;
+        c1[0][k] = u[r][0][k].y; c1[1][k] = u[r][1][k].y; c1[2][k] = u[r][2][k].y; c1[3][k] = u[r][0][k].x; c1[4][k] = ur[r][k];
+      }
+      pure_cell<N, K1>(m, c64, th_row(m, g, y, false), b, c0, m0);
+      pure_cell<N, K1>(m, c64, th_row(m, g, y + 1, false), b, c1, m1);
+      const int64_t o = (int64_t)(xr + 4 * r) * g.pitch + y;
+#pragma unroll
+      for (int k = 0; k < K1; k++) *reinterpret_cast<double2*>(mu_out + o + k * g.plane) = make_double2(m0[k], m1[k]);
+      if (write_phi) {
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          const double v = a == b ? 1.0 : 0.0;
+          *reinterpret_cast<double2*>(phi_out + o + a * g.plane) = make_double2(v, v);
+        }
+      }
+    }
+  } else {  // a tile at the grid's edge: cell by cell through the boundary map
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {
+      const int x = xr + 4 * (q >> 1), yq = y + (q & 1);
+      if (x >= g.mx || yq >= g.my) continue;
+      double u[5][K1], mnew[K1];
+      load_mu<K1>(mu, g, x, yq, u[0]);
+      load_mu<K1>(mu, g, x - 1, yq, u[1]);
+      load_mu<K1>(mu, g, x + 1, yq, u[2]);
+      load_mu<K1>(mu, g, x, yq - 1, u[3]);
+      load_mu<K1>(mu, g, x, yq + 1, u[4]);
+      pure_cell<N, K1>(m, c64, th_row(m, g, yq, false), b, u, mnew);
+      const int64_t o = (int64_t)x * g.pitch + yq;
+#pragma unroll
+      for (int k = 0; k < K1; k++) mu_out[o + k * g.plane] = mnew[k];
+      if (write_phi) {
+#pragma unroll
+        for (int a = 0; a < N; a++) phi_out[o + a * g.plane] = a == b ? 1.0 : 0.0;
+      }
+    }
+  }
+  __syncwarp();
+  if (lane == 0) wout[t] = pf_all(1 + b);
+}
+
+// The step of the listed tiles (blocks take entries blockIdx.x, + gridDim.x, ...), each through
+// shared memory.
+//
+// What each step of the arithmetic yields is what k_dphi and k_update yield: the same expressions
+// in the same order.  What is evaluated once instead of two or four times: the gradient-energy
+// terms of a face (the front face of one cell is the back face of the next: the same operands in
+// the same order), those of the pairs (a, b) and (b, a) (q, its anisotropy derivative and Q_n only
+// change sign), s(phi) of a cell and a face's antitrapping current.  The host sends models here whose
+// pair constants are symmetric and whose spacings are powers of two (division is a product).
+//
+// Bound by instruction fetch, then latency: a launch holds few interface tiles, each runs the
+// whole chain stage -> flags -> face terms -> lambda -> Delta-phi -> currents -> update once, and
+// warps wait for its code (no_instruction is the first stall reason).  So every phase is one copy of
+// its code: x- and y-faces share a loop through strides, phases and pairs are items spread over the
+// threads or rolled loops, and no division by a spacing is left.  Tiles of 128 cells spread an
+// interface over twice the SMs of 8 x 32 ones.
+template <int N, int K1>
+__global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
+    k_step64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64, Geo g, uint32_t* __restrict__ wout,
+             const double* __restrict__ phi, const double* __restrict__ mu, double* __restrict__ phi_out,
+             double* __restrict__ mu_out, const int* __restrict__ list, const int* __restrict__ cnt,
+             int* __restrict__ next_cnt) {
+  using T = T64<N, K1>;
+  constexpr int TX = T::TX, TY = T::TY, NT = T::NT, X1 = T::X1, Y1 = T::Y1, X2 = T::X2, Y2 = T::Y2;
+  constexpr int R1 = X1 * Y1, R2 = X2 * Y2, FX = T::FX, NF = T::NF, JX = T::JX, NJ = T::NJ, L = N - 1;
+  extern __shared__ __align__(16) double sm64[];
+  double* const sphi = sm64 + T::o_phi;
+  double* const smu = sm64 + T::o_mu;
+  double* const sdp = sm64 + T::o_dp;
+  double* const sface = sm64 + T::o_face;
+  double* const sjat = sface;             // [K1][NJ]
+  double* const ssob = sface + K1 * NJ;   // [N-1][X1][Y1]
+  __shared__ uint8_t s_act[R1], s_cls[TX * TY];
+  __shared__ uint16_t s_list[R1];
+  __shared__ int s_n, s_bad;
+  const int tid = threadIdx.x, lane = tid & 31, ti = tid / TY, tj = tid % TY;
+  const int nty = (g.my + TY - 1) / TY;
+  const double ix = c64.ix, iy = c64.iy, i2y = c64.i2y;
+  const MulSpacing spacing = {ix, iy};
+
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const int ntile = *cnt;
+  if (blockIdx.x == 0 && tid == 0) *next_cnt = 0;  // the next step's list starts empty (read last by the step before)
+  {
+#pragma unroll 1
+    for (int q = blockIdx.x; q < ntile; q += gridDim.x) {
+      const int t = list[q], x0 = (t / nty) * TX, y0 = (t % nty) * TY;
+      __syncthreads();  // the previous tile's shared state has been read
+      if (tid == 0) s_n = s_bad = 0;
+#pragma unroll 1
+      for (int e = tid; e < R2; e += NT) {
+        const int i = e / Y2, j = e % Y2;
+        const double* p = phi + (int64_t)gp_map_any(x0 - 2 + i, g.mx, g.bc.phi_x) * g.pitch + gp_map_any(y0 - 2 + j, g.my, g.bc.phi_y);
+#pragma unroll
+        for (int a = 0; a < N; a++) copy8(sphi + a * R2 + e, p + a * g.plane);
+      }
+#pragma unroll 1
+      for (int e = tid; e < R1; e += NT) {
+        const int i = e / Y1, j = e % Y1;
+        const double* p = mu + (int64_t)gp_map_any(x0 - 1 + i, g.mx, g.bc.mu_x) * g.pitch + gp_map_any(y0 - 1 + j, g.my, g.bc.mu_y);
+#pragma unroll
+        for (int k = 0; k < K1; k++) copy8(smu + k * R1 + e, p + k * g.plane);
+      }
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+
+      // ring cells whose 3x3 phi block is flat (flat_block): Delta-phi +0; the others are listed
+#pragma unroll 1
+      for (int e0 = 0; e0 < R1; e0 += NT) {
+        const int e = e0 + tid;
+        bool act = false;
+        if (e < R1) {
+          const int i = e / Y1, j = e % Y1;
+          if (x0 - 1 + i <= g.mx && y0 - 1 + j <= g.my) {
+            bool flat = true;
+#pragma unroll T::unroll
+            for (int a = 0; a < N; a++) {
+              const double* p = sphi + a * R2 + i * Y2 + j;
+              const double c = p[Y2 + 1];
+              bool f = (c >= 0.0) & (c <= 1.0);
+#pragma unroll
+              for (int di = 0; di < 3; di++)
+#pragma unroll
+                for (int dj = 0; dj < 3; dj++) f &= p[di * Y2 + dj] == c;
+              flat &= f;
+            }
+            act = !flat;
+          }
+          s_act[e] = act;
+#pragma unroll
+          for (int a = 0; a < N; a++) sdp[a * R1 + e] = 0.0;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, act);
+        int base = 0;
+        if (lane == 0 && bal) base = atomicAdd(&s_n, __popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (act) s_list[base + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)e;
+      }
+      __syncthreads();
+      const int nact = s_n;
+
+      // Gradient-energy terms of the faces next to a listed cell, per pair a < b: A = a_c^2 Q_n and
+      // B = a_c |q|^2 (R^-1 da_c/dq)_n (anisotropic), A = Q_n (isotropic); function_A_01.h:101-219.
+      // Face f: x-faces between rows i and i + 1 (of tile +- 2) at column j, then y-faces between
+      // columns j and j + 1 at row i; sn, st: strides along and across its normal.
+#pragma unroll 1
+      for (int e = tid; nact && e < T::P * NF; e += NT) {
+        const int p = T::P == 1 ? 0 : e / NF, f = T::P == 1 ? e : e % NF;
+        const bool xf = f < FX;
+        const int r = xf ? f : f - FX, w = xf ? Y1 : TY + 3;
+        const int i = r / w + (xf ? 0 : 1), j = r % w + (xf ? 1 : 0);
+        const int lo = (i - 1) * Y1 + j - 1, hi = xf ? lo + Y1 : lo + 1;  // the two cells' ring positions
+        const bool in_lo = xf ? i >= 1 : j >= 1, in_hi = xf ? i <= TX + 1 : j <= TY + 1;
+        if (!((in_lo && s_act[lo]) || (in_hi && s_act[hi]))) continue;
+        int a = 0, b = 1;
+        if (N > 2) pair_of<N>(p, a, b);
+        const int sn = xf ? Y2 : 1, st = xf ? 1 : Y2;
+        const double* const pa = sphi + a * R2 + i * Y2 + j;
+        const double* const pb = sphi + b * R2 + i * Y2 + j;
+        const double h = xf ? ix : iy;
+        const double sa = 0.5 * (pa[sn] + pa[0]), sb = 0.5 * (pb[sn] + pb[0]);
+        const double ga = (pa[sn] - pa[0]) * h, gb = (pb[sn] - pb[0]) * h;
+        const double Qn = (sa * gb - sb * ga);
+        double A = Qn, B = 0.0;
+        if (m.anisotropy) {
+          auto tang = [&](const double* v) {
+            return xf ? (v[st] - v[-st]) * i2y : 0.5 * ((v[st] - v[0]) * ix + (v[0] - v[-st]) * ix);
+          };
+          const double Qt = 0.5 * (sa * (tang(pb) + tang(pb + sn)) - sb * (tang(pa) + tang(pa + sn)));
+          double q0, q1, e0, e1, r0, r1;
+          mul2(m.R[a][b], xf ? Qn : Qt, xf ? Qt : Qn, q0, q1);
+          double ac;
+          aniso_both(m.dab[a][b], q0, q1, ac, e0, e1);
+          const double ac2 = ac * ac;
+          mul2(m.Rinv[a][b], e0, e1, r0, r1);
+          const double q2 = q0 * q0 + q1 * q1;
+          A = ac2 * Qn;
+          B = ac * q2 * (xf ? r0 : r1);
+        }
+        sface[(2 * p) * NF + f] = A;
+        sface[(2 * p + 1) * NF + f] = B;
+      }
+      __syncthreads();
+
+      // divphi of phase a at the ring cell whose phi is at p
+      auto div_of = [&](const double* p) {
+        const double c = p[0], gx = (p[Y2] - c) * ix, bgx = (c - p[-Y2]) * ix, gy = (p[1] - c) * iy, lgy = (c - p[-1]) * iy;
+        double d = (gx - bgx) * ix;
+        d += (gy - lgy) * iy;
+        return d;
+      };
+      // lambda of every phase of the listed cells, an item each (calculate_divergence_phasefield.h:4-40)
+#pragma unroll 1
+      for (int it = tid; it < nact * N; it += NT) {
+        const int cell = it / N, a = it - cell * N, e = s_list[cell], i1 = e / Y1, j1 = e % Y1;
+        const double* const pc = sphi + (i1 + 1) * Y2 + j1 + 1;
+        const double* const pp = pc + a * R2;
+        if (!(fabs(div_of(pp)) > 0.0)) continue;  // its lambda stays 0
+        double ph[N], divphi[N];
+#pragma unroll
+        for (int b = 0; b < N; b++) {
+          ph[b] = pc[b * R2];
+          divphi[b] = div_of(pc + b * R2);
+        }
+        const double pa = pp[0];
+        const double cxa = 0.5 * ((pp[Y2] - pa) * ix + (pa - pp[-Y2]) * ix), cya = (pp[1] - pp[-1]) * i2y;
+        // the face terms around the cell: front (back one row before), right (left one before)
+        const double* const fx = sface + (i1 + 1) * Y1 + j1;
+        const double* const fy = sface + FX + i1 * (TY + 3) + j1 + 1;
+        double s1 = 0.0, s2 = 0.0, d1s = 0.0, d2s = 0.0;
+#pragma unroll 1
+        for (int b = 0; b < N; b++) {
+          if (b == a) continue;
+          const double* const pq = pc + b * R2;
+          const double gam = m.Gamma[a][b], pb = pq[0];
+          const double cxb = 0.5 * ((pq[Y2] - pb) * ix + (pb - pq[-Y2]) * ix), cyb = (pq[1] - pq[-1]) * i2y;
+          const double Qcx = (pa * cxb - pb * cxa), Qcy = (pa * cyb - pb * cya);
+          const int o = (a < b ? pair_index<N>(a, b) : pair_index<N>(b, a)) * 2 * NF, oB = o + NF;
+          const double sg = a < b ? 1.0 : -1.0;
+          const double sf = 0.5 * (pq[Y2] + pb), sb = 0.5 * (pb + pq[-Y2]), sr = 0.5 * (pq[1] + pb), sl = 0.5 * (pb + pq[-1]);
+          double e1 = (((sg * fx[o]) * (-sf)) - ((sg * fx[o - Y1]) * (-sb))) * ix;
+          e1 += (((sg * fy[o]) * (-sr)) - ((sg * fy[o - 1]) * (-sl))) * iy;
+          e1 *= gam;
+          d1s += e1;
+          if (!m.anisotropy) {
+            double sp = 0.0;
+            sp += Qcx * cxb;
+            sp += Qcy * cyb;
+            sp *= gam;
+            s1 += sp;
+            continue;
+          }
+          double q0, q1, d0, d1, r0, r1;
+          mul2(m.R[a][b], Qcx, Qcy, q0, q1);
+          double ac1;
+          aniso_both(m.dab[a][b], q0, q1, ac1, d0, d1);
+          const double q2 = (q0 * q0 + q1 * q1);
+          const double ac2 = ac1 * ac1;
+          mul2(m.R[a][b], cxb, cyb, r0, r1);
+          double sp1 = 0.0, sp2 = 0.0;
+          sp1 += q0 * r0;
+          sp1 += q1 * r1;
+          sp2 += (d0)*r0;
+          sp2 += (d1)*r1;
+          sp1 *= gam * ac2;
+          sp2 *= gam * ac1 * q2;
+          s1 += sp1;
+          s2 += sp2;
+          double e2 = ((sg * fx[oB]) * (-sf) - (sg * fx[oB - Y1]) * (-sb)) * ix;
+          e2 += ((sg * fy[oB]) * (-sr) - (sg * fy[oB - 1]) * (-sl)) * iy;
+          e2 *= gam;
+          d2s += e2;
+        }
+        double tt;
+        if (!m.anisotropy) {
+          const double dA = 2.0 * s1, divA = 2.0 * d1s;
+          tt = -dA + divA;
+        } else {
+          const double dA = 2.0 * (s1 + s2), divA = (2.0 * (d1s + d2s) + 0.0);
+          tt = -dA + divA;
+        }
+        double muc[K1], ds = 0.0;
+#pragma unroll
+        for (int k = 0; k < K1; k++) muc[k] = smu[k * R1 + e];
+        const Th th = th_row(m, g, y0 - 1 + j1, g.t_linear);
+#pragma unroll 1
+        for (int b = 0; b < N; b++) {
+          double c[K1];
+          double psi = 0.0;
+#pragma unroll
+          for (int k = 0; k < K1; k++) {
+            c[k] = c_mu<K1>(m, th, muc, b, k);
+            psi -= muc[k] * c[k];
+          }
+          psi += free_energy<N, K1>(m, th, c, b);
+          ds += psi * dhphi<N>(ph, pc[b * R2], pa, b, a);
+        }
+        sdp[a * R1 + e] = m.epsilon * (tt)-m.inv_eps * dwdphi<N>(m, ph, divphi, pa, a) - ds;
+      }
+      __syncthreads();
+      // Delta-phi of the listed cells (calculate_divergence_phasefield.h:41-62, simplex_projection.h:1-49)
+#pragma unroll 1
+      for (int idx = tid; idx < nact; idx += NT) {
+        const int e = s_list[idx];
+        const double* const pc = sphi + (e / Y1 + 1) * Y2 + e % Y1 + 1;
+        double ph[N], divphi[N], lambda[N], dp[N], sum_lambda = 0.0;
+        int active = 0;
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          ph[a] = pc[a * R2];
+          divphi[a] = div_of(pc + a * R2);
+          lambda[a] = sdp[a * R1 + e];
+          if (fabs(divphi[a]) > 0.0) {
+            sum_lambda += lambda[a];
+            active++;
+          }
+        }
+        if (N == 2) sum_lambda = active == 2 ? sum_lambda * 0.5 : sum_lambda;
+        else if (active) sum_lambda = gp_ddiv(sum_lambda, (double)active);
+        const double te = tau_phi<N>(m, ph) * m.epsilon, yte = 1.0 / te;
+#pragma unroll
+        for (int a = 0; a < N; a++) dp[a] = fabs(divphi[a]) > 0.0 ? quot(m.dt * (lambda[a] - sum_lambda), te, yte) : 0.0;
+        project_simplex<N>(ph, divphi, dp);
+#pragma unroll
+        for (int a = 0; a < N; a++) sdp[a * R1 + e] = dp[a];
+      }
+      // s(phi) of the antitrapping term (obstacle), a ring cell and solid phase per item
+      if (m.obstacle) {
+#pragma unroll 1
+        for (int it = tid; nact && it < L * R1; it += NT) {
+          const int a = L == 1 ? 0 : it / R1, e = L == 1 ? it : it % R1;
+          const double* const pc = sphi + (e / Y1 + 1) * Y2 + e % Y1 + 1;
+          double ph[N];
+#pragma unroll
+          for (int b = 0; b < N; b++) ph[b] = pc[b * R2];
+          const double pa = pc[a * R2];
+          double s1 = 0.0, h = 3.0 * pa * pa - 2.0 * pa * pa * pa;  // hphi
+#pragma unroll
+          for (int b = 0; b < N; b++)
+#pragma unroll
+            for (int c = b + 1; c < N; c++)
+              if (b != a && c != a) s1 += ph[b] * ph[c];
+          s1 *= 2.0 * pa;
+          h = h + s1;
+          double s = 0.0;
+          if (pa * (1.0 - pa) > 0.0) s = pa * (1.0 - h) / (sqrt(pa * (1.0 - pa)));
+          ssob[it] = s;
+        }
+      }
+      __syncthreads();
+
+      // antitrapping currents of the tile's faces next to a listed cell (calculate_fluxes_concentration.h:4-145)
+#pragma unroll 1
+      for (int f = tid; nact && f < NJ; f += NT) {
+        const bool xf = f < JX;
+        const int r = xf ? f : f - JX, w = xf ? TY : TY + 1;
+        const int ic = r / w + (xf ? 0 : 1), jc = r % w + (xf ? 1 : 0);  // the lower cell's ring position
+        const int ec = ic * Y1 + jc, en = xf ? ec + Y1 : ec + 1;
+        if (!s_act[ec] && !s_act[en]) continue;
+        const int sn = xf ? Y2 : 1, st = xf ? 1 : Y2;
+        const double* const pc = sphi + (ic + 1) * Y2 + jc + 1;
+        const double h = xf ? ix : iy;
+        auto tang = [&](const double* v) {
+          return xf ? (v[st] - v[-st]) * i2y : 0.5 * ((v[st] - v[0]) * ix + (v[0] - v[-st]) * ix);
+        };
+        const double* const pl = pc + L * R2;
+        const double gl = (pl[sn] - pl[0]) * h;
+        const double tl = 0.5 * (tang(pl) + tang(pl + sn));
+        const double norm_l = sqrt(tl * tl + gl * gl);
+        const int y = y0 - 1 + jc;  // the lower cell's row; the face of ghosted row MESH_Y-2 carries none
+        const bool skip = !xf && ((y + 3 == g.my - 2) || (y + 3 == 0));
+        const Th th_c = th_row(m, g, y, false), th_n = xf ? th_c : th_row(m, g, y + 1, false);
+        double j[K1], uc[K1], un[K1];
+#pragma unroll
+        for (int k = 0; k < K1; k++) {
+          j[k] = 0.0;
+          uc[k] = smu[k * R1 + ec];
+          un[k] = smu[k * R1 + en];
+        }
+#pragma unroll 1
+        for (int a = 0; a < L; a++) {
+          const double* const pa = pc + a * R2;
+          const double ga = (pa[sn] - pa[0]) * h;
+          const double ta = 0.5 * (tang(pa) + tang(pa + sn));
+          const double normg = sqrt(ta * ta + ga * ga);
+          if (normg == 0.0 || skip) continue;
+          double sp = ga * gl;
+          sp += ta * tl;
+          if (norm_l > 0.0) sp /= (norm_l * normg);
+          const double dn = sdp[a * R1 + en], dc = sdp[a * R1 + ec];
+#pragma unroll
+          for (int k = 0; k < K1; k++) {
+            const double cl_n = c_mu<K1>(m, th_n, un, L, k), cl_c = c_mu<K1>(m, th_c, uc, L, k);
+            const double cs_n = c_mu<K1>(m, th_n, un, a, k), cs_c = c_mu<K1>(m, th_c, uc, a, k);
+            const double fk = c64.atf[a][k];
+            double v;
+            if (m.obstacle)
+              v = fk * fabs(sp) * 0.5 * (ssob[a * R1 + en] * (cl_n - cs_n) * dn + ssob[a * R1 + ec] * (cl_c - cs_c) * dc) * ga;
+            else
+              v = fk * fabs(sp) * m.s_well * ((cl_n - cs_n) * dn + (cl_c - cs_c) * dc) * ga;
+            j[k] += v / normg;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < K1; k++) sjat[k * NJ + f] = j[k];
+      }
+      __syncthreads();
+
+      // mu and phi of the tile (calculate_divergence_concentration.h:4-153)
+      const int x = x0 + ti, y = y0 + tj, e = (ti + 1) * Y1 + tj + 1;
+      if (ti < TX && x < g.mx && y < g.my) {
+        const double* const pc = sphi + (ti + 2) * Y2 + tj + 2;
+        double ph[N], phb[N], phf[N], phl[N], phr[N], Dc[N], U0[5][K1], jt[4][K1];
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          ph[a] = pc[a * R2];
+          phb[a] = pc[a * R2 - Y2];
+          phf[a] = pc[a * R2 + Y2];
+          phl[a] = pc[a * R2 - 1];
+          phr[a] = pc[a * R2 + 1];
+          Dc[a] = sdp[a * R1 + e];
+        }
+        const bool act = s_act[e];  // a flat cell carries no current on any face
+        const int fx = ti * TY + tj, fy = JX + ti * (TY + 1) + tj;
+#pragma unroll
+        for (int k = 0; k < K1; k++) {
+          const double* const u = smu + k * R1 + e;
+          U0[0][k] = u[0];
+          U0[1][k] = u[-Y1];
+          U0[2][k] = u[Y1];
+          U0[3][k] = u[-1];
+          U0[4][k] = u[1];
+          const double* const jk = sjat + k * NJ;
+          jt[0][k] = act ? jk[fx + TY] : 0.0;
+          jt[1][k] = act ? jk[fx] : 0.0;
+          jt[2][k] = act ? jk[fy + 1] : 0.0;
+          jt[3][k] = act ? jk[fy] : 0.0;
+        }
+        double mnew[K1];
+        int one = -1;  // a flat cell of one pure phase
+        bool pure = !act;
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          if (ph[a] == 1.0 && one < 0) one = a;
+          else pure = pure && ph[a] == 0.0;
+        }
+        if (pure && one >= 0)
+          pure_cell<N, K1>(m, c64, th_row(m, g, y, false), one, U0, mnew);
+        else
+          cell_update<N, K1, false>(m, spacing, th_row(m, g, y, false), ph, phb, phf, phl, phr, U0[0], U0[1], U0[2], U0[3],
+                                    U0[4], Dc, jt[0], jt[1], jt[2], jt[3], mnew);
+        const int64_t o = (int64_t)x * g.pitch + y;
+#pragma unroll
+        for (int k = 0; k < K1; k++) mu_out[o + k * g.plane] = mnew[k];
+        int hot = -1;
+        bool onehot = true;
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          const double v = ph[a] + Dc[a];
+          phi_out[o + a * g.plane] = v;
+          if (v == 1.0 && hot < 0) hot = a;
+          else if (__double_as_longlong(v) != 0) onehot = false;  // -0 is not the pure field's +0
+        }
+        s_cls[tid] = onehot && hot >= 0 ? (uint8_t)hot : (uint8_t)0xFF;
+      }
+      __syncthreads();
+      // purity word of the output tile (whole tile, first/last two rows, first/last two columns)
+      const int ex = min(TX, g.mx - x0), ey = min(TY, g.my - y0);
+      const int r0 = s_cls[0], rxh = s_cls[(ex - 1) * TY], ryh = s_cls[ey - 1];
+      unsigned bad = 0u;
+      if (ti < ex && tj < ey) {
+        const int v = s_cls[tid];
+        if (v != r0) bad |= (ti < 2 ? 3u : 1u) | (tj < 2 ? 8u : 0u);
+        if (ti >= ex - 2 && v != rxh) bad |= 4u;
+        if (tj >= ey - 2 && v != ryh) bad |= 16u;
+      }
+      bad = __reduce_or_sync(0xffffffffu, bad);
+      if (lane == 0 && bad) atomicOr(&s_bad, (int)bad);
+      __syncthreads();
+      if (tid == 0) {
+        const unsigned B = (unsigned)s_bad;
+        uint32_t w = 0u;
+        if (!(B & 1u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_CORE;
+        if (!(B & 2u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_XLO;
+        if (!(B & 4u) && rxh != 0xFF) w |= (uint32_t)(1 + rxh) << PF_XHI;
+        if (!(B & 8u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_YLO;
+        if (!(B & 16u) && ryh != 0xFF) w |= (uint32_t)(1 + ryh) << PF_YHI;
+        wout[t] = w;
+      }
+    }
+  }
 }
 
 template <int N, int K1, bool SMOOTH>
@@ -987,11 +1659,8 @@ cudaError_t launch_step(const gp_model& m, const Geo& g, const double* phi, cons
 
 }  // namespace
 
-// Host entry used by the C ABI (gp_capi.cu).  Two launches per step.
-cudaError_t gp_f64_step(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane,
-                        const double* phi, const double* mu, double* dphi, double* phi_out, double* mu_out,
-                        cudaStream_t s, bool smooth, const double* ghost_rows, const gp_temp_step* temp) {
-  if (m.nonisothermal && !temp) return cudaErrorInvalidValue;  // the step needs its temperature
+static Geo make_geo(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane, const gp_temp_step* temp,
+                    const double* ghost_rows) {
   Geo g;
   g.noniso = m.nonisothermal ? 1 : 0;
   g.t_linear = temp ? temp->linear : 0;
@@ -1006,15 +1675,188 @@ cudaError_t gp_f64_step(const gp_model& m, int pitch, int64_t plane, int rpitch,
   g.rplane = rplane;
   g.bc = gp_bc_of(m);
   g.gov = ghost_rows;
+  return g;
+}
+
+#define GP_ALL_CASES                                        \
+  GP_CASE(2, 1) GP_CASE(2, 2) GP_CASE(2, 3)                 \
+  GP_CASE(3, 1) GP_CASE(3, 2) GP_CASE(3, 3)                 \
+  GP_CASE(4, 1) GP_CASE(4, 2) GP_CASE(4, 3)                 \
+  GP_CASE(5, 1) GP_CASE(5, 2) GP_CASE(5, 3)                 \
+  GP_CASE(6, 1) GP_CASE(6, 2) GP_CASE(6, 3)
+
+// The tiles of a grid stepped by k_step64: static facts, purity words of the two state buffers.
+struct gp_f64_tiles {
+  C64 c;
+  uint32_t* geo = nullptr;    // [n]
+  uint32_t* words = nullptr;  // [2][n]
+  int* list = nullptr;        // [n] tiles of the current step for k_step64, then its two alternating counts
+  int n = 0, grid = 0;
+};
+
+void gp_f64_tiles_destroy(gp_f64_tiles* t) {
+  if (!t) return;
+  cudaFree(t->geo);
+  cudaFree(t->words);
+  cudaFree(t->list);
+  delete t;
+}
+
+static bool power_of_two(double d) {
+  int e;
+  return frexp(d, &e) == 0.5 && e > -500 && e < 500;
+}
+
+// Whether k_step64 takes the model: it evaluates a pair's terms once for both of its phases, and
+// multiplies by the spacings' reciprocals.
+static bool tile_model(const gp_model& m) {
+  if (!power_of_two(m.dx) || !power_of_two(m.dy)) return false;
+  for (int a = 0; a < m.N; a++)
+    for (int b = a + 1; b < m.N; b++) {
+      if (!(m.Gamma[a][b] == m.Gamma[b][a]) || !(m.dab[a][b] == m.dab[b][a])) return false;
+      for (int i = 0; i < 2; i++)
+        for (int j = 0; j < 2; j++)
+          if (!(m.R[a][b][i][j] == m.R[b][a][i][j]) || !(m.Rinv[a][b][i][j] == m.Rinv[b][a][i][j])) return false;
+    }
+  return true;
+}
+
+// *out stays nullptr for a model the tile kernel does not take.
+cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
+  *out = nullptr;
+  if (!tile_model(m)) return cudaSuccess;
+  constexpr int TX = T64<2, 1>::TX, TY = T64<2, 1>::TY;
+  const int64_t n = ((m.mesh_x + TX - 1) / TX) * ((m.mesh_y + TY - 1) / TY);
+  if (n > INT32_MAX / 8) return cudaSuccess;
+  int dev = 0, sms = 0, occ = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#define GP_CASE(NN, KK)                                                                                           \
+  if (m.N == NN && m.K1 == KK) {                                                                                  \
+    if (e == cudaSuccess)                                                                                         \
+      e = cudaFuncSetAttribute(k_step64<NN, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,                     \
+                               (int)T64<NN, KK>::bytes);                                                          \
+    if (e == cudaSuccess)                                                                                         \
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step64<NN, KK>, T64<NN, KK>::NT, T64<NN, KK>::bytes); \
+  }
+  GP_ALL_CASES
+#undef GP_CASE
+  if (e != cudaSuccess) return e;
+  gp_f64_tiles* t = new gp_f64_tiles();
+  t->n = (int)n;
+  memset(&t->c, 0, sizeof t->c);
+  t->c.ix = 1.0 / m.dx;
+  t->c.iy = 1.0 / m.dy;
+  t->c.i2y = 1.0 / (2.0 * m.dy);
+  for (int a = 0; a < m.N; a++)
+    for (int i = 0; i < m.K1; i++) {
+      t->c.atf[a][i] = (1.0 - m.Diff[a][i][i] / m.Diff[m.N - 1][i][i]);
+      for (int j = 0; j < m.K1; j++) {
+        volatile double s = 0.0;  // each product and sum rounded, as the kernels do
+        for (int b = 0; b < m.N; b++)
+          for (int k = 0; k < m.K1; k++) {
+            volatile double v = m.Diff[b][i][k] * m.cmu[b][k][j];
+            v = v * (a == b ? 1.0 : 0.0);
+            s = s + v;
+          }
+        t->c.Dp[a][i][j] = s;
+      }
+    }
+  const int most = sms * (occ > 0 ? occ : 1);
+  t->grid = t->n < most ? t->n : most;
+  std::vector<uint32_t> geo(t->n);
+  const gp_bc bc = gp_bc_of(m);
+  for (int k = 0; k < t->n; k++) geo[k] = tile_geo((int)m.mesh_x, (int)m.mesh_y, bc, k, TX, TY);
+  e = cudaMalloc(&t->geo, sizeof(uint32_t) * n);
+  if (e == cudaSuccess) e = cudaMemcpy(t->geo, geo.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc(&t->words, 2 * sizeof(uint32_t) * n);
+  if (e == cudaSuccess) e = cudaMemset(t->words, 0, 2 * sizeof(uint32_t) * n);
+  if (e == cudaSuccess) e = cudaMalloc(&t->list, sizeof(int) * (n + 2));
+  if (e == cudaSuccess) e = cudaMemset(t->list + n, 0, 2 * sizeof(int));
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    gp_f64_tiles_destroy(t);
+    return e;
+  }
+  *out = t;
+  return cudaSuccess;
+}
+
+// The buffers' contents changed behind the kernels' back, or a step was taken without them: nothing is
+// known of the tiles, and both list counts start at 0 again (they alternate with the buffers).
+cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s) {
+  if (!t) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(t->words, 0, 2 * sizeof(uint32_t) * (size_t)t->n, s);
+  return e == cudaSuccess ? cudaMemsetAsync(t->list + t->n, 0, 2 * sizeof(int), s) : e;
+}
+
+// Launched as a programmatic dependent of the kernel before it on the stream: its blocks are scheduled
+// while that kernel runs and wait in the kernel (griddepcontrol.wait) for its end.
+template <typename... Params, typename... Args>
+static cudaError_t launch_dependent(void (*fn)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+}
+
+// One step by the tile kernels from buffer parity p into the other: two launches.
+cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
+                              const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
+                              const gp_temp_step* temp) {
+  if (m.nonisothermal && !temp) return cudaErrorInvalidValue;
+  const Geo g = make_geo(m, pitch, plane, 0, 0, temp, nullptr);
+  const uint32_t* win = t->words + (size_t)p * t->n;
+  uint32_t* wout = t->words + (size_t)(p ^ 1) * t->n;
+  int *cnt = t->list + t->n + p, *next = t->list + t->n + (p ^ 1);
+#define GP_CASE(NN, KK)                                                                                              \
+  if (m.N == NN && m.K1 == KK) {                                                                                     \
+    cudaError_t e = launch_dependent(k_lean64<NN, KK>, (t->n + 7) / 8, 256, 0, s, m, t->c, g, t->geo, win, wout,     \
+                                     t->n, mu, phi_out, mu_out, t->list, cnt);                                       \
+    if (e == cudaSuccess)                                                                                            \
+      e = launch_dependent(k_step64<NN, KK>, t->grid, T64<NN, KK>::NT, T64<NN, KK>::bytes, s, m, t->c, g, wout, phi, \
+                           mu, phi_out, mu_out, t->list, cnt, next);                                                 \
+    return e;                                                                                                        \
+  }
+  GP_ALL_CASES
+#undef GP_CASE
+  return cudaErrorInvalidValue;
+}
+
+// Delta-phi of a state into the ring array alone (the tile kernel keeps its own in shared memory).
+cudaError_t gp_f64_dphi(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane, const double* phi,
+                        const double* mu, double* dphi, cudaStream_t s, const gp_temp_step* temp) {
+  if (m.nonisothermal && !temp) return cudaErrorInvalidValue;
+  const Geo g = make_geo(m, pitch, plane, rpitch, rplane, temp, nullptr);
+  const dim3 blk(32, 8), grd((g.my + 2 + 31) / 32, (g.mx + 2 + 7) / 8);
+#define GP_CASE(NN, KK)                                                     \
+  if (m.N == NN && m.K1 == KK) {                                            \
+    k_dphi<NN, KK, false><<<grd, blk, 0, s>>>(m, g, phi, mu, dphi);         \
+    return cudaGetLastError();                                              \
+  }
+  GP_ALL_CASES
+#undef GP_CASE
+  return cudaErrorInvalidValue;
+}
+
+// One step through the ring array: two launches.
+cudaError_t gp_f64_step(const gp_model& m, int pitch, int64_t plane, int rpitch, int64_t rplane,
+                        const double* phi, const double* mu, double* dphi, double* phi_out, double* mu_out,
+                        cudaStream_t s, bool smooth, const double* ghost_rows, const gp_temp_step* temp) {
+  if (m.nonisothermal && !temp) return cudaErrorInvalidValue;  // the step needs its temperature
+  const Geo g = make_geo(m, pitch, plane, rpitch, rplane, temp, ghost_rows);
 #define GP_CASE(NN, KK)                                                                           \
   if (m.N == NN && m.K1 == KK)                                                                    \
     return smooth ? launch_step<NN, KK, true>(m, g, phi, mu, dphi, phi_out, mu_out, s)            \
                   : launch_step<NN, KK, false>(m, g, phi, mu, dphi, phi_out, mu_out, s);
-  GP_CASE(2, 1) GP_CASE(2, 2) GP_CASE(2, 3)
-  GP_CASE(3, 1) GP_CASE(3, 2) GP_CASE(3, 3)
-  GP_CASE(4, 1) GP_CASE(4, 2) GP_CASE(4, 3)
-  GP_CASE(5, 1) GP_CASE(5, 2) GP_CASE(5, 3)
-  GP_CASE(6, 1) GP_CASE(6, 2) GP_CASE(6, 3)
+  GP_ALL_CASES
 #undef GP_CASE
   return cudaErrorInvalidValue;
 }
