@@ -25,6 +25,7 @@
 // Memory: ceil(N / every) + every states (every = ceil(sqrt(N)) by default).
 
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <vector>
@@ -64,19 +65,6 @@ __device__ __forceinline__ int64_t ix_ring(const Geo& g, int x, int y, int a) {
   return a * g.rplane + (int64_t)(x + 1) * g.rpitch + (y + 1);
 }
 
-// x / d; when d is a power of two (dx = dy = 1 in most inputs) the product with its exact
-// reciprocal, which has the same bits as the quotient.
-__device__ __forceinline__ float pdiv(float x, float d) {
-  const int b = __float_as_int(d), e = (b >> 23) & 0xFF;
-  if ((b & 0x807FFFFF) == 0 && e > 1 && e < 253) return x * __int_as_float((254 - e) << 23);
-  return x / d;
-}
-__device__ __forceinline__ double pdiv(double x, double d) {
-  const long long b = __double_as_longlong(d), e = (b >> 52) & 0x7FF;
-  if ((b & 0x800FFFFFFFFFFFFFLL) == 0 && e > 1 && e < 2045) return x * __longlong_as_double((2046LL - e) << 52);
-  return x / d;
-}
-
 template <typename T>
 __device__ __forceinline__ void load_P(const T* st, const Geo& g, int x, int y, T (&P)[3][3][2]) {
 #pragma unroll
@@ -95,26 +83,23 @@ __device__ __forceinline__ bool flat_P(const T (&P)[3][3][2]) {
 #pragma unroll
   for (int a = 0; a < 2; a++) {
     const T c = P[1][1][a];
-    f = f && c >= (T)0 && c <= (T)1;
+    f &= (c >= (T)0) & (c <= (T)1);  // no short circuit: a branch per compare costs more than the compares
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-      for (int j = 0; j < 3; j++) f = f && P[i][j][a] == c;
+      for (int j = 0; j < 3; j++) f &= P[i][j][a] == c;
   }
   return f;
 }
 
 // Face k of interior cell (x, y): 0 = x+, 1 = x-, 2 = y+, 3 = y-; M[5], D[5]:
 // mu and Delta-phi (phase 0) of the cell and its x-, x+, y-, y+ neighbours.
-template <typename T>
-__device__ __forceinline__ Face<T> cell_face(const AM<T>& m, const Geo& g, int y, const T (&P)[3][3][2],
+template <typename T, bool POW2>
+__device__ __forceinline__ Face<T> cell_face(const AM<T, POW2>& m, const Geo& g, int y, const T (&P)[3][3][2],
                                              const T (&M)[5], const T (&D)[5], int k) {
   Face<T> f;
-  const T ty = (T)2 * m.dy;
-  auto cy = [&](int i, int a) { return pdiv(P[i][2][a] - P[i][0][a], ty); };
-  auto cx = [&](int j, int a) {
-    return (T)0.5 * (pdiv(P[2][j][a] - P[1][j][a], m.dx) + pdiv(P[1][j][a] - P[0][j][a], m.dx));
-  };
+  auto cy = [&](int i, int a) { return m.qt(P[i][2][a] - P[i][0][a]); };
+  auto cx = [&](int j, int a) { return (T)0.5 * (m.qx(P[2][j][a] - P[1][j][a]) + m.qx(P[1][j][a] - P[0][j][a])); };
   for (int a = 0; a < 2; a++) {
     if (k == 0) {
       f.pc[a] = P[1][1][a]; f.pn[a] = P[2][1][a]; f.tc[a] = cy(1, a); f.tn[a] = cy(2, a);
@@ -131,17 +116,26 @@ __device__ __forceinline__ Face<T> cell_face(const AM<T>& m, const Geo& g, int y
   f.muc = M[cs]; f.mun = M[ns];
   f.dpc = D[cs]; f.dpn = D[ns];
   f.h = (k >> 1) ? m.dy : m.dx;
+  f.ih = (k >> 1) ? m.iy : m.ix;
   const int ylow = k == 3 ? y - 1 : y;  // the face's lower cell
   f.skip = (k >> 1) && (ylow + 3 == g.my - 2);
   return f;
 }
 
 // the diffusion flux of face k alone (fface on the cell's operands, without the antitrapping ones)
-template <typename T>
-__device__ __forceinline__ T cell_flux(const AM<T>& m, T pc0, T pc1, T pn0, T pn1, T muc, T mun, T h) {
+template <typename T, bool POW2>
+__device__ __forceinline__ T cell_flux(const AM<T, POW2>& m, int dir, T pc0, T pc1, T pn0, T pn1, T muc,
+                                       T mun) {
   const T Dc = m.Ds * m.cmu[0] * pc0 + m.Dl * m.cmu[1] * pc1;
   const T Dn = m.Ds * m.cmu[0] * pn0 + m.Dl * m.cmu[1] * pn1;
-  return (Dn + Dc) * (T)0.5 * pdiv(mun - muc, h);
+  return (Dn + Dc) * (T)0.5 * m.qd(dir, mun - muc);
+}
+
+// Start of a kernel launched as a programmatic dependent of the one before it on the stream: its blocks
+// are scheduled while that one runs; everything it reads waits for that one's end.
+__device__ __forceinline__ void begin_dependent() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 // Block tile of the dense kernels: a cell per thread, y fastest (a warp per tile row).
@@ -170,12 +164,14 @@ __device__ __forceinline__ bool owns_ring(const Geo& g, int x, int y, int i, int
 // Delta-phi -> update.  Cells with a flat block (all but a few percent) skip the phase-field
 // arithmetic; the others are compacted first, so that a warp of the tile does not wait for the few
 // of its lanes that hold an interface.
-template <typename T>
-__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+template <typename T, bool POW2>
+__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
                                             T* __restrict__ out, T* __restrict__ ring, int* __restrict__ list,
                                             int* __restrict__ cnt) {
+  begin_dependent();
   __shared__ T sp[2][X2][Y2], su[X1][Y1], sd[2][X1][Y1];
   __shared__ int s_list[X1 * Y1], s_own[X1 * Y1], s_n, s_m, s_base;
+  __shared__ uint8_t s_act[X1 * Y1];
   int x0, y0;
   tile_origin(g, x0, y0);
   const int tid = threadIdx.x, lane = tid & 31;
@@ -210,6 +206,7 @@ __global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T> m, Geo
         T P[3][3][2];
         block3(i, j, P);
         act = !flat_P(P);
+        s_act[e] = act;
         own = act && ring && owns_ring(g, x, y, i, j);
       }
     }
@@ -252,14 +249,14 @@ __global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T> m, Geo
   block3(i + 1, j + 1, P);
   const T M[5] = {su[i + 1][j + 1], su[i][j + 1], su[i + 2][j + 1], su[i + 1][j], su[i + 1][j + 2]};
   const T ph[2] = {P[1][1][0], P[1][1][1]};
-  F[0] = cell_flux(m, ph[0], ph[1], P[2][1][0], P[2][1][1], M[0], M[2], m.dx);
-  F[1] = cell_flux(m, P[0][1][0], P[0][1][1], ph[0], ph[1], M[1], M[0], m.dx);
-  F[2] = cell_flux(m, ph[0], ph[1], P[1][2][0], P[1][2][1], M[0], M[4], m.dy);
-  F[3] = cell_flux(m, P[1][0][0], P[1][0][1], ph[0], ph[1], M[3], M[0], m.dy);
+  F[0] = cell_flux(m, 0, ph[0], ph[1], P[2][1][0], P[2][1][1], M[0], M[2]);
+  F[1] = cell_flux(m, 0, P[0][1][0], P[0][1][1], ph[0], ph[1], M[1], M[0]);
+  F[2] = cell_flux(m, 1, ph[0], ph[1], P[1][2][0], P[1][2][1], M[0], M[4]);
+  F[3] = cell_flux(m, 1, P[1][0][0], P[1][0][1], ph[0], ph[1], M[3], M[0]);
   const T Dc[2] = {sd[0][i + 1][j + 1], sd[1][i + 1][j + 1]};
 #pragma unroll
   for (int k = 0; k < 4; k++) J[k] = (T)0;
-  if (!flat_P(P)) {
+  if (s_act[(i + 1) * Y1 + j + 1]) {
     const T D[5] = {Dc[0], sd[0][i][j + 1], sd[0][i + 2][j + 1], sd[0][i + 1][j], sd[0][i + 1][j + 2]};
 #pragma unroll
     for (int k = 0; k < 4; k++) J[k] = jface(m, cell_face(m, g, y, P, M, D, k));
@@ -274,8 +271,8 @@ __global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T> m, Geo
 
 // Adjoint of a cell's divflux (gdf) over dt: d mu_new / d c times lambda_mu (mu_new_rev); that of
 // divjat is its negative.
-template <typename T>
-__device__ __forceinline__ T cell_ldc(const AM<T>& m, T p0, T p1, T lmn) {
+template <typename T, bool POW2>
+__device__ __forceinline__ T cell_ldc(const AM<T, POW2>& m, T p0, T p1, T lmn) {
   if (p0 == (T)1) return (T)2 * m.A[0] * lmn;
   if (p1 == (T)1) return (T)2 * m.A[1] * lmn;
   return lmn / (m.cmu[0] * hfun(p0) + m.cmu[1] * hfun(p1));
@@ -302,11 +299,12 @@ __device__ __forceinline__ void block_add(double v, double* slot) {
 // the ghost cell that maps to it).  Writes lam_out and the cell's Delta-phi adjoint (ldphi; 0 on the
 // ghost ring).  part[block] accumulates the D_liquid gradient, each face counted by its lower cell.
 // Bound by its loads: 6 planes in, 5 out, with one synchronisation.
-template <typename T>
-__global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+template <typename T, bool POW2>
+__global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
                                                  const T* __restrict__ ring, const T* __restrict__ lam_in,
                                                  T* __restrict__ lam_out, T* __restrict__ ldphi,
                                                  double* __restrict__ part) {
+  begin_dependent();
   __shared__ T sp[2][X1][Y1], su[X1][Y1], sg[X1][Y1];
   int x0, y0;
   tile_origin(g, x0, y0);
@@ -364,22 +362,22 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T> m
     // the diffusion fluxes: s = +1 where the cell is the face's lower one
     const T k0 = m.Ds * m.cmu[0], k1 = m.Dl * m.cmu[1];
     const T Dme = k0 * ph[0] + k1 * ph[1];
-    auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, T h, bool to_phi, bool to_mu) {
-      const T lF = pdiv(g_lo - g_hi, h), gr = pdiv(mu_hi - mu_lo, h), lD = (T)0.5 * gr * lF;
+    auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, int dir, bool to_phi, bool to_mu) {
+      const T lF = m.qd(dir, g_lo - g_hi), gr = m.qd(dir, mu_hi - mu_lo), lD = (T)0.5 * gr * lF;
       if (to_phi) {
         lph[0] += lD * k0;
         lph[1] += lD * k1;
       }
-      if (to_mu) lmu -= s * pdiv(Dsum * (T)0.5 * lF, h);
+      if (to_mu) lmu -= s * m.qd(dir, Dsum * (T)0.5 * lF);
       return lD;
     };
     const T gme = sg[i][j];
     auto nb = [&](int a, int ii, int jj) { return sp[a][ii][jj]; };
     auto Dnb = [&](int ii, int jj) { return k0 * nb(0, ii, jj) + k1 * nb(1, ii, jj); };
-    const T a0 = gather((T)1, gme, sg[i + 1][j], M[0], M[2], Dnb(i + 1, j) + Dme, m.dx, true, true);
-    const T a1 = gather((T)-1, sg[i - 1][j], gme, M[1], M[0], Dme + Dnb(i - 1, j), m.dx, true, true);
-    const T a2 = gather((T)1, gme, sg[i][j + 1], M[0], M[4], Dnb(i, j + 1) + Dme, m.dy, true, true);
-    const T a3 = gather((T)-1, sg[i][j - 1], gme, M[3], M[0], Dme + Dnb(i, j - 1), m.dy, true, true);
+    const T a0 = gather((T)1, gme, sg[i + 1][j], M[0], M[2], Dnb(i + 1, j) + Dme, 0, true, true);
+    const T a1 = gather((T)-1, sg[i - 1][j], gme, M[1], M[0], Dme + Dnb(i - 1, j), 0, true, true);
+    const T a2 = gather((T)1, gme, sg[i][j + 1], M[0], M[4], Dnb(i, j + 1) + Dme, 1, true, true);
+    const T a3 = gather((T)-1, sg[i][j - 1], gme, M[3], M[0], Dme + Dnb(i, j - 1), 1, true, true);
     dl += (double)(a0 * m.cmu[1] * (ph[1] + nb(1, i + 1, j))) + (double)(a2 * m.cmu[1] * (ph[1] + nb(1, i, j + 1)));
     if (x == 0) dl += (double)(a1 * m.cmu[1] * (nb(1, i - 1, j) + ph[1]));
     if (y == 0) dl += (double)(a3 * m.cmu[1] * (nb(1, i, j - 1) + ph[1]));
@@ -393,9 +391,9 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T> m
       const T v0 = ld_phi(st, g, vx, vy, 0), v1 = ld_phi(st, g, vx, vy, 1);
       const T ge = cell_ldc(m, e0, e1, lmu_in[(int64_t)ex * g.pitch + ey]) * m.dt;
       const T ue = st[2 * g.plane + (int64_t)ex * g.pitch + ey], uv = ld_mu(st, g, vx, vy);
-      const T Ds2 = (k0 * v0 + k1 * v1) + (k0 * e0 + k1 * e1), h = along_x ? m.dx : m.dy;
-      if (low) gather((T)1, (T)0, ge, uv, ue, Ds2, h, mp == own, mm == own);
-      else gather((T)-1, ge, (T)0, ue, uv, Ds2, h, mp == own, mm == own);
+      const T Ds2 = (k0 * v0 + k1 * v1) + (k0 * e0 + k1 * e1);
+      if (low) gather((T)1, (T)0, ge, uv, ue, Ds2, along_x ? 0 : 1, mp == own, mm == own);
+      else gather((T)-1, ge, (T)0, ue, uv, Ds2, along_x ? 0 : 1, mp == own, mm == own);
     };
     if (x <= 2 || x >= g.mx - 3) {
       ghost(true, true);
@@ -422,12 +420,13 @@ __device__ __forceinline__ void add_nz(T* p, T v) {
 // cell_face).  A face between two listed cells belongs to its lower one; one whose lower cell is flat
 // to its upper one.  Faces between two flat cells carry no current and no derivative.
 // Bound by latency (a few thousand threads with one dependent chain of square roots and divisions).
-template <typename T>
-__global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+template <typename T, bool POW2>
+__global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
                                                  const T* __restrict__ ring, const T* __restrict__ lam_in,
                                                  T* __restrict__ lam_out, T* __restrict__ ldphi,
                                                  const int* __restrict__ list, const int* __restrict__ cnt,
                                                  double* __restrict__ part) {
+  begin_dependent();
   double dl = 0.0;
   const int n = 4 * *cnt;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -447,28 +446,28 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T> m
     const int xn = dir == 0 ? x + 1 : x, yn = dir == 0 ? y : y + 1;
     const T h = dir == 0 ? m.dx : m.dy;
     Face<T> f;
-    const T ty = (T)2 * m.dy;
     for (int a = 0; a < 2; a++) {
       f.pc[a] = ld_phi(st, g, x, y, a);
       f.pn[a] = ld_phi(st, g, xn, yn, a);
       if (dir == 0) {
-        f.tc[a] = pdiv(ld_phi(st, g, x, y + 1, a) - ld_phi(st, g, x, y - 1, a), ty);
-        f.tn[a] = pdiv(ld_phi(st, g, xn, y + 1, a) - ld_phi(st, g, xn, y - 1, a), ty);
+        f.tc[a] = m.qt(ld_phi(st, g, x, y + 1, a) - ld_phi(st, g, x, y - 1, a));
+        f.tn[a] = m.qt(ld_phi(st, g, xn, y + 1, a) - ld_phi(st, g, xn, y - 1, a));
       } else {
-        f.tc[a] = (T)0.5 * (pdiv(ld_phi(st, g, x + 1, y, a) - f.pc[a], m.dx) + pdiv(f.pc[a] - ld_phi(st, g, x - 1, y, a), m.dx));
-        f.tn[a] = (T)0.5 * (pdiv(ld_phi(st, g, x + 1, yn, a) - f.pn[a], m.dx) + pdiv(f.pn[a] - ld_phi(st, g, x - 1, yn, a), m.dx));
+        f.tc[a] = (T)0.5 * (m.qx(ld_phi(st, g, x + 1, y, a) - f.pc[a]) + m.qx(f.pc[a] - ld_phi(st, g, x - 1, y, a)));
+        f.tn[a] = (T)0.5 * (m.qx(ld_phi(st, g, x + 1, yn, a) - f.pn[a]) + m.qx(f.pn[a] - ld_phi(st, g, x - 1, yn, a)));
       }
     }
     T lc = (T)0, ln = (T)0;  // the two cells' divjat adjoints
     if (x >= 0 && y >= 0) lc = -cell_ldc(m, f.pc[0], f.pc[1], lam_in[2 * g.plane + (int64_t)x * g.pitch + y]);
     if (xn < g.mx && yn < g.my) ln = -cell_ldc(m, f.pn[0], f.pn[1], lam_in[2 * g.plane + (int64_t)xn * g.pitch + yn]);
-    const T lJ = pdiv((lc - ln) * m.jscale, h);
+    const T lJ = m.qd(dir, (lc - ln) * m.jscale);
     if (lJ == (T)0) continue;
     f.muc = ld_mu(st, g, x, y);
     f.mun = ld_mu(st, g, xn, yn);
     f.dpc = ring[ix_ring(g, x, y, 0)];
     f.dpn = ring[ix_ring(g, xn, yn, 0)];
     f.h = h;
+    f.ih = dir == 0 ? m.ix : m.iy;
     f.skip = dir == 1 && (y + 3 == g.my - 2);
     FaceAdj<T> L = {};
     T lp[NPARAM] = {(T)0, (T)0, (T)0, (T)0};
@@ -478,13 +477,13 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T> m
       add_nz(lam_out + ix_phi(g, x, y, a), L.pc[a]);
       add_nz(lam_out + ix_phi(g, xn, yn, a), L.pn[a]);
       if (dir == 0) {
-        const T hc = pdiv(L.tc[a], ty), hn = pdiv(L.tn[a], ty);
+        const T hc = m.qt(L.tc[a]), hn = m.qt(L.tn[a]);
         add_nz(lam_out + ix_phi(g, x, y + 1, a), hc);
         add_nz(lam_out + ix_phi(g, x, y - 1, a), -hc);
         add_nz(lam_out + ix_phi(g, xn, y + 1, a), hn);
         add_nz(lam_out + ix_phi(g, xn, y - 1, a), -hn);
       } else {
-        const T hc = pdiv((T)0.5 * L.tc[a], m.dx), hn = pdiv((T)0.5 * L.tn[a], m.dx);
+        const T hc = m.qx((T)0.5 * L.tc[a]), hn = m.qx((T)0.5 * L.tn[a]);
         add_nz(lam_out + ix_phi(g, x + 1, y, a), hc);
         add_nz(lam_out + ix_phi(g, x - 1, y, a), -hc);
         add_nz(lam_out + ix_phi(g, x + 1, yn, a), hn);
@@ -504,16 +503,16 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T> m
 // centre and the projection are evaluated by all eight, and lanes 0 and 1 of each phase scatter the
 // centre's contributions with their faces'.  One thread per cell is a chain of twenty a_c(q)
 // evaluations with their reverses on a few thousand threads, far too few to hide it.
-template <typename T>
-__global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> m, Geo g, const T* __restrict__ st,
+template <typename T, bool POW2>
+__global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
                                                   const T* __restrict__ ldphi, T* __restrict__ lam_out,
                                                   const int* __restrict__ list, const int* __restrict__ cnt,
                                                   double* __restrict__ part) {
+  begin_dependent();
   constexpr unsigned ALL = 0xffffffffu;
   double acc[3] = {0.0, 0.0, 0.0};  // mobility, delta, gamma
   const int lane = threadIdx.x & 31, sub = lane & 7, a = sub >> 2, k = sub & 3, dir = k >> 1;
   const int n = *cnt, warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const T ty = (T)2 * m.dy, h = dir ? m.dy : m.dx;
   for (int base = 4 * warp; base < n; base += 4 * warps) {
     const int q = base + (lane >> 3);
     const int o = list[q < n ? q : n - 1], x = o / g.rpitch - 1, y = o % g.rpitch - 1;
@@ -528,11 +527,11 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> 
     bool act[2];
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      const T gx = pdiv(P[2][1][p] - P[1][1][p], m.dx), bgx = pdiv(P[1][1][p] - P[0][1][p], m.dx);
-      const T gy = pdiv(P[1][2][p] - P[1][1][p], m.dy), lgy = pdiv(P[1][1][p] - P[1][0][p], m.dy);
+      const T gx = m.qx(P[2][1][p] - P[1][1][p]), bgx = m.qx(P[1][1][p] - P[0][1][p]);
+      const T gy = m.qy(P[1][2][p] - P[1][1][p]), lgy = m.qy(P[1][1][p] - P[1][0][p]);
       cx[p] = (T)0.5 * (gx + bgx);
-      cy[p] = pdiv(P[1][2][p] - P[1][0][p], ty);
-      act[p] = fabs(pdiv(gx - bgx, m.dx) + pdiv(gy - lgy, m.dy)) > (T)0;
+      cy[p] = m.qt(P[1][2][p] - P[1][0][p]);
+      act[p] = fabs(m.qx(gx - bgx) + m.qy(gy - lgy)) > (T)0;
     }
     on = on && (act[0] || act[1]);  // no active phase: Delta-phi is 0 whatever the inputs
     // the lane's face: f[n][t] along its normal (n = 0 lower, 1 upper cell) and tangent (t = 0 .. 2)
@@ -546,12 +545,12 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> 
         for (int t = 0; t < 3; t++)
           f[nn][t] = dir == 0 ? (k == 0 ? P[1 + nn][t][p] : P[nn][t][p]) : (k == 2 ? P[t][1 + nn][p] : P[t][nn][p]);
       s[p] = (T)0.5 * (f[1][1] + f[0][1]);
-      gn[p] = pdiv(f[1][1] - f[0][1], h);
+      gn[p] = m.qd(dir, f[1][1] - f[0][1]);
       T tt[2];
 #pragma unroll
       for (int nn = 0; nn < 2; nn++)
-        tt[nn] = dir == 0 ? pdiv(f[nn][2] - f[nn][0], ty)
-                          : (T)0.5 * (pdiv(f[nn][2] - f[nn][1], m.dx) + pdiv(f[nn][1] - f[nn][0], m.dx));
+        tt[nn] = dir == 0 ? m.qt(f[nn][2] - f[nn][0])
+                          : (T)0.5 * (m.qx(f[nn][2] - f[nn][1]) + m.qx(f[nn][1] - f[nn][0]));
       tg[p] = tt[0] + tt[1];
     }
     const T sa = a ? s[1] : s[0], sb = a ? s[0] : s[1], ga = a ? gn[1] : gn[0], gb = a ? gn[0] : gn[1];
@@ -562,7 +561,7 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> 
     const T Qn = sa * gb - sb * ga, Qt = (T)0.5 * (sa * tb - sb * ta);
     const T Qx = dir ? Qt : Qn, Qy = dir ? Qn : Qt;
     const T sg = (k & 1) ? (T)-1 : (T)1;
-    T sum4 = sg * pdiv(face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir), h);
+    T sum4 = sg * m.qd(dir, face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir));
     sum4 += __shfl_xor_sync(ALL, sum4, 1);
     sum4 += __shfl_xor_sync(ALL, sum4, 2);
     // the centre term (tterm)
@@ -597,7 +596,7 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> 
     // the face's reverse
     const T lt = m.eps * la;
     T lQx = (T)0, lQy = (T)0, lS = (T)0, ldab = (T)0, lgam = (T)0, lmu = (T)0;
-    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir, pdiv((T)2 * m.gam * sg, h) * lt, lQx, lQy, lS, ldab);
+    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir, m.qd(dir, (T)2 * m.gam * sg) * lt, lQx, lQy, lS, ldab);
     const T lQn = dir ? lQy : lQx, lQt = dir ? lQx : lQy;
     const T lsa = lQn * gb + (T)0.5 * lQt * tb, lsb = -lQn * ga - (T)0.5 * lQt * ta + lS;
     const T lga = -lQn * sb, lgb = lQn * sa, lta = -(T)0.5 * lQt * sb, ltb = (T)0.5 * lQt * sa;
@@ -653,10 +652,10 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T> 
     T mine[2][3], other[2][3];
 #pragma unroll
     for (int w = 0; w < 2; w++) {
-      const T lg = pdiv(w ? lgb : lga, h), ls = (T)0.5 * (w ? lsb : lsa), lT = w ? ltb : lta;
-      const T tv = dir == 0 ? pdiv(lT, ty) : pdiv((T)0.5 * lT, m.dx);
+      const T lg = m.qd(dir, w ? lgb : lga), ls = (T)0.5 * (w ? lsb : lsa), lT = w ? ltb : lta;
+      const T tv = dir == 0 ? m.qt(lT) : m.qx((T)0.5 * lT);
       T v[2][3] = {{-tv, ls - lg, tv}, {-tv, ls + lg, tv}};
-      const T hx = pdiv((T)0.5 * (w ? lcxb : lcxa), m.dx), hy = pdiv(w ? lcyb : lcya, ty);
+      const T hx = m.qx((T)0.5 * (w ? lcxb : lcxa)), hy = m.qt(w ? lcyb : lcya);
       if (k == 0) {  // rows x, x + 1: the centre and its x+, y-, y+ neighbours
         v[0][1] += w ? lpb : lpa;
         v[1][1] += hx;
@@ -715,9 +714,9 @@ __global__ void __launch_bounds__(256) k_fields(T* __restrict__ st, double* __re
 
 // ------------------------------------------------------------------ host side
 
-template <typename T>
-AM<T> make_am(const gp_model& g) {
-  AM<T> m;
+template <typename T, bool POW2>
+AM<T, POW2> make_am(const gp_model& g) {
+  AM<T, POW2> m;
   m.dx = (T)g.dx;
   m.dy = (T)g.dy;
   m.dt = (T)g.dt;
@@ -747,7 +746,24 @@ AM<T> make_am(const gp_model& g) {
   m.Dl = (T)g.Diff[1][0][0];
   m.obstacle = g.obstacle ? 1 : 0;
   m.skip_row = (int)g.mesh_y - 5;
+  m.ix = (T)1 / m.dx;
+  m.iy = (T)1 / m.dy;
+  m.it = (T)1 / ((T)2 * m.dy);
   return m;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*fn)(Params...), int grid, int threads, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
 }
 
 struct AdjBase {
@@ -770,7 +786,11 @@ struct AdjBase {
 template <typename T>
 struct Adj : AdjBase {
   gp_model gm;
-  AM<T> m;
+  // the spacings' quotients as products where dx and dy are powers of two (a template switch: the list
+  // kernels wait for their instructions, and a division is ten times a product's)
+  AM<T, true> mp;
+  AM<T, false> md;
+  bool pow2 = false;
   Geo g;
   cudaStream_t s = nullptr;
   T *ckpt = nullptr, *seg = nullptr, *cur = nullptr, *nxt = nullptr;
@@ -809,7 +829,8 @@ struct Adj : AdjBase {
 
   int init(const gp_model& model) {
     gm = model;
-    m = make_am<T>(model);
+    mp = make_am<T, true>(model);
+    md = make_am<T, false>(model);
     g.mx = (int)model.mesh_x;
     g.my = (int)model.mesh_y;
     g.pitch = (int)gp_round_up(g.my, 32);
@@ -821,6 +842,8 @@ struct Adj : AdjBase {
       gp_set_error("adjoint: %d x %d cells do not fit", g.mx, g.my);
       return GP_E_NOMEM;
     }
+    int ex, ey;
+    pow2 = frexp(model.dx, &ex) == 0.5 && frexp(model.dy, &ey) == 0.5 && abs(ex) < 60 && abs(ey) < 60;
     int dev = 0, sms = 0;
     ADJ_CUDA(cudaGetDevice(&dev));
     ADJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -840,16 +863,22 @@ struct Adj : AdjBase {
   }
 
   cudaError_t step(const T* in, T* out, T* r = nullptr, int* l = nullptr, int* c = nullptr) {
-    k_fwd<T><<<ntile, NT, 0, s>>>(m, g, in, out, r, l, c);
-    return cudaGetLastError();
+    return pow2 ? launch_dependent(k_fwd<T, true>, ntile, NT, s, mp, g, in, out, r, l, c)
+                : launch_dependent(k_fwd<T, false>, ntile, NT, s, md, g, in, out, r, l, c);
   }
 
   // lin = adjoint of the state after x, lout = adjoint of x; r, l, c: x's Delta-phi, list and its length
   cudaError_t rev_step(const T* x, const T* r, const int* l, const int* c, const T* lin, T* lout) {
-    k_rev_cell<T><<<ntile, NT, 0, s>>>(m, g, x, r, lin, lout, ldphi, part);
-    k_rev_jat<T><<<nlist, 128, 0, s>>>(m, g, x, r, lin, lout, ldphi, l, c, part + ntile);
-    k_rev_dphi<T><<<nlist, 128, 0, s>>>(m, g, x, ldphi, lout, l, c, part + ntile + nlist);
-    return cudaGetLastError();
+    return pow2 ? rev_step(mp, x, r, l, c, lin, lout) : rev_step(md, x, r, l, c, lin, lout);
+  }
+  template <bool POW2>
+  cudaError_t rev_step(const AM<T, POW2>& m, const T* x, const T* r, const int* l, const int* c, const T* lin, T* lout) {
+    cudaError_t e = launch_dependent(k_rev_cell<T, POW2>, ntile, NT, s, m, g, x, r, lin, lout, ldphi, part);
+    if (e == cudaSuccess)
+      e = launch_dependent(k_rev_jat<T, POW2>, nlist, 128, s, m, g, x, r, lin, lout, ldphi, l, c, part + ntile);
+    if (e == cudaSuccess)
+      e = launch_dependent(k_rev_dphi<T, POW2>, nlist, 128, s, m, g, x, ldphi, lout, l, c, part + ntile + nlist);
+    return e;
   }
 
   // Host [planes][mx][my] doubles <-> device [planes][mx][pitch] T, converted on the device through a

@@ -38,7 +38,9 @@ namespace gpadj {
 enum { P_MOB = 0, P_DELTA = 1, P_GAMMA = 2, P_DLIQ = 3, NPARAM = 4 };
 
 // Model constants of one instance, in the working precision T.
-template <typename T>
+// POW2: the spacings are powers of two and quotients by them products with their exact reciprocals
+// (ix, iy, it; the same bits); else divisions, and the reciprocals are not read.
+template <typename T, bool POW2 = false>
 struct AM {
   T dx, dy, dt, eps, inv_eps;
   T mob;             // 1 / tau_ab[0][1]
@@ -52,6 +54,13 @@ struct AM {
   T Ds, Dl;          // Diff of the solid (phase 0) and the liquid (phase 1)
   int obstacle;
   int skip_row;      // interior row whose upper y-face carries no antitrapping current
+  T ix, iy, it;      // 1 / dx, 1 / dy, 1 / (2 dy)
+  GP_HD T qx(T v) const { return POW2 ? v * ix : v / dx; }
+  GP_HD T qy(T v) const { return POW2 ? v * iy : v / dy; }
+  GP_HD T qt(T v) const { return POW2 ? v * it : v / ((T)2 * dy); }
+  GP_HD T qd(int dir, T v) const { return dir ? qy(v) : qx(v); }  // dir: 0 along x, 1 along y
+  template <typename F>
+  GP_HD T qh(const F& f, T v) const { return POW2 ? v * f.ih : v / f.h; }
 };
 
 // ------------------------------------------------------------------ small pieces
@@ -63,17 +72,17 @@ GP_HD T dhfun(T p) { return (T)6 * p * ((T)1 - p); }     // dh_a / dphi_a
 template <typename T>
 GP_HD T d2hfun(T p) { return (T)6 - (T)12 * p; }
 
-template <typename T>
-GP_HD T cmu_of(const AM<T>& m, int a, T mu) { return m.cmu[a] * (mu - m.Beff[a]); }  // c_a(mu)
+template <typename T, bool POW2>
+GP_HD T cmu_of(const AM<T, POW2>& m, int a, T mu) { return m.cmu[a] * (mu - m.Beff[a]); }  // c_a(mu)
 
 // psi_a(mu) = f_a(c) - mu c, c = c_a(mu); and d psi_a / d mu
-template <typename T>
-GP_HD T psi_of(const AM<T>& m, int a, T mu) {
+template <typename T, bool POW2>
+GP_HD T psi_of(const AM<T, POW2>& m, int a, T mu) {
   const T c = cmu_of(m, a, mu);
   return m.A[a] * c * c + m.B[a] * c + m.C[a] - mu * c;
 }
-template <typename T>
-GP_HD T dpsi_dmu(const AM<T>& m, int a, T mu) {
+template <typename T, bool POW2>
+GP_HD T dpsi_dmu(const AM<T, POW2>& m, int a, T mu) {
   const T c = cmu_of(m, a, mu);
   return ((T)2 * m.A[a] * c + m.B[a] - mu) * m.cmu[a] - c;
 }
@@ -142,48 +151,46 @@ struct Grad {
   T gx[2], sx[2], gy[2], sy[2], cy[2], bgx[2], cx[2], bsx[2], bcy[2], fcy[2], lgy[2], lsy[2], lcx[2], rcx[2];
 };
 
-template <typename T>
-GP_HD void grad_fwd(const AM<T>& m, const T (&P)[3][3][2], Grad<T>& G) {
-  const T ty = (T)2 * m.dy;
+template <typename T, bool POW2>
+GP_HD void grad_fwd(const AM<T, POW2>& m, const T (&P)[3][3][2], Grad<T>& G) {
   for (int a = 0; a < 2; a++) {
-    G.gx[a] = (P[2][1][a] - P[1][1][a]) / m.dx;
+    G.gx[a] = m.qx(P[2][1][a] - P[1][1][a]);
     G.sx[a] = (T)0.5 * (P[2][1][a] + P[1][1][a]);
-    G.gy[a] = (P[1][2][a] - P[1][1][a]) / m.dy;
+    G.gy[a] = m.qy(P[1][2][a] - P[1][1][a]);
     G.sy[a] = (T)0.5 * (P[1][2][a] + P[1][1][a]);
-    G.cy[a] = (P[1][2][a] - P[1][0][a]) / ty;
-    G.bgx[a] = (P[1][1][a] - P[0][1][a]) / m.dx;
+    G.cy[a] = m.qt(P[1][2][a] - P[1][0][a]);
+    G.bgx[a] = m.qx(P[1][1][a] - P[0][1][a]);
     G.cx[a] = (T)0.5 * (G.gx[a] + G.bgx[a]);
     G.bsx[a] = (T)0.5 * (P[1][1][a] + P[0][1][a]);
-    G.bcy[a] = (P[0][2][a] - P[0][0][a]) / ty;
-    G.fcy[a] = (P[2][2][a] - P[2][0][a]) / ty;
-    G.lgy[a] = (P[1][1][a] - P[1][0][a]) / m.dy;
+    G.bcy[a] = m.qt(P[0][2][a] - P[0][0][a]);
+    G.fcy[a] = m.qt(P[2][2][a] - P[2][0][a]);
+    G.lgy[a] = m.qy(P[1][1][a] - P[1][0][a]);
     G.lsy[a] = (T)0.5 * (P[1][1][a] + P[1][0][a]);
-    G.lcx[a] = (T)0.5 * ((P[2][0][a] - P[1][0][a]) / m.dx + (P[1][0][a] - P[0][0][a]) / m.dx);
-    G.rcx[a] = (T)0.5 * ((P[2][2][a] - P[1][2][a]) / m.dx + (P[1][2][a] - P[0][2][a]) / m.dx);
+    G.lcx[a] = (T)0.5 * (m.qx(P[2][0][a] - P[1][0][a]) + m.qx(P[1][0][a] - P[0][0][a]));
+    G.rcx[a] = (T)0.5 * (m.qx(P[2][2][a] - P[1][2][a]) + m.qx(P[1][2][a] - P[0][2][a]));
   }
 }
 
 // reverse of grad_fwd: LG holds the adjoints of the record, accumulated into LP
-template <typename T>
-GP_HD void grad_rev(const AM<T>& m, const Grad<T>& LG, T (&LP)[3][3][2]) {
-  const T ty = (T)2 * m.dy;
+template <typename T, bool POW2>
+GP_HD void grad_rev(const AM<T, POW2>& m, const Grad<T>& LG, T (&LP)[3][3][2]) {
   for (int a = 0; a < 2; a++) {
     const T lgx = LG.gx[a] + (T)0.5 * LG.cx[a], lbgx = LG.bgx[a] + (T)0.5 * LG.cx[a];
-    LP[2][1][a] += lgx / m.dx + (T)0.5 * LG.sx[a];
-    LP[1][1][a] += -lgx / m.dx + (T)0.5 * LG.sx[a];
-    LP[1][2][a] += LG.gy[a] / m.dy + (T)0.5 * LG.sy[a];
-    LP[1][1][a] += -LG.gy[a] / m.dy + (T)0.5 * LG.sy[a];
-    LP[1][2][a] += LG.cy[a] / ty;
-    LP[1][0][a] -= LG.cy[a] / ty;
-    LP[1][1][a] += lbgx / m.dx + (T)0.5 * LG.bsx[a];
-    LP[0][1][a] += -lbgx / m.dx + (T)0.5 * LG.bsx[a];
-    LP[0][2][a] += LG.bcy[a] / ty;
-    LP[0][0][a] -= LG.bcy[a] / ty;
-    LP[2][2][a] += LG.fcy[a] / ty;
-    LP[2][0][a] -= LG.fcy[a] / ty;
-    LP[1][1][a] += LG.lgy[a] / m.dy + (T)0.5 * LG.lsy[a];
-    LP[1][0][a] += -LG.lgy[a] / m.dy + (T)0.5 * LG.lsy[a];
-    const T hl = (T)0.5 * LG.lcx[a] / m.dx, hr = (T)0.5 * LG.rcx[a] / m.dx;
+    LP[2][1][a] += m.qx(lgx) + (T)0.5 * LG.sx[a];
+    LP[1][1][a] += m.qx(-lgx) + (T)0.5 * LG.sx[a];
+    LP[1][2][a] += m.qy(LG.gy[a]) + (T)0.5 * LG.sy[a];
+    LP[1][1][a] += m.qy(-LG.gy[a]) + (T)0.5 * LG.sy[a];
+    LP[1][2][a] += m.qt(LG.cy[a]);
+    LP[1][0][a] -= m.qt(LG.cy[a]);
+    LP[1][1][a] += m.qx(lbgx) + (T)0.5 * LG.bsx[a];
+    LP[0][1][a] += m.qx(-lbgx) + (T)0.5 * LG.bsx[a];
+    LP[0][2][a] += m.qt(LG.bcy[a]);
+    LP[0][0][a] -= m.qt(LG.bcy[a]);
+    LP[2][2][a] += m.qt(LG.fcy[a]);
+    LP[2][0][a] -= m.qt(LG.fcy[a]);
+    LP[1][1][a] += m.qy(LG.lgy[a]) + (T)0.5 * LG.lsy[a];
+    LP[1][0][a] += m.qy(-LG.lgy[a]) + (T)0.5 * LG.lsy[a];
+    const T hl = m.qx((T)0.5 * LG.lcx[a]), hr = m.qx((T)0.5 * LG.rcx[a]);
     LP[2][0][a] += hl;
     LP[0][0][a] -= hl;
     LP[2][2][a] += hr;
@@ -301,8 +308,8 @@ GP_HD void face_ops_rev(const Grad<T>& G, int a, int k, T lQx, T lQy, T lS, Grad
 
 // t_a = -dA/dphi_a + div dA/dgrad phi_a for the pair (a, 1-a)
 // (function_A_01.h:4-71, 101-219)
-template <typename T>
-GP_HD T tterm(const AM<T>& m, const Grad<T>& G, const T (&ph)[2], int a) {
+template <typename T, bool POW2>
+GP_HD T tterm(const AM<T, POW2>& m, const Grad<T>& G, const T (&ph)[2], int a) {
   const int b = 1 - a;
   const T v0 = ph[a] * G.cx[b] - ph[b] * G.cx[a], v1 = ph[a] * G.cy[b] - ph[b] * G.cy[a];
   T q0, q1, r0, r1;
@@ -317,14 +324,14 @@ GP_HD T tterm(const AM<T>& m, const Grad<T>& G, const T (&ph)[2], int a) {
     T Qx, Qy, S;
     face_ops(G, a, k, Qx, Qy, S);
     const T V = face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1);
-    const T h = (k >> 1) ? m.dy : m.dx;
-    sum += (k & 1) ? -V / h : V / h;
+    const T W = m.qd(k >> 1, V);
+    sum += (k & 1) ? -W : W;
   }
   return -dA + (T)2 * m.gam * sum;
 }
 
-template <typename T>
-GP_HD void tterm_rev(const AM<T>& m, const Grad<T>& G, const T (&ph)[2], int a, T lam, Grad<T>& LG, T (&lph)[2],
+template <typename T, bool POW2>
+GP_HD void tterm_rev(const AM<T, POW2>& m, const Grad<T>& G, const T (&ph)[2], int a, T lam, Grad<T>& LG, T (&lph)[2],
                      T& ldab, T& lgam) {
   const int b = 1 - a;
   // divA = 2 gam sum_k sign_k V_k / h_k
@@ -332,11 +339,10 @@ GP_HD void tterm_rev(const AM<T>& m, const Grad<T>& G, const T (&ph)[2], int a, 
   for (int k = 0; k < 4; k++) {
     T Qx, Qy, S;
     face_ops(G, a, k, Qx, Qy, S);
-    const T h = (k >> 1) ? m.dy : m.dx;
     const T sg = (k & 1) ? (T)-1 : (T)1;
-    sum += sg * face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1) / h;
+    sum += m.qd(k >> 1, sg * face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1));
     T lQx = 0, lQy = 0, lS = 0;
-    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1, (T)2 * m.gam * sg / h * lam, lQx, lQy, lS, ldab);
+    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1, m.qd(k >> 1, (T)2 * m.gam * sg) * lam, lQx, lQy, lS, ldab);
     face_ops_rev(G, a, k, lQx, lQy, lS, LG);
   }
   lgam += (T)2 * sum * lam;
@@ -451,15 +457,15 @@ GP_HD void proj_rev(const T (&ph)[2], const bool (&act)[2], const Proj& r, T Dsu
 
 // Effective mobility 1/tau(phi) (functionTau.h:1-16 for two phases:
 // tau_ab when phi_0 phi_1 != 0, else tau)
-template <typename T>
-GP_HD T mob_eff(const AM<T>& m, const T (&ph)[2]) {
+template <typename T, bool POW2>
+GP_HD T mob_eff(const AM<T, POW2>& m, const T (&ph)[2]) {
   const T st1 = ph[0] * ph[1];
   return (st1 != (T)0 || st1 != st1) ? m.mob : m.mob / m.tau_ratio;
 }
 
 // obstacle / well derivative w_a (functionW_01.h:6-39, functionW_02.h:4-33)
-template <typename T>
-GP_HD T wfun(const AM<T>& m, const T (&ph)[2], const bool (&act)[2], int a) {
+template <typename T, bool POW2>
+GP_HD T wfun(const AM<T, POW2>& m, const T (&ph)[2], const bool (&act)[2], int a) {
   const int b = 1 - a;
   if (!act[b]) return (T)0;
   if (m.obstacle) return m.wobs * ((ph[a] * ph[b] >= (T)0) ? m.gam : -m.gam) * ph[b];
@@ -468,8 +474,8 @@ GP_HD T wfun(const AM<T>& m, const T (&ph)[2], const bool (&act)[2], int a) {
 
 // Delta-phi of a cell from its 3x3 phi stencil and its mu
 // (calculate_divergence_phasefield.h:4-62)
-template <typename T>
-GP_HD void dphi_fwd(const AM<T>& m, const T (&P)[3][3][2], T mu, T (&dp)[2]) {
+template <typename T, bool POW2>
+GP_HD void dphi_fwd(const AM<T, POW2>& m, const T (&P)[3][3][2], T mu, T (&dp)[2]) {
   Grad<T> G;
   grad_fwd(m, P, G);
   const T ph[2] = {P[1][1][0], P[1][1][1]};
@@ -477,7 +483,7 @@ GP_HD void dphi_fwd(const AM<T>& m, const T (&P)[3][3][2], T mu, T (&dp)[2]) {
   T lam[2], sum = (T)0;
   int cnt = 0;
   for (int a = 0; a < 2; a++) {
-    const T dv = (G.gx[a] - G.bgx[a]) / m.dx + (G.gy[a] - G.lgy[a]) / m.dy;
+    const T dv = m.qx(G.gx[a] - G.bgx[a]) + m.qy(G.gy[a] - G.lgy[a]);
     act[a] = fabs(dv) > (T)0;
   }
   for (int a = 0; a < 2; a++) {
@@ -497,8 +503,8 @@ GP_HD void dphi_fwd(const AM<T>& m, const T (&P)[3][3][2], T mu, T (&dp)[2]) {
 }
 
 // reverse of dphi_fwd: ldp = adjoint of dp; accumulates LP, lmu, lpar
-template <typename T>
-GP_HD void dphi_rev(const AM<T>& m, const T (&P)[3][3][2], T mu, const T (&ldp)[2], T (&LP)[3][3][2], T& lmu,
+template <typename T, bool POW2>
+GP_HD void dphi_rev(const AM<T, POW2>& m, const T (&P)[3][3][2], T mu, const T (&ldp)[2], T (&LP)[3][3][2], T& lmu,
                     T (&lpar)[NPARAM]) {
   Grad<T> G;
   grad_fwd(m, P, G);
@@ -507,7 +513,7 @@ GP_HD void dphi_rev(const AM<T>& m, const T (&P)[3][3][2], T mu, const T (&ldp)[
   T lam[2], sum = (T)0;
   int cnt = 0;
   for (int a = 0; a < 2; a++) {
-    const T dv = (G.gx[a] - G.bgx[a]) / m.dx + (G.gy[a] - G.lgy[a]) / m.dy;
+    const T dv = m.qx(G.gx[a] - G.bgx[a]) + m.qy(G.gy[a] - G.lgy[a]);
     act[a] = fabs(dv) > (T)0;
   }
   for (int a = 0; a < 2; a++) {
@@ -573,6 +579,7 @@ GP_HD void dphi_rev(const AM<T>& m, const T (&P)[3][3][2], T mu, const T (&ldp)[
 template <typename T>
 struct Face {
   T pc[2], pn[2], tc[2], tn[2], muc, mun, dpc, dpn, h;
+  T ih;       // 1 / h, read where AM says that the spacings are powers of two
   bool skip;  // the face carries no antitrapping current
 };
 template <typename T>
@@ -582,22 +589,22 @@ struct FaceAdj {
 
 // diffusion flux D_face (mu_n - mu_c) / h, D_face = (D(phi_n) + D(phi_c)) / 2,
 // D(phi) = sum_b Diff_b cmu_b phi_b (functionD.h:1-16, calculate_gradients.h:132-185)
-template <typename T>
-GP_HD T fface(const AM<T>& m, const Face<T>& f) {
+template <typename T, bool POW2>
+GP_HD T fface(const AM<T, POW2>& m, const Face<T>& f) {
   const T Dc = m.Ds * m.cmu[0] * f.pc[0] + m.Dl * m.cmu[1] * f.pc[1];
   const T Dn = m.Ds * m.cmu[0] * f.pn[0] + m.Dl * m.cmu[1] * f.pn[1];
-  return (Dn + Dc) * (T)0.5 * ((f.mun - f.muc) / f.h);
+  return (Dn + Dc) * (T)0.5 * (m.qh(f, f.mun - f.muc));
 }
 
-template <typename T>
-GP_HD void fface_rev(const AM<T>& m, const Face<T>& f, T lF, FaceAdj<T>& L, T (&lpar)[NPARAM]) {
+template <typename T, bool POW2>
+GP_HD void fface_rev(const AM<T, POW2>& m, const Face<T>& f, T lF, FaceAdj<T>& L, T (&lpar)[NPARAM]) {
   const T Dc = m.Ds * m.cmu[0] * f.pc[0] + m.Dl * m.cmu[1] * f.pc[1];
   const T Dn = m.Ds * m.cmu[0] * f.pn[0] + m.Dl * m.cmu[1] * f.pn[1];
-  const T g = (f.mun - f.muc) / f.h;
+  const T g = m.qh(f, f.mun - f.muc);
   const T lD = (T)0.5 * g * lF;  // adjoint of Dc and of Dn
   const T lg = (Dn + Dc) * (T)0.5 * lF;
-  L.mun += lg / f.h;
-  L.muc -= lg / f.h;
+  L.mun += m.qh(f, lg);
+  L.muc -= m.qh(f, lg);
   L.pc[0] += lD * m.Ds * m.cmu[0];
   L.pn[0] += lD * m.Ds * m.cmu[0];
   L.pc[1] += lD * m.Dl * m.cmu[1];
@@ -622,10 +629,10 @@ GP_HD T dsfun(T p) {
 
 // antitrapping current through the face, solid phase 0 against the liquid
 // (calculate_fluxes_concentration.h:25-141 with N = 2, one component)
-template <typename T>
-GP_HD T jface(const AM<T>& m, const Face<T>& f) {
+template <typename T, bool POW2>
+GP_HD T jface(const AM<T, POW2>& m, const Face<T>& f) {
   if (f.skip) return (T)0;
-  const T gn0 = (f.pn[0] - f.pc[0]) / f.h, gn1 = (f.pn[1] - f.pc[1]) / f.h;
+  const T gn0 = m.qh(f, f.pn[0] - f.pc[0]), gn1 = m.qh(f, f.pn[1] - f.pc[1]);
   const T ta = (T)0.5 * (f.tc[0] + f.tn[0]), tl = (T)0.5 * (f.tc[1] + f.tn[1]);
   const T norm_l = sqrt(tl * tl + gn1 * gn1), normg = sqrt(ta * ta + gn0 * gn0);
   if (normg == (T)0) return (T)0;
@@ -639,10 +646,10 @@ GP_HD T jface(const AM<T>& m, const Face<T>& f) {
   return fa * fabs(sp) * K * gn0 / normg;
 }
 
-template <typename T>
-GP_HD void jface_rev(const AM<T>& m, const Face<T>& f, T lJ, FaceAdj<T>& L, T (&lpar)[NPARAM]) {
+template <typename T, bool POW2>
+GP_HD void jface_rev(const AM<T, POW2>& m, const Face<T>& f, T lJ, FaceAdj<T>& L, T (&lpar)[NPARAM]) {
   if (f.skip) return;
-  const T gn0 = (f.pn[0] - f.pc[0]) / f.h, gn1 = (f.pn[1] - f.pc[1]) / f.h;
+  const T gn0 = m.qh(f, f.pn[0] - f.pc[0]), gn1 = m.qh(f, f.pn[1] - f.pc[1]);
   const T ta = (T)0.5 * (f.tc[0] + f.tn[0]), tl = (T)0.5 * (f.tc[1] + f.tn[1]);
   const T norm_l = sqrt(tl * tl + gn1 * gn1), normg = sqrt(ta * ta + gn0 * gn0);
   if (normg == (T)0) return;
@@ -701,19 +708,19 @@ GP_HD void jface_rev(const AM<T>& m, const Face<T>& f, T lJ, FaceAdj<T>& L, T (&
   L.tn[0] += (T)0.5 * lta;
   L.tc[1] += (T)0.5 * ltl;
   L.tn[1] += (T)0.5 * ltl;
-  L.pn[0] += lgn0 / f.h;
-  L.pc[0] -= lgn0 / f.h;
-  L.pn[1] += lgn1 / f.h;
-  L.pc[1] -= lgn1 / f.h;
+  L.pn[0] += m.qh(f, lgn0);
+  L.pc[0] -= m.qh(f, lgn0);
+  L.pn[1] += m.qh(f, lgn1);
+  L.pc[1] -= m.qh(f, lgn1);
 }
 
 // ------------------------------------------------------------------ mu and phi update of a cell
 
 // F[k], J[k]: fluxes of the faces x+, x-, y+, y- (calculate_divergence_concentration.h:4-153)
-template <typename T>
-GP_HD T mu_new(const AM<T>& m, const T (&ph)[2], T mu, const T (&dp)[2], const T (&F)[4], const T (&J)[4]) {
-  const T divflux = (F[0] - F[1]) / m.dx + (F[2] - F[3]) / m.dy;
-  const T divjat = (J[0] - J[1]) * m.jscale / m.dx + (J[2] - J[3]) * m.jscale / m.dy;
+template <typename T, bool POW2>
+GP_HD T mu_new(const AM<T, POW2>& m, const T (&ph)[2], T mu, const T (&dp)[2], const T (&F)[4], const T (&J)[4]) {
+  const T divflux = m.qx(F[0] - F[1]) + m.qy(F[2] - F[3]);
+  const T divjat = m.qx((J[0] - J[1]) * m.jscale) + m.qy((J[2] - J[3]) * m.jscale);
   const int bulk = ph[0] == (T)1 ? 0 : (ph[1] == (T)1 ? 1 : -1);
   if (bulk >= 0) {
     const T c = cmu_of(m, bulk, mu) + m.dt * divflux - divjat;
@@ -729,8 +736,8 @@ GP_HD T mu_new(const AM<T>& m, const T (&ph)[2], T mu, const T (&dp)[2], const T
 
 // reverse of mu_new for the adjoint lmn of the new mu: accumulates lph, lmu,
 // ldp; returns the adjoints of divflux and divjat in gdf, gdj
-template <typename T>
-GP_HD void mu_new_rev(const AM<T>& m, const T (&ph)[2], T mu, const T (&dp)[2], const T (&F)[4], const T (&J)[4],
+template <typename T, bool POW2>
+GP_HD void mu_new_rev(const AM<T, POW2>& m, const T (&ph)[2], T mu, const T (&dp)[2], const T (&F)[4], const T (&J)[4],
                       T lmn, T (&lph)[2], T& lmu, T (&ldp)[2], T& gdf, T& gdj) {
   const int bulk = ph[0] == (T)1 ? 0 : (ph[1] == (T)1 ? 1 : -1);
   if (bulk >= 0) {
@@ -740,8 +747,8 @@ GP_HD void mu_new_rev(const AM<T>& m, const T (&ph)[2], T mu, const T (&dp)[2], 
     gdj = -lc;
     return;
   }
-  const T divflux = (F[0] - F[1]) / m.dx + (F[2] - F[3]) / m.dy;
-  const T divjat = (J[0] - J[1]) * m.jscale / m.dx + (J[2] - J[3]) * m.jscale / m.dy;
+  const T divflux = m.qx(F[0] - F[1]) + m.qy(F[2] - F[3]);
+  const T divjat = m.qx((J[0] - J[1]) * m.jscale) + m.qy((J[2] - J[3]) * m.jscale);
   T sum = (T)0, dcdmu = (T)0;
   for (int a = 0; a < 2; a++) {
     sum += cmu_of(m, a, mu) * dhfun(ph[a]) * dp[a];
