@@ -700,6 +700,23 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
     return ac * ac * Qy + ac * (m.Rinv[a][b][1][0] * e0 + m.Rinv[a][b][1][1] * e1);
   };
 
+  // Phases with a nonzero value on the six cells a face's bracket reads (the face's two cells, the
+  // second one (ni, nj) away, and their neighbours (ti, tj) to either side): a pair with an absent
+  // phase has Q = 0 there and a bracket of 0, so with three or more phases most pairs of a face, an
+  // interface of two of them, are not evaluated.
+  auto present = [&](int i, int j, int ni, int nj, int ti, int tj) -> unsigned {
+    if (N == 2) return 3u;
+    unsigned nz = 0u;
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      const bool p = (PH(a, i, j) != 0.f) | (PH(a, i + ni, j + nj) != 0.f) | (PH(a, i + ti, j + tj) != 0.f) |
+                     (PH(a, i - ti, j - tj) != 0.f) | (PH(a, i + ni + ti, j + nj + tj) != 0.f) |
+                     (PH(a, i + ni - ti, j + nj - tj) != 0.f);
+      nz |= (p ? 1u : 0u) << a;
+    }
+    return nz;
+  };
+
   // x-face between region-2 rows i and i+1 (i in [0, TX+2]) at region-2 columns
   // j in [1, TY+2]; read by ring cell (i-1, j-1) as its +x face and by ring cell
   // (i, j-1) as its -x face (region-1 coordinates)
@@ -707,22 +724,24 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
     const int i = e / (TY + 2), j = 1 + e % (TY + 2);
     const bool need = (i >= 1 && s_act[(i - 1) * Y1 + (j - 1)]) || (i <= TX + 1 && s_act[i * Y1 + (j - 1)]);
     if (!need) continue;
+    const unsigned nz = present(i, j, 1, 0, 0, 1);
 #pragma unroll
     for (int a = 0; a < N; a++)
 #pragma unroll
       for (int b = a + 1; b < N; b++)
-        sbx[(Pairs<N>::index(a, b) * (TX + 3) + i) * (TY + 2) + (j - 1)] = bk_x(i, j, a, b);
+        sbx[(Pairs<N>::index(a, b) * (TX + 3) + i) * (TY + 2) + (j - 1)] = (nz >> a) & (nz >> b) & 1u ? bk_x(i, j, a, b) : 0.f;
   }
   // y-face between region-2 columns j and j+1 (j in [0, TY+2]) at rows i in [1, TX+2]
   for (int e = threadIdx.x; e < (TX + 2) * (TY + 3); e += nt) {
     const int i = 1 + e / (TY + 3), j = e % (TY + 3);
     const bool need = (j >= 1 && s_act[(i - 1) * Y1 + (j - 1)]) || (j <= TY + 1 && s_act[(i - 1) * Y1 + j]);
     if (!need) continue;
+    const unsigned nz = present(i, j, 0, 1, 1, 0);
 #pragma unroll
     for (int a = 0; a < N; a++)
 #pragma unroll
       for (int b = a + 1; b < N; b++)
-        sby[(Pairs<N>::index(a, b) * (TX + 2) + (i - 1)) * (TY + 3) + j] = bk_y(i, j, a, b);
+        sby[(Pairs<N>::index(a, b) * (TX + 2) + (i - 1)) * (TY + 3) + j] = (nz >> a) & (nz >> b) & 1u ? bk_y(i, j, a, b) : 0.f;
   }
   __syncthreads();
 
@@ -732,9 +751,12 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
     const int i1 = e / Y1, j1 = e % Y1;  // region-1 coordinates
     const int i = i1 + 1, j = j1 + 1;    // region-2 coordinates
     float ph[N], cx[N], cy[N], divphi[N];
+    unsigned nz = 0u;  // phases present on the cell and its four neighbours
 #pragma unroll
     for (int a = 0; a < N; a++) {
       ph[a] = PH(a, i, j);
+      nz |= ((ph[a] != 0.f) | (PH(a, i + 1, j) != 0.f) | (PH(a, i - 1, j) != 0.f) | (PH(a, i, j + 1) != 0.f) |
+             (PH(a, i, j - 1) != 0.f) ? 1u : 0u) << a;
       const float gf = (PH(a, i + 1, j) - ph[a]) * m.dx_inv, gb = (ph[a] - PH(a, i - 1, j)) * m.dx_inv;
       const float gr = (PH(a, i, j + 1) - ph[a]) * m.dy_inv, gl = (ph[a] - PH(a, i, j - 1)) * m.dy_inv;
       divphi[a] = (gf - gb) * m.dx_inv + (gr - gl) * m.dy_inv;
@@ -755,6 +777,7 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
 #pragma unroll
         for (int bb = aa + 1; bb < N; bb++)
           if (Pairs<N>::index(aa, bb) == p) { a = aa; b = bb; }
+      if (N > 2 && !((nz >> a) & (nz >> b) & 1u)) continue;  // every term of the pair is 0
       float pha = 0.f, phb = 0.f, cxa = 0.f, cxb = 0.f, cya = 0.f, cyb = 0.f;
 #pragma unroll
       for (int aa = 0; aa < N; aa++) {
