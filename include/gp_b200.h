@@ -194,9 +194,10 @@ int gp_download(gp_ctx *ctx, double *phi, double *mu);
 /* nsteps explicit steps: phase-field half step, ghost fill, concentration
  * half step, ghost fill -- microsim_gp.c:102-106 for t = 1..nsteps.
  * Asynchronous on the context's stream; errors of earlier launches surface here
- * or in gp_sync.  An isothermal FP64 context replays runs of eight steps from a
- * CUDA graph captured on the first such run from each of its two buffers (the
- * same kernels and arguments as direct launches, one host launch instead of 16). */
+ * or in gp_sync.  Runs of eight steps replay a CUDA graph captured from each of
+ * the context's two buffers (the same kernels and arguments as direct launches, one
+ * host launch for all of them): isothermal FP64 contexts from the first such run,
+ * FP32 contexts once 64 steps were taken, or asked for in one call. */
 int gp_step(gp_ctx *ctx, int64_t nsteps);
 /* The context's step count (the frozen temperature gradient's clock: step t uses the temperature
  * the reference sets after step t - 1).  Starts at 0 on creation; gp_step advances it. */
@@ -294,7 +295,10 @@ int gp_batch_get_stats(gp_batch *b, int i, gp_stats *out);
 #define GP_STAT_VALUES 64
 int gp_batch_get_stats_async(gp_batch *b, int i, double *raw);
 int gp_batch_stats_from_raw(gp_batch *b, int i, const double *raw, gp_stats *out);
-/* Tile shape of the fused kernel (tx along x, ty along y): 16x32, 8x32, 32x32, 16x64. */
+/* Tile shape of the fused kernel (tx along x, ty along y): 16x32, 8x32, 32x32, 16x64.
+ * Until it is set or tuned: 8x32 with the widest full-kernel blocks when the batch has
+ * at most 1,184 tiles of that shape and four phases or fewer, else 16x32 with 256
+ * threads.  The results do not depend on it. */
 int gp_batch_set_tile(gp_batch *b, int tx, int ty);
 /* Narrow band (on by default): tiles whose cells and two-cell ring were one
  * pure phase after the previous step (per-tile purity words written by every

@@ -128,11 +128,14 @@ struct gp_ctx {
   int red_blocks;
   int64_t launches;
   int64_t tstep = 0;  // steps taken (the frozen gradient's clock)
-  cudaGraphExec_t g64[2];  // FP64 isothermal: kF64GraphSteps steps from buffer parity 0 / 1, captured on first use
+  int64_t direct = 0; // FP32 form: steps launched directly (kGraphAfter)
+  cudaGraphExec_t graph[2];  // kGraphSteps steps from buffer parity 0 / 1, captured on first use
   // running extrema (microsim_gp.c prints running values since t = 0)
   double run_phi_max[GP_MAX_PHASES], run_phi_min[GP_MAX_PHASES];
   double run_mu_max[GP_MAX_K1], run_mu_min[GP_MAX_K1];
 };
+
+static void drop_graphs(gp_ctx* c);
 
 static int check_model(const gp_model* m) {
   if (!m) return GP_E_ARG;
@@ -162,6 +165,25 @@ static int check_model(const gp_model* m) {
     return GP_E_ARG;
   }
   return GP_OK;
+}
+
+// Tile shape and full-kernel block size of an FP32 context, and of a batch until they are set or tuned.  The full
+// kernel's interface tiles run a chain of barrier-separated phases whose length follows the items per
+// thread, so a grid whose tiles all fit a few rounds of blocks is fastest with the smallest tiles and
+// (binary alloys) the widest blocks, however much of it is interface; beyond that the halo of small
+// tiles costs more than their shorter chain saves when much of the grid is interface.  Measured, us per
+// step, 16x32 tiles / 256 threads against 8x32 / 512: 400x700 planar front (1,100 tiles of 8x32) 18.2
+// and 13.2, 300x280 obstacle grains (342) 19.0 and 13.5, 300x280 well grains (342, 60% interface) 18.5
+// and 14.5; three phases 517x333 (715) at 256 threads 21.1 and 16.7, four 300x280 30.4 and 23.5; but
+// 1024^2 well grains (4,096, 31% interface) 30.8 and 42.1, four phases 2048^2 191 and 228.
+static void default_tiles(const gp_model* models, int n, int* tx, int* ty, int* threads) {
+  const gp_model& m = models[0];
+  int64_t tiles = 0;
+  for (int i = 0; i < n; i++) tiles += ((models[i].mesh_x + 7) / 8) * ((models[i].mesh_y + 31) / 32);
+  const bool small = m.N <= 4 && tiles <= 1184;  // four rounds of 296 blocks
+  *tx = small ? 8 : 16;
+  *ty = 32;
+  *threads = small && m.N == 2 && m.K1 == 1 ? 512 : 256;
 }
 
 extern "C" int gp_create(const gp_model* m, int precision, gp_ctx** out) {
@@ -213,7 +235,9 @@ extern "C" int gp_create(const gp_model* m, int precision, gp_ctx** out) {
     if (ok) {
       gp_f32_batch_bind(c->f32, 0, (float*)c->phi[0], (float*)c->mu[0], (float*)c->phi[1], (float*)c->mu[1], c->pitch,
                         c->plane);
-      ok = gp_f32_batch_set_tiles(c->f32, 16, 32) == cudaSuccess;
+      int tx, ty, threads;
+      default_tiles(m, 1, &tx, &ty, &threads);
+      ok = gp_f32_batch_set_tiles(c->f32, tx, ty) == cudaSuccess && gp_f32_batch_set_step_threads(c->f32, threads);
     }
   }
   if (!ok) {
@@ -232,8 +256,7 @@ extern "C" int gp_destroy(gp_ctx* c) {
     if (c->phi[i]) cudaFree(c->phi[i]);
     if (c->mu[i]) cudaFree(c->mu[i]);
   }
-  for (int i = 0; i < 2; i++)
-    if (c->g64[i]) cudaGraphExecDestroy(c->g64[i]);
+  drop_graphs(c);
   if (c->dphi) cudaFree(c->dphi);
   if (c->gov) cudaFree(c->gov);
   gp_f64_tiles_destroy(c->tiles);
@@ -387,21 +410,31 @@ static int f64_launch(gp_ctx* c, int p, const gp_temp_step& ts, const double* go
   return 2;
 }
 
-// An isothermal FP64 step is the same two launches every time (no per-step temperature), so
-// runs of kF64GraphSteps steps replay a CUDA graph captured once per starting buffer: one host
-// launch instead of 2 * kF64GraphSteps, which is what bounds many small instances stepped from
+// A step is the same launches every time (the FP32 form counts its temperature's clock on the device;
+// an FP64 step takes its temperature as an argument, so only isothermal ones qualify), so runs of
+// kGraphSteps steps replay a CUDA graph captured once per starting buffer: one host launch instead
+// of two to seven per step, which is what bounds a small grid, and several small instances stepped from
 // one host thread.  An even count returns the state to the buffer it started in.
-static const int kF64GraphSteps = 8;
+static const int kGraphSteps = 8;
+// Steps an FP32 context takes directly before it captures, unless one call asks for as many: capturing
+// and instantiating its seven nodes a step over two streams takes about 200 us, and a replayed step
+// saves about 3 (1024^2 grid, 19.4 against 16.9 us with the same tiles), so a context that lives for a
+// few dozen steps would pay more than it gains.
+static const int64_t kGraphAfter = 64;
 
-static int f64_graph(gp_ctx* c, cudaGraphExec_t* out) {
-  cudaGraphExec_t& ge = c->g64[c->cur];
+static int step_graph(gp_ctx* c, cudaGraphExec_t* out) {
+  cudaGraphExec_t& ge = c->graph[c->cur];
   if (!ge) {
     const gp_temp_step ts = gp_temp_after(c->m, 0);  // not read by an isothermal step
     cudaGraph_t g = nullptr;
     GP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
-    for (int t = 0, p = c->cur; t < kF64GraphSteps && rc >= 0; t++, p ^= 1) rc = f64_launch(c, p, ts, nullptr);
-    cudaError_t e = rc < 0 ? cudaErrorUnknown : cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    for (int t = 0, p = c->cur; t < kGraphSteps && rc >= 0 && e == cudaSuccess; t++, p ^= 1) {
+      if (c->precision == GP_FP64) rc = f64_launch(c, p, ts, nullptr);
+      else e = gp_f32_batch_launch(c->f32, p, c->stream);
+    }
+    if (rc < 0) e = cudaErrorUnknown;
     const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&ge, g, 0);
@@ -413,19 +446,29 @@ static int f64_graph(gp_ctx* c, cudaGraphExec_t* out) {
   return GP_OK;
 }
 
+static void drop_graphs(gp_ctx* c) {
+  for (cudaGraphExec_t& ge : c->graph)
+    if (ge) {
+      cudaGraphExecDestroy(ge);
+      ge = nullptr;
+    }
+}
+
 extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
   if (!c || nsteps < 0) return GP_E_ARG;
   for (int64_t t = 0; t < nsteps; t++) {
-    if (c->precision == GP_FP64 && !c->m.nonisothermal && !c->gov_pending && nsteps - t >= kF64GraphSteps) {
+    const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphAfter
+                                               : !c->m.nonisothermal && !c->gov_pending;
+    if (graph && nsteps - t >= kGraphSteps) {
       cudaGraphExec_t ge;
-      const int rc = f64_graph(c, &ge);
+      const int rc = step_graph(c, &ge);
       if (rc != GP_OK) return rc;
       GP_CUDA(cudaGraphLaunch(ge, c->stream));
-      c->launches += 2 * kF64GraphSteps;
+      c->launches += (c->f32 ? gp_f32_batch_launches_per_step(c->f32) : 2) * kGraphSteps;
       c->dphi_stale = c->tiles != nullptr;
       c->have_prev = 1;
-      c->tstep += kF64GraphSteps;
-      t += kF64GraphSteps - 1;
+      c->tstep += kGraphSteps;
+      t += kGraphSteps - 1;
       continue;
     }
     const int nxt = 1 - c->cur;
@@ -438,6 +481,7 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
       c->last_temp = ts;
     } else {
       GP_CUDA(gp_f32_batch_launch(c->f32, c->cur, c->stream));
+      c->direct++;
       c->launches += gp_f32_batch_launches_per_step(c->f32);
     }
     c->cur = nxt;
@@ -455,6 +499,7 @@ extern "C" int gp_set_compensated(gp_ctx* c, int on) {
   }
   GP_CUDA(cudaStreamSynchronize(c->stream));
   GP_CUDA(gp_f32_batch_set_compensated(c->f32, on));
+  drop_graphs(c);  // they hold the lean kernel of the previous mode
   return GP_OK;
 }
 
@@ -975,6 +1020,7 @@ struct gp_batch {
   int red_blocks = 296;
   int64_t launches = 0;
   int tx = 16, ty = 32;
+  int auto_block = 1;  // the full kernel's block size is default_tiles' (a tile shape set by hand goes with 256)
   int lose_pending = 0;  // failure-detection test armed for the next step
   int narrowband_on = 1;
 };
@@ -1053,7 +1099,9 @@ extern "C" int gp_batch_create(const gp_model* models, int n, gp_batch** out) {
                         b->pool + b->off_mu[1][i], b->pitch[i], b->plane[i]);
       gp_f32_batch_bind_x(b->f32, i, b->pool + b->off_phi_x[i], b->pool + b->off_mu_x[i]);
     }
-    ok = gp_f32_batch_set_tiles(b->f32, b->tx, b->ty) == cudaSuccess;
+    int threads;
+    default_tiles(models, n, &b->tx, &b->ty, &threads);
+    ok = gp_f32_batch_set_tiles(b->f32, b->tx, b->ty) == cudaSuccess && gp_f32_batch_set_step_threads(b->f32, threads);
   }
   if (!ok) {
     gp_set_error("gp_batch_create: allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1352,6 +1400,7 @@ extern "C" int gp_batch_set_tile(gp_batch* b, int tx, int ty) {
     gp_set_error("tile shape %dx%d not available", tx, ty);
     return GP_E_ARG;
   }
+  if (b->auto_block) gp_f32_batch_set_step_threads(b->f32, 256);
   batch_drop_graphs(b);
   b->tx = tx;
   b->ty = ty;
@@ -1503,6 +1552,7 @@ extern "C" int gp_batch_set_block(gp_batch* b, int threads) {
                  threads);
     return GP_E_ARG;
   }
+  b->auto_block = 0;
   batch_drop_graphs(b);
   return GP_OK;
 }

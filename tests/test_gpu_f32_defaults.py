@@ -1,0 +1,53 @@
+"""What an FP32 context and a batch choose by themselves against a batch told to use 16x32 tiles, 256
+threads and (by odd step counts) direct launches: bit for bit, on grids either side of the line where
+the small tiles give way (1,184 tiles of 8x32), isothermal and in a frozen gradient, across a switch of
+the accumulation mode (which drops the captured steps) and runs split so that both replayed and direct
+steps occur."""
+import numpy as np
+import pytest
+
+import microsim_b200 as mb
+from microsim_b200 import configs
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(4, 4), (8, 32), (9, 33), (70, 90), (592, 512), (600, 512)]  # the last two: 1,184 and 1,200 tiles
+
+
+def _case(kind, mx, my):
+    if kind == "four":
+        c = configs.c3(steps=10, mesh=max(mx, 16), nseeds=6, rng_seed=8)
+        c.mesh_x, c.mesh_y = mx, my
+        c.fills = [("FILLCYLINDER", [i, (i + 1) * mx // 4, my // 3, 0, 0, max(1.5, min(mx, my) / 9.0)]) for i in range(3)]
+        return c
+    c = configs.binary_case(mx, my, gap=1.0, supersat=0.5, eps=4.0, delta=0.03, theta=10.0, dt=0.05, tau=1.7776,
+                            function_w=2 if kind == "well" else 1, seed=(0, 0, 0.3 * min(mx, my)))
+    if kind == "gradient":
+        c.tempgrady = (0.97, 0.08, float(my), 2.0, 0.5)
+    return c
+
+
+@pytest.mark.parametrize("kind", ["obstacle", "well", "gradient", "four"])
+@pytest.mark.parametrize("size", SIZES)
+def test_defaults_equal_large_tiles_and_direct_steps(size, kind):
+    m, phi, mu = mb.load_case(_case(kind, *size))
+    with mb.Context(m, mb.GP_FP32) as c, mb.Batch([m]) as d, mb.Batch([m]) as b:
+        b.set_tile(16, 32)
+        if kind != "four":
+            b.set_block(256)
+        c.upload(phi, mu)
+        d.upload(0, phi, mu)
+        b.upload(0, phi, mu)
+        for n, comp in ((3, False), (64, False), (21, True), (75, True), (9, False)):
+            c.set_compensated(comp)
+            d.set_compensated(comp)
+            b.set_compensated(comp)
+            c.step(n)
+            d.step(n)
+            for _ in range(n):
+                b.step(1)
+            pc, uc = c.download()
+            pd, ud = d.download(0)
+            pb, ub = b.download(0)
+            assert np.array_equal(pc, pb) and np.array_equal(uc, ub), (n, comp)
+            assert np.array_equal(pd, pb) and np.array_equal(ud, ub), (n, comp)
