@@ -717,13 +717,20 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
     return nz;
   };
 
+  // Brackets of the faces of the listed cells, an item per cell and side: the upper face of every
+  // listed cell, the lower face of those whose lower neighbour is not listed (the neighbour's upper
+  // face otherwise).  Walking the list instead of all faces of the tile fills the warps: an interface
+  // crosses a few cells of every tile row, so most warps of a walk over all faces held some of its
+  // faces and ran the bracket for them.
   // x-face between region-2 rows i and i+1 (i in [0, TX+2]) at region-2 columns
   // j in [1, TY+2]; read by ring cell (i-1, j-1) as its +x face and by ring cell
   // (i, j-1) as its -x face (region-1 coordinates)
-  for (int e = threadIdx.x; e < (TX + 3) * (TY + 2); e += nt) {
-    const int i = e / (TY + 2), j = 1 + e % (TY + 2);
-    const bool need = (i >= 1 && s_act[(i - 1) * Y1 + (j - 1)]) || (i <= TX + 1 && s_act[i * Y1 + (j - 1)]);
-    if (!need) continue;
+  const int nact = s_nact;
+  for (int it = threadIdx.x; it < 2 * nact; it += nt) {
+    const bool low = it >= nact;
+    const int e = s_list[low ? it - nact : it], i1 = e / Y1, j = e % Y1 + 1;
+    if (low && i1 > 0 && s_act[e - Y1]) continue;
+    const int i = low ? i1 : i1 + 1;
     const unsigned nz = present(i, j, 1, 0, 0, 1);
 #pragma unroll
     for (int a = 0; a < N; a++)
@@ -732,10 +739,11 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
         sbx[(Pairs<N>::index(a, b) * (TX + 3) + i) * (TY + 2) + (j - 1)] = (nz >> a) & (nz >> b) & 1u ? bk_x(i, j, a, b) : 0.f;
   }
   // y-face between region-2 columns j and j+1 (j in [0, TY+2]) at rows i in [1, TX+2]
-  for (int e = threadIdx.x; e < (TX + 2) * (TY + 3); e += nt) {
-    const int i = 1 + e / (TY + 3), j = e % (TY + 3);
-    const bool need = (j >= 1 && s_act[(i - 1) * Y1 + (j - 1)]) || (j <= TY + 1 && s_act[(i - 1) * Y1 + j]);
-    if (!need) continue;
+  for (int it = threadIdx.x; it < 2 * nact; it += nt) {
+    const bool low = it >= nact;
+    const int e = s_list[low ? it - nact : it], i = e / Y1 + 1, j1 = e % Y1;
+    if (low && j1 > 0 && s_act[e - 1]) continue;
+    const int j = low ? j1 : j1 + 1;
     const unsigned nz = present(i, j, 0, 1, 1, 0);
 #pragma unroll
     for (int a = 0; a < N; a++)
@@ -745,7 +753,6 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
   }
   __syncthreads();
 
-  const int nact = s_nact;
   for (int idx = threadIdx.x; idx < nact; idx += nt) {
     const int e = s_list[idx];
     const int i1 = e / Y1, j1 = e % Y1;  // region-1 coordinates
