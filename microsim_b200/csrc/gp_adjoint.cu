@@ -793,10 +793,14 @@ struct Adj : AdjBase {
   bool pow2 = false;
   Geo g;
   cudaStream_t s = nullptr;
-  T *ckpt = nullptr, *seg = nullptr, *cur = nullptr, *nxt = nullptr;
-  int64_t ckpt_states = 0, seg_states = 0;  // capacities, kept between calls
+  T *cur = nullptr, *nxt = nullptr;
+  // one allocation for what a run keeps (grown when a longer run needs more, kept between calls):
+  // the checkpoints, a segment's states and their slots below
+  char* arena = nullptr;
+  int64_t arena_bytes = 0;
+  T *ckpt = nullptr, *seg = nullptr;
   // Delta-phi, list of the cells that are not flat and its length: of every state of a segment
-  // (slots == seg_states), or of one state at a time, recomputed before its reverse, where that
+  // (slots == every), or of one state at a time, recomputed before its reverse, where that
   // does not fit (slots == 1)
   T* ring = nullptr;
   int *list = nullptr, *cnt = nullptr;
@@ -811,13 +815,9 @@ struct Adj : AdjBase {
 
   ~Adj() {
     if (s) cudaStreamSynchronize(s);
-    cudaFree(ckpt);
-    cudaFree(seg);
+    cudaFree(arena);
     cudaFree(cur);
     cudaFree(nxt);
-    cudaFree(ring);
-    cudaFree(list);
-    cudaFree(cnt);
     cudaFree(lam[0]);
     cudaFree(lam[1]);
     cudaFree(ldphi);
@@ -913,38 +913,27 @@ struct Adj : AdjBase {
     return rc;
   }
 
-  // at least `need` states in *p, the old ones released first when there are too few
-  bool reserve(T** p, int64_t* have_states, int64_t need) {
-    if (*have_states >= need) return true;
-    cudaFree(*p);
-    *p = nullptr;
-    *have_states = 0;
-    if (cudaMalloc(p, sizeof(T) * state() * need) != cudaSuccess) {
-      cudaGetLastError();
-      *p = nullptr;
-      return false;
-    }
-    *have_states = need;
-    return true;
-  }
-
-  // Delta-phi, list and count slots for `need` states, or for one where they do not fit
-  bool reserve_slots(int64_t need) {
-    if (slots >= need) return true;
-    for (int64_t n = need;; n = 1) {
-      cudaFree(ring);
-      cudaFree(list);
-      cudaFree(cnt);
-      ring = nullptr;
-      list = cnt = nullptr;
-      slots = 0;
-      if (cudaMalloc(&ring, sizeof(T) * 2 * g.rplane * n) == cudaSuccess &&
-          cudaMalloc(&list, sizeof(int) * g.rplane * n) == cudaSuccess &&
-          cudaMalloc(&cnt, sizeof(int) * n) == cudaSuccess) {
+  // Room for nc checkpoints, ev segment states and their slots, or one slot where not all fit.
+  bool reserve(int64_t nc, int64_t ev) {
+    for (int64_t n = ev;; n = 1) {
+      const int64_t states = sizeof(T) * state() * (nc + ev), rings = sizeof(T) * 2 * g.rplane * n;
+      const int64_t lists = sizeof(int) * g.rplane * n, need = states + rings + lists + sizeof(int) * n;
+      if (arena_bytes < need) {
+        cudaFree(arena);
+        arena = nullptr;
+        arena_bytes = 0;
+        if (cudaMalloc(&arena, need) == cudaSuccess) arena_bytes = need;
+        else cudaGetLastError();
+      }
+      if (arena_bytes >= need) {
+        ckpt = reinterpret_cast<T*>(arena);
+        seg = ckpt + state() * nc;
+        ring = reinterpret_cast<T*>(arena + states);
+        list = reinterpret_cast<int*>(arena + states + rings);
+        cnt = reinterpret_cast<int*>(arena + states + rings + lists);
         slots = n;
         return true;
       }
-      cudaGetLastError();
       if (n == 1) return false;
     }
   }
@@ -956,22 +945,8 @@ struct Adj : AdjBase {
     if (ev > n) ev = n;
     const int64_t nc = (n + ev - 1) / ev;
     have = false;
-    ADJ_CUDA(cudaStreamSynchronize(s));  // buffers are released below only when too small
-    bool ok = reserve(&ckpt, &ckpt_states, nc) && reserve(&seg, &seg_states, ev) && reserve_slots(ev);
-    if (!ok) {  // what an earlier, other split keeps may stand in the way: start over
-      cudaFree(ckpt);
-      cudaFree(seg);
-      ckpt = seg = nullptr;
-      ckpt_states = seg_states = 0;
-      cudaFree(ring);
-      cudaFree(list);
-      cudaFree(cnt);
-      ring = nullptr;
-      list = cnt = nullptr;
-      slots = 0;
-      ok = reserve(&ckpt, &ckpt_states, nc) && reserve(&seg, &seg_states, ev) && reserve_slots(ev);
-    }
-    if (!ok) {
+    ADJ_CUDA(cudaStreamSynchronize(s));  // nothing queued reads the arena, which may be replaced
+    if (!reserve(nc, ev)) {
       gp_set_error("adjoint: %lld checkpoints + %lld segment states do not fit", (long long)nc, (long long)ev);
       return GP_E_NOMEM;
     }
