@@ -703,18 +703,22 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
   // Phases with a nonzero value on the six cells a face's bracket reads (the face's two cells, the
   // second one (ni, nj) away, and their neighbours (ti, tj) to either side): a pair with an absent
   // phase has Q = 0 there and a bracket of 0, so with three or more phases most pairs of a face, an
-  // interface of two of them, are not evaluated.
+  // interface of two of them, are not evaluated.  (Not for five and six phases: ten and fifteen guarded
+  // copies of the bracket per loop cost the compiler more than those sizes are used.)
   auto present = [&](int i, int j, int ni, int nj, int ti, int tj) -> unsigned {
-    if (N == 2) return 3u;
+    if (N == 2 || N > 4) return (1u << N) - 1u;
     unsigned nz = 0u;
+    float z = 0.f;  // not 0 when a value is not finite: every pair is then evaluated
 #pragma unroll
     for (int a = 0; a < N; a++) {
+      z += 0.f * PH(a, i, j) + 0.f * PH(a, i + ni, j + nj) + 0.f * PH(a, i + ti, j + tj) + 0.f * PH(a, i - ti, j - tj) +
+           0.f * PH(a, i + ni + ti, j + nj + tj) + 0.f * PH(a, i + ni - ti, j + nj - tj);
       const bool p = (PH(a, i, j) != 0.f) | (PH(a, i + ni, j + nj) != 0.f) | (PH(a, i + ti, j + tj) != 0.f) |
                      (PH(a, i - ti, j - tj) != 0.f) | (PH(a, i + ni + ti, j + nj + tj) != 0.f) |
                      (PH(a, i + ni - ti, j + nj - tj) != 0.f);
       nz |= (p ? 1u : 0u) << a;
     }
-    return nz;
+    return z == 0.f ? nz : (1u << N) - 1u;
   };
 
   // Brackets of the faces of the listed cells, an item per cell and side: the upper face of every
@@ -770,6 +774,12 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
       cx[a] = 0.5f * (gf + gb);
       cy[a] = (PH(a, i, j + 1) - PH(a, i, j - 1)) * m.half_dy_inv;
     }
+    if (N > 2 && N <= 4) {
+      float z = 0.f;
+#pragma unroll
+      for (int a = 0; a < N; a++) z += 0.f * ph[a] + 0.f * divphi[a] + 0.f * cx[a] + 0.f * cy[a];
+      if (!(z == 0.f)) nz = (1u << N) - 1u;  // something is not finite: every pair is evaluated
+    }
     // -dA/dphi_a + div dA/dgrad phi_a, accumulated per phase over pairs (one
     // copy of the pair code: the loops below are not unrolled, keeping the
     // register count of the fused kernel low)
@@ -784,7 +794,7 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
 #pragma unroll
         for (int bb = aa + 1; bb < N; bb++)
           if (Pairs<N>::index(aa, bb) == p) { a = aa; b = bb; }
-      if (N > 2 && !((nz >> a) & (nz >> b) & 1u)) continue;  // every term of the pair is 0
+      if (N > 2 && N <= 4 && !((nz >> a) & (nz >> b) & 1u)) continue;  // every term of the pair is 0
       float pha = 0.f, phb = 0.f, cxa = 0.f, cxb = 0.f, cya = 0.f, cyb = 0.f;
 #pragma unroll
       for (int aa = 0; aa < N; aa++) {
