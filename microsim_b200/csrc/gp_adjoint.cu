@@ -164,6 +164,7 @@ __device__ __forceinline__ bool owns_ring(const Geo& g, int x, int y, int i, int
 // Delta-phi -> update.  Cells with a flat block (all but a few percent) skip the phase-field
 // arithmetic; the others are compacted first, so that a warp of the tile does not wait for the few
 // of its lanes that hold an interface.
+// 18 us (ncu, 512^2 FP32, flushed caches) against about 50 for the two dense kernels before.
 template <typename T, bool POW2>
 __global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
                                             T* __restrict__ out, T* __restrict__ ring, int* __restrict__ list,

@@ -1226,6 +1226,9 @@ __global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model
 // its code: x- and y-faces share a loop through strides, phases and pairs are items spread over the
 // threads or rolled loops, and no division by a spacing is left.  Tiles of 128 cells spread an
 // interface over twice the SMs of 8 x 32 ones.
+// A step with k_lean64, against k_dphi and k_update: 1024^2 dendrite 43.4 -> 24.2 us, 611x500 four-phase
+// ternary 242 -> 127, 300x451 frozen gradient 43 -> 28, 200^2 22 -> 18; one kernel over 8 x 32 tiles for
+// bulk and interface was slower than the two it replaced (0.83x on the dendrite).
 template <int N, int K1>
 __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
     k_step64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64, Geo g, uint32_t* __restrict__ wout,
