@@ -131,11 +131,11 @@ __device__ __forceinline__ T cell_flux(const AM<T, POW2>& m, int dir, T pc0, T p
   return (Dn + Dc) * (T)0.5 * m.qd(dir, mun - muc);
 }
 
-// Start of a kernel launched as a programmatic dependent of the one before it on the stream: its blocks
-// are scheduled while that one runs; everything it reads waits for that one's end.
+// Start of a kernel launched as a dependent of the one before it: what its pointers lead to is written by
+// kernels of the same chain, so none of them is `const __restrict__` (gp_common.cuh).
 __device__ __forceinline__ void begin_dependent() {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  gp_allow_dependents();
+  gp_wait_for_earlier_kernels();
 }
 
 // Block tile of the dense kernels: a cell per thread, y fastest (a warp per tile row).
@@ -166,9 +166,8 @@ __device__ __forceinline__ bool owns_ring(const Geo& g, int x, int y, int i, int
 // of its lanes that hold an interface.
 // 18 us (ncu, 512^2 FP32, flushed caches) against about 50 for the two dense kernels before.
 template <typename T, bool POW2>
-__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
-                                            T* __restrict__ out, T* __restrict__ ring, int* __restrict__ list,
-                                            int* __restrict__ cnt) {
+__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ AM<T, POW2> m, Geo g, const T* st, T* out, T* ring,
+                                            int* list, int* cnt) {
   begin_dependent();
   __shared__ T sp[2][X2][Y2], su[X1][Y1], sd[2][X1][Y1];
   __shared__ int s_list[X1 * Y1], s_own[X1 * Y1], s_n, s_m, s_base;
@@ -301,10 +300,8 @@ __device__ __forceinline__ void block_add(double v, double* slot) {
 // ghost ring).  part[block] accumulates the D_liquid gradient, each face counted by its lower cell.
 // Bound by its loads: 6 planes in, 5 out, with one synchronisation.
 template <typename T, bool POW2>
-__global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
-                                                 const T* __restrict__ ring, const T* __restrict__ lam_in,
-                                                 T* __restrict__ lam_out, T* __restrict__ ldphi,
-                                                 double* __restrict__ part) {
+__global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, POW2> m, Geo g, const T* st, const T* ring,
+                                                 const T* lam_in, T* lam_out, T* ldphi, double* part) {
   begin_dependent();
   __shared__ T sp[2][X1][Y1], su[X1][Y1], sg[X1][Y1];
   int x0, y0;
@@ -422,11 +419,9 @@ __device__ __forceinline__ void add_nz(T* p, T v) {
 // to its upper one.  Faces between two flat cells carry no current and no derivative.
 // Bound by latency (a few thousand threads with one dependent chain of square roots and divisions).
 template <typename T, bool POW2>
-__global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
-                                                 const T* __restrict__ ring, const T* __restrict__ lam_in,
-                                                 T* __restrict__ lam_out, T* __restrict__ ldphi,
-                                                 const int* __restrict__ list, const int* __restrict__ cnt,
-                                                 double* __restrict__ part) {
+__global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, POW2> m, Geo g, const T* st, const T* ring,
+                                                 const T* lam_in, T* lam_out, T* ldphi, const int* list,
+                                                 const int* cnt, double* part) {
   begin_dependent();
   double dl = 0.0;
   const int n = 4 * *cnt;
@@ -505,10 +500,8 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, P
 // centre's contributions with their faces'.  One thread per cell is a chain of twenty a_c(q)
 // evaluations with their reverses on a few thousand threads, far too few to hide it.
 template <typename T, bool POW2>
-__global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, POW2> m, Geo g, const T* __restrict__ st,
-                                                  const T* __restrict__ ldphi, T* __restrict__ lam_out,
-                                                  const int* __restrict__ list, const int* __restrict__ cnt,
-                                                  double* __restrict__ part) {
+__global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, POW2> m, Geo g, const T* st, const T* ldphi,
+                                                  T* lam_out, const int* list, const int* cnt, double* part) {
   begin_dependent();
   constexpr unsigned ALL = 0xffffffffu;
   double acc[3] = {0.0, 0.0, 0.0};  // mobility, delta, gamma
@@ -753,20 +746,6 @@ AM<T, POW2> make_am(const gp_model& g) {
   return m;
 }
 
-template <typename... Params, typename... Args>
-cudaError_t launch_dependent(void (*fn)(Params...), int grid, int threads, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
-}
-
 struct AdjBase {
   virtual ~AdjBase() {}
   virtual int forward(const double* phi0, const double* mu0, int64_t nsteps, int64_t every, double* phi_out,
@@ -864,8 +843,8 @@ struct Adj : AdjBase {
   }
 
   cudaError_t step(const T* in, T* out, T* r = nullptr, int* l = nullptr, int* c = nullptr) {
-    return pow2 ? launch_dependent(k_fwd<T, true>, ntile, NT, s, mp, g, in, out, r, l, c)
-                : launch_dependent(k_fwd<T, false>, ntile, NT, s, md, g, in, out, r, l, c);
+    return pow2 ? gp_launch_dependent(k_fwd<T, true>, ntile, NT, 0, s, mp, g, in, out, r, l, c)
+                : gp_launch_dependent(k_fwd<T, false>, ntile, NT, 0, s, md, g, in, out, r, l, c);
   }
 
   // lin = adjoint of the state after x, lout = adjoint of x; r, l, c: x's Delta-phi, list and its length
@@ -874,11 +853,11 @@ struct Adj : AdjBase {
   }
   template <bool POW2>
   cudaError_t rev_step(const AM<T, POW2>& m, const T* x, const T* r, const int* l, const int* c, const T* lin, T* lout) {
-    cudaError_t e = launch_dependent(k_rev_cell<T, POW2>, ntile, NT, s, m, g, x, r, lin, lout, ldphi, part);
+    cudaError_t e = gp_launch_dependent(k_rev_cell<T, POW2>, ntile, NT, 0, s, m, g, x, r, lin, lout, ldphi, part);
     if (e == cudaSuccess)
-      e = launch_dependent(k_rev_jat<T, POW2>, nlist, 128, s, m, g, x, r, lin, lout, ldphi, l, c, part + ntile);
+      e = gp_launch_dependent(k_rev_jat<T, POW2>, nlist, 128, 0, s, m, g, x, r, lin, lout, ldphi, l, c, part + ntile);
     if (e == cudaSuccess)
-      e = launch_dependent(k_rev_dphi<T, POW2>, nlist, 128, s, m, g, x, ldphi, lout, l, c, part + ntile + nlist);
+      e = gp_launch_dependent(k_rev_dphi<T, POW2>, nlist, 128, 0, s, m, g, x, ldphi, lout, l, c, part + ntile + nlist);
     return e;
   }
 

@@ -28,6 +28,34 @@ __host__ __device__ __forceinline__ int gp_map_any(int v, int M, int type) {
   return gp_map(v, M, type);
 }
 
+// Programmatic dependent launch.  Such a kernel is scheduled while the ones before it on the stream still
+// run; it calls gp_wait_for_earlier_kernels before it touches anything they write, and (gp_allow_dependents)
+// lets the kernel after it be scheduled.  A buffer that an earlier kernel may be writing at that time is
+// not read-only for the whole life of this one: it is a plain pointer parameter read by plain loads (or
+// asynchronous copies) after the wait, never `const __restrict__` or __ldg, which promise that it is and
+// allow the load to be moved above the wait.  Only what was complete before the first launch of the chain
+// (tile facts, model constants) may carry them.
+__device__ __forceinline__ void gp_allow_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void gp_wait_for_earlier_kernels() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+template <typename... Params, typename... Args>
+cudaError_t gp_launch_dependent(void (*fn)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+}
+
 // Per-field, per-axis copy types.  The reference forces both sides of an axis
 // to periodic when either is, and the kernels accept only types 1 and 3, so one
 // type per (field, axis) describes the copy.

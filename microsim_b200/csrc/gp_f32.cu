@@ -412,7 +412,7 @@ template <int N, int K1, bool ANISO, int TX, int TY, int THREADS = 256>
 __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
                                                               : (K1 >= 3 || N >= 5 || THREADS > 256 ? 1 : 2))
     k_step32(const Inst* __restrict__ insts, const Model* __restrict__ models, const int* __restrict__ tile_inst,
-             const int2* __restrict__ glist, int* __restrict__ cnt, uint32_t* __restrict__ flags_out, int total,
+             const int2* glist, int* cnt, uint32_t* __restrict__ flags_out, int total,
              const int4* __restrict__ tile_desc, const uint32_t* __restrict__ flags_in, int keep_list) {
   using T = Tile<N, K1, ANISO, TX, TY>;
   constexpr int X2 = T::X2, Y2 = T::Y2, X1 = T::X1, Y1 = T::Y1, W = T::W, Q = T::Q;
@@ -435,10 +435,9 @@ __global__ void __launch_bounds__(THREADS, (N == 2 && K1 == 1) ? 1024 / THREADS
     s_scan_n = s_scan_k = s_chunk = 0;
     s_scan_done = (int)blockIdx.x >= total;
   }
-  // Launched as a programmatic dependent of the tile list (the blocks start while the list kernel
-  // runs): nothing an earlier kernel wrote is read before this wait, which returns once the list
-  // kernel and everything before it have completed.  Without that launch attribute it returns at once.
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  // Launched as a dependent of the tile list alone (glist and cnt are what it may be writing: the list
+  // kernel itself starts when all else has completed).  Without that launch attribute it returns at once.
+  gp_wait_for_earlier_kernels();
 
   for (int iter = 0;; iter++) {
   __syncthreads();  // the previous tile's shared state is no longer read
@@ -2028,7 +2027,7 @@ __global__ void __launch_bounds__(256) k_general_list(const int4* __restrict__ t
                                                       int2* __restrict__ glist, int* __restrict__ cnt,
                                                       uint8_t* __restrict__ genb, int depth) {
   // the full kernel that reads this list may start its blocks now; they wait for this kernel's end
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  gp_allow_dependents();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   int4 d = make_int4(0, 0, 0, 0);
   if (t < total) d = tile_desc[t];
@@ -2696,24 +2695,6 @@ static cudaError_t timing_slot(gp_f32_batch* b, int steps, cudaEvent_t** E) {
   return cudaSuccess;
 }
 
-// The full kernel launched right after the tile list on the same stream, as its programmatic
-// dependent: its blocks are scheduled while the list kernel runs and wait in the kernel
-// (griddepcontrol.wait) for the list, instead of the launch waiting for the list to finish.
-template <typename Fn, typename... Args>
-static cudaError_t launch_after_list(Fn fn, int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, args...);
-}
-
 // One step of every instance, reading buffer parity `parity`.
 cudaError_t gp_f32_batch_launch(gp_f32_batch* b, int parity, cudaStream_t s) {
   const KernelSet& k = b->ks;
@@ -2768,7 +2749,7 @@ cudaError_t gp_f32_batch_launch(gp_f32_batch* b, int parity, cudaStream_t s) {
         b->dinst[p], b->dmodel, b->dtile_inst, b->scan ? nullptr : b->dglist, b->scan ? nullptr : b->dcnt, flags_out,
         b->total_tiles, b->scan ? b->dtile_desc : nullptr, b->scan ? flags_in : nullptr, 0);
   else
-    e = launch_after_list(full, b->grid_general, b->step_threads, k.smem_general, s, (const Inst*)b->dinst[p],
+    e = gp_launch_dependent(full, b->grid_general, b->step_threads, k.smem_general, s, (const Inst*)b->dinst[p],
                           (const Model*)b->dmodel, (const int*)b->dtile_inst, (const int2*)b->dglist, b->dcnt,
                           flags_out, b->total_tiles, (const int4*)nullptr, (const uint32_t*)nullptr, 0);
   if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) return e;
@@ -2831,7 +2812,7 @@ cudaError_t gp_f32_batch_launch_pair(gp_f32_batch* b, int parity, cudaStream_t s
                                                                    b->dglist, b->dcnt, flags_x, b->total_tiles,
                                                                    nullptr, nullptr, 1);
   else
-    e = launch_after_list(full, b->grid_general, b->step_threads, k.smem_general, s, (const Inst*)b->dinst_x1[p],
+    e = gp_launch_dependent(full, b->grid_general, b->step_threads, k.smem_general, s, (const Inst*)b->dinst_x1[p],
                           (const Model*)b->dmodel, (const int*)b->dtile_inst, (const int2*)b->dglist, b->dcnt,
                           flags_x, b->total_tiles, (const int4*)nullptr, (const uint32_t*)nullptr, 1);
   if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) return e;

@@ -86,9 +86,9 @@ __device__ __forceinline__ void load_phi(const double* __restrict__ phi, const G
   for (int a = 0; a < N; a++) out[a] = __ldg(p + a * g.plane);
 }
 
-template <int K1>
-__device__ __forceinline__ void load_mu(const double* __restrict__ mu, const Geo& g, int x, int y, double* out,
-                                        int nphase = 0) {
+// STABLE: no kernel that may still be running writes mu (__ldg; gp_common.cuh, dependent launches)
+template <int K1, bool STABLE = true>
+__device__ __forceinline__ void load_mu(const double* mu, const Geo& g, int x, int y, double* out, int nphase = 0) {
   if (g.gov && (y < 0 || y >= g.my)) {
 #pragma unroll
     for (int k = 0; k < K1; k++) out[k] = *ghost_row(g, x, y, g.bc.mu_x, nphase + k);
@@ -97,7 +97,7 @@ __device__ __forceinline__ void load_mu(const double* __restrict__ mu, const Geo
   const int ix = gp_map(x, g.mx, g.bc.mu_x), iy = gp_map(y, g.my, g.bc.mu_y);
   const double* p = mu + (int64_t)ix * g.pitch + iy;
 #pragma unroll
-  for (int k = 0; k < K1; k++) out[k] = __ldg(p + k * g.plane);
+  for (int k = 0; k < K1; k++) out[k] = STABLE ? __ldg(p + k * g.plane) : p[k * g.plane];
 }
 
 // The 3x3 phi block around (x, y).  A cell whose block lies inside the grid reads it with plain
@@ -1130,18 +1130,14 @@ __device__ __forceinline__ void pure_cell(const gp_model& m, const C64& c64, Th 
 template <int N, int K1>
 __global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64,
                                                 Geo g, const uint32_t* __restrict__ geo,
-                                                const uint32_t* __restrict__ win, uint32_t* __restrict__ wout,
-                                                int ntile, const double* __restrict__ mu, double* __restrict__ phi_out,
-                                                double* __restrict__ mu_out, int* __restrict__ list,
-                                                int* __restrict__ cnt) {
+                                                const uint32_t* win, uint32_t* wout, int ntile, const double* mu,
+                                                double* phi_out, double* mu_out, int* list, int* cnt) {
   constexpr int TX = T64<N, K1>::TX, TY = T64<N, K1>::TY;
-  // the list's reader may be scheduled now; it waits for this kernel's end.  This kernel itself was
-  // scheduled while the previous step ran and reads nothing before that has ended.
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  gp_allow_dependents();  // the list's reader
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= ntile) return;
   const uint32_t tg = geo[t];
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  gp_wait_for_earlier_kernels();
   const int b = lean_phase(win, tg, t);
   if (b < 0) {
     if (lane == 0) list[atomicAdd(cnt, 1)] = t;
@@ -1158,11 +1154,11 @@ __global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model
 #pragma unroll
       for (int k = 0; k < K1; k++) {
         const double* p = mu + k * g.plane + (int64_t)(xr + 4 * r) * g.pitch + y;
-        u[r][0][k] = __ldg(reinterpret_cast<const double2*>(p));
-        u[r][1][k] = __ldg(reinterpret_cast<const double2*>(p - g.pitch));
-        u[r][2][k] = __ldg(reinterpret_cast<const double2*>(p + g.pitch));
-        ul[r][k] = __ldg(p - 1);
-        ur[r][k] = __ldg(p + 2);
+        u[r][0][k] = *reinterpret_cast<const double2*>(p);
+        u[r][1][k] = *reinterpret_cast<const double2*>(p - g.pitch);
+        u[r][2][k] = *reinterpret_cast<const double2*>(p + g.pitch);
+        ul[r][k] = p[-1];
+        ur[r][k] = p[2];
       }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
@@ -1191,11 +1187,11 @@ __global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model
       const int x = xr + 4 * (q >> 1), yq = y + (q & 1);
       if (x >= g.mx || yq >= g.my) continue;
       double u[5][K1], mnew[K1];
-      load_mu<K1>(mu, g, x, yq, u[0]);
-      load_mu<K1>(mu, g, x - 1, yq, u[1]);
-      load_mu<K1>(mu, g, x + 1, yq, u[2]);
-      load_mu<K1>(mu, g, x, yq - 1, u[3]);
-      load_mu<K1>(mu, g, x, yq + 1, u[4]);
+      load_mu<K1, false>(mu, g, x, yq, u[0]);
+      load_mu<K1, false>(mu, g, x - 1, yq, u[1]);
+      load_mu<K1, false>(mu, g, x + 1, yq, u[2]);
+      load_mu<K1, false>(mu, g, x, yq - 1, u[3]);
+      load_mu<K1, false>(mu, g, x, yq + 1, u[4]);
       pure_cell<N, K1>(m, c64, th_row(m, g, yq, false), b, u, mnew);
       const int64_t o = (int64_t)x * g.pitch + yq;
 #pragma unroll
@@ -1231,10 +1227,9 @@ __global__ void __launch_bounds__(256) k_lean64(const __grid_constant__ gp_model
 // bulk and interface was slower than the two it replaced (0.83x on the dendrite).
 template <int N, int K1>
 __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
-    k_step64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64, Geo g, uint32_t* __restrict__ wout,
-             const double* __restrict__ phi, const double* __restrict__ mu, double* __restrict__ phi_out,
-             double* __restrict__ mu_out, const int* __restrict__ list, const int* __restrict__ cnt,
-             int* __restrict__ next_cnt) {
+    k_step64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64, Geo g, uint32_t* wout,
+             const double* phi, const double* mu, double* phi_out, double* mu_out, const int* list, const int* cnt,
+             int* next_cnt) {
   using T = T64<N, K1>;
   constexpr int TX = T::TX, TY = T::TY, NT = T::NT, X1 = T::X1, Y1 = T::Y1, X2 = T::X2, Y2 = T::Y2;
   constexpr int R1 = X1 * Y1, R2 = X2 * Y2, FX = T::FX, NF = T::NF, JX = T::JX, NJ = T::NJ, L = N - 1;
@@ -1253,8 +1248,8 @@ __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
   const double ix = c64.ix, iy = c64.iy, i2y = c64.i2y;
   const MulSpacing spacing = {ix, iy};
 
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  gp_allow_dependents();
+  gp_wait_for_earlier_kernels();
   const int ntile = *cnt;
   if (blockIdx.x == 0 && tid == 0) *next_cnt = 0;  // the next step's list starts empty (read last by the step before)
   {
@@ -1793,23 +1788,6 @@ cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s) {
   return e == cudaSuccess ? cudaMemsetAsync(t->list + t->n, 0, 2 * sizeof(int), s) : e;
 }
 
-// Launched as a programmatic dependent of the kernel before it on the stream: its blocks are scheduled
-// while that kernel runs and wait in the kernel (griddepcontrol.wait) for its end.
-template <typename... Params, typename... Args>
-static cudaError_t launch_dependent(void (*fn)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
-}
-
 // One step by the tile kernels from buffer parity p into the other: two launches.
 cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
                               const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
@@ -1821,10 +1799,10 @@ cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pit
   int *cnt = t->list + t->n + p, *next = t->list + t->n + (p ^ 1);
 #define GP_CASE(NN, KK)                                                                                              \
   if (m.N == NN && m.K1 == KK) {                                                                                     \
-    cudaError_t e = launch_dependent(k_lean64<NN, KK>, (t->n + 7) / 8, 256, 0, s, m, t->c, g, t->geo, win, wout,     \
+    cudaError_t e = gp_launch_dependent(k_lean64<NN, KK>, (t->n + 7) / 8, 256, 0, s, m, t->c, g, t->geo, win, wout,     \
                                      t->n, mu, phi_out, mu_out, t->list, cnt);                                       \
     if (e == cudaSuccess)                                                                                            \
-      e = launch_dependent(k_step64<NN, KK>, t->grid, T64<NN, KK>::NT, T64<NN, KK>::bytes, s, m, t->c, g, wout, phi, \
+      e = gp_launch_dependent(k_step64<NN, KK>, t->grid, T64<NN, KK>::NT, T64<NN, KK>::bytes, s, m, t->c, g, wout, phi, \
                            mu, phi_out, mu_out, t->list, cnt, next);                                                 \
     return e;                                                                                                        \
   }
