@@ -424,9 +424,9 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, P
                                                  const int* cnt, double* part) {
   begin_dependent();
   double dl = 0.0;
-  const int n = 4 * *cnt;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int o = list[q >> 2], k = q & 3, dir = k >> 1;
+  const int64_t thread = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = gridDim.x * (int64_t)blockDim.x;
+  for (ListWalk q(*cnt, 4, thread, threads); q.more(); q.next()) {
+    const int o = list[q.at >> 2], k = (int)(q.at & 3), dir = k >> 1;
     int x = o / g.rpitch - 1, y = o % g.rpitch - 1;  // the listed cell, then the face's lower cell
     if (k & 1) {
       if (dir == 0) x--;
@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, 
   double acc[3] = {0.0, 0.0, 0.0};  // mobility, delta, gamma
   const int lane = threadIdx.x & 31, sub = lane & 7, a = sub >> 2, k = sub & 3, dir = k >> 1;
   const int n = *cnt, warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (int base = 4 * warp; base < n; base += 4 * warps) {
-    const int q = base + (lane >> 3);
+  for (ListWalk four(n, 1, 4 * warp, 4 * warps); four.more(); four.next()) {  // four cells a warp
+    const int64_t q = four.at + (lane >> 3);
     const int o = list[q < n ? q : n - 1], x = o / g.rpitch - 1, y = o % g.rpitch - 1;
     const T ldp[2] = {q < n ? ldphi[o] : (T)0, q < n ? ldphi[o + g.rplane] : (T)0};
     bool on = ldp[0] != (T)0 || ldp[1] != (T)0;

@@ -28,6 +28,7 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
 
 #ifndef GP_HD
 #define GP_HD __host__ __device__ __forceinline__
@@ -36,6 +37,16 @@
 namespace gpadj {
 
 enum { P_MOB = 0, P_DELTA = 1, P_GAMMA = 2, P_DLIQ = 3, NPARAM = 4 };
+
+// Items first, first + step, ... of a list of cells with `per` items each, as a thread of the list kernels
+// takes them.  64 bits: four faces for each of up to 2^31 - 1 listed cells do not fit 32, nor does the last
+// stride past a list of nearly that length.
+struct ListWalk {
+  int64_t at, end, step;
+  GP_HD ListWalk(int cells, int per, int64_t first, int64_t step_) : at(first), end((int64_t)cells * per), step(step_) {}
+  GP_HD bool more() const { return at < end; }
+  GP_HD void next() { at += step; }
+};
 
 // Model constants of one instance, in the working precision T.
 // POW2: the spacings are powers of two and quotients by them products with their exact reciprocals
