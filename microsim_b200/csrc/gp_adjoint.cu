@@ -361,12 +361,13 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, P
     const T k0 = m.Ds * m.cmu[0], k1 = m.Dl * m.cmu[1];
     const T Dme = k0 * ph[0] + k1 * ph[1];
     auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, int dir, bool to_phi, bool to_mu) {
-      const T lF = m.qd(dir, g_lo - g_hi), gr = m.qd(dir, mu_hi - mu_lo), lD = (T)0.5 * gr * lF;
+      T lD, lg;
+      flux_rev(m.qd(dir, mu_hi - mu_lo), Dsum, m.qd(dir, g_lo - g_hi), lD, lg);
       if (to_phi) {
         lph[0] += lD * k0;
         lph[1] += lD * k1;
       }
-      if (to_mu) lmu -= s * m.qd(dir, Dsum * (T)0.5 * lF);
+      if (to_mu) lmu -= s * m.qd(dir, lg);
       return lD;
     };
     const T gme = sg[i][j];

@@ -607,13 +607,20 @@ GP_HD T fface(const AM<T, POW2>& m, const Face<T>& f) {
   return (Dn + Dc) * (T)0.5 * (m.qh(f, f.mun - f.muc));
 }
 
+// Reverse of a flux D_face grad, D_face = Dsum / 2, for its adjoint lF: the adjoints of either cell's D and
+// of grad.  A flux without adjoint passes nothing on, not even where its operands are not finite.
+template <typename T>
+GP_HD void flux_rev(T grad, T Dsum, T lF, T& lD, T& lg) {
+  lD = lF != (T)0 ? (T)0.5 * grad * lF : (T)0;
+  lg = lF != (T)0 ? Dsum * (T)0.5 * lF : (T)0;
+}
+
 template <typename T, bool POW2>
 GP_HD void fface_rev(const AM<T, POW2>& m, const Face<T>& f, T lF, FaceAdj<T>& L, T (&lpar)[NPARAM]) {
   const T Dc = m.Ds * m.cmu[0] * f.pc[0] + m.Dl * m.cmu[1] * f.pc[1];
   const T Dn = m.Ds * m.cmu[0] * f.pn[0] + m.Dl * m.cmu[1] * f.pn[1];
-  const T g = m.qh(f, f.mun - f.muc);
-  const T lD = (T)0.5 * g * lF;  // adjoint of Dc and of Dn
-  const T lg = (Dn + Dc) * (T)0.5 * lF;
+  T lD, lg;
+  flux_rev(m.qh(f, f.mun - f.muc), Dn + Dc, lF, lD, lg);
   L.mun += m.qh(f, lg);
   L.muc -= m.qh(f, lg);
   L.pc[0] += lD * m.Ds * m.cmu[0];

@@ -83,3 +83,28 @@ def test_runs_of_different_lengths_on_one_object():
                 g2 = b.backward(w)
             assert np.array_equal(q, q2) and np.array_equal(u, u2)
             np.testing.assert_allclose(g, g2, rtol=1e-10)
+
+
+@pytest.mark.parametrize("precision", [mb.GP_FP64, mb.GP_FP32])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_loss_that_does_not_see_a_nonfinite_cell_has_finite_gradients(bad, precision):
+    """mu is not finite in one cell of the bulk liquid, the loss takes phi around the crystal alone: where no
+    adjoint arrives, none leaves, whatever the fields hold there."""
+    m, phi, mu = _case(48, 90, (1, 1, 1, 1), 0)
+    with mb.Context(m, mb.GP_FP64) as c:
+        c.upload(phi, mu)
+        c.step(60)
+        phi, mu = c.download()
+    assert phi[1, 36:, 70:].min() == 1.0  # bulk there
+    w = np.random.default_rng(3).standard_normal(phi.shape) * ((phi > 0) & (phi < 1))
+    spoilt = mu.copy()
+    spoilt[0, 42, 80] = bad
+    got = []
+    for u in (mu, spoilt):
+        with adjoint.Adjoint(m, precision) as a:
+            a.forward(phi, u, 3)
+            got.append(a.backward(w, None, initial=True))
+    rtol = 1e-9 if precision == mb.GP_FP64 else 1e-4  # the order of the atomic additions
+    for clean, x in zip(*got):
+        assert np.isfinite(x).all()
+        np.testing.assert_allclose(x, clean, rtol=rtol, atol=rtol * np.abs(clean).max())
