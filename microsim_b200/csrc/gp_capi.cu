@@ -25,6 +25,7 @@ struct gp_f64_tiles;
 cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out);
 void gp_f64_tiles_destroy(gp_f64_tiles* t);
 cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s);
+cudaError_t gp_f64_tiles_empty_list(gp_f64_tiles* t, int p, cudaStream_t s);
 cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
                               const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
                               const gp_temp_step* temp);
@@ -456,10 +457,14 @@ static void drop_graphs(gp_ctx* c) {
 
 extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
   if (!c || nsteps < 0) return GP_E_ARG;
+  // a caller that is capturing the context's stream records direct launches: a capture does not nest
+  cudaStreamCaptureStatus cs;
+  GP_CUDA(cudaStreamIsCapturing(c->stream, &cs));
+  const bool captured = cs != cudaStreamCaptureStatusNone;
   for (int64_t t = 0; t < nsteps; t++) {
     const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphAfter
                                                : !c->m.nonisothermal && !c->gov_pending;
-    if (graph && nsteps - t >= kGraphSteps) {
+    if (graph && !captured && nsteps - t >= kGraphSteps) {
       cudaGraphExec_t ge;
       const int rc = step_graph(c, &ge);
       if (rc != GP_OK) return rc;
@@ -474,6 +479,7 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
     const int nxt = 1 - c->cur;
     if (c->precision == GP_FP64) {
       const gp_temp_step ts = gp_temp_after(c->m, c->tstep);  // T reset after the previous step
+      if (captured && c->tiles) GP_CUDA(gp_f64_tiles_empty_list(c->tiles, c->cur, c->stream));
       const int n = f64_launch(c, c->cur, ts, c->gov_pending ? c->gov : nullptr);
       if (n < 0) return n;
       c->gov_pending = 0;

@@ -1788,6 +1788,13 @@ cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s) {
   return e == cudaSuccess ? cudaMemsetAsync(t->list + t->n, 0, 2 * sizeof(int), s) : e;
 }
 
+// The list of the step from buffer parity p is empty.  A step leaves the next parity's count at 0, which is
+// enough while steps alternate; a caller's captured step may be replayed from one parity again and again, so
+// there this goes first.
+cudaError_t gp_f64_tiles_empty_list(gp_f64_tiles* t, int p, cudaStream_t s) {
+  return cudaMemsetAsync(t->list + t->n + p, 0, sizeof(int), s);
+}
+
 // One step by the tile kernels from buffer parity p into the other: two launches.
 cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
                               const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
