@@ -26,6 +26,8 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out);
 void gp_f64_tiles_destroy(gp_f64_tiles* t);
 cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s);
 cudaError_t gp_f64_tiles_empty_list(gp_f64_tiles* t, int p, cudaStream_t s);
+cudaError_t gp_f64_tiles_survey(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
+                                cudaStream_t s);
 cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
                               const double* mu, double* phi_out, double* mu_out, cudaStream_t s,
                               const gp_temp_step* temp);
@@ -115,6 +117,8 @@ struct gp_ctx {
   void* mu[2];
   double* dphi;    // FP64 form: Delta-phi of the last phase-field half step
   gp_f64_tiles* tiles;    // FP64 form: the tile kernels' tables (nullptr: every step through dphi)
+  int words_unknown;      // the tables do not describe the current state: the next tiled step surveys it first
+  int replayed;           // a caller captured work of this context and may replay it
   int dphi_stale;         // the tile kernels took the last step: dphi follows from buffer 1-cur when asked for
   gp_temp_step last_temp; // the temperature that step ran at
   double* gov;     // FP64 form: the ghost rows a moving-frame shift leaves ([N+K1][mx][6])
@@ -137,6 +141,27 @@ struct gp_ctx {
 };
 
 static void drop_graphs(gp_ctx* c);
+
+static int stream_captured(gp_ctx* c, bool* yes) {
+  cudaStreamCaptureStatus cs;
+  GP_CUDA(cudaStreamIsCapturing(c->stream, &cs));
+  *yes = cs != cudaStreamCaptureStatusNone;
+  return GP_OK;
+}
+
+// FP64 form: the state changed other than by the tile kernels; the next tiled step surveys it.  Steps that a
+// caller captured know nothing of that when they are replayed: from the first such capture on the words are
+// zeroed at once too (0 claims nothing).
+static int tiles_unknown(gp_ctx* c) {
+  if (!c->tiles) return GP_OK;
+  bool captured;
+  const int rc = stream_captured(c, &captured);
+  if (rc != GP_OK) return rc;
+  if (captured) c->replayed = 1;
+  if (c->replayed) GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+  c->words_unknown = 1;
+  return GP_OK;
+}
 
 static int check_model(const gp_model* m) {
   if (!m) return GP_E_ARG;
@@ -356,7 +381,7 @@ extern "C" int gp_upload(gp_ctx* c, const double* phi, const double* mu) {
   int rc = copy_planes(c, phi, c->phi[c->cur], c->m.N, true);
   if (rc == GP_OK) rc = copy_planes(c, mu, c->mu[c->cur], c->m.K1, true);
   if (rc == GP_OK && c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
-  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+  if (rc == GP_OK) rc = tiles_unknown(c);
   if (rc == GP_OK) GP_CUDA(cudaStreamSynchronize(c->stream));
   c->have_prev = 0;
   return rc;
@@ -406,7 +431,8 @@ static int f64_launch(gp_ctx* c, int p, const gp_temp_step& ts, const double* go
   }
   GP_CUDA(gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[p], (const double*)c->mu[p],
                       c->dphi, (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream, false, gov, &ts));
-  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+  const int rc = tiles_unknown(c);
+  if (rc != GP_OK) return rc;
   c->dphi_stale = 0;
   return 2;
 }
@@ -458,12 +484,21 @@ static void drop_graphs(gp_ctx* c) {
 extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
   if (!c || nsteps < 0) return GP_E_ARG;
   // a caller that is capturing the context's stream records direct launches: a capture does not nest
-  cudaStreamCaptureStatus cs;
-  GP_CUDA(cudaStreamIsCapturing(c->stream, &cs));
-  const bool captured = cs != cudaStreamCaptureStatusNone;
+  bool captured;
+  const int rc = stream_captured(c, &captured);
+  if (rc != GP_OK) return rc;
+  if (captured) {
+    c->replayed = 1;
+    if (c->words_unknown) GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
+  }
   for (int64_t t = 0; t < nsteps; t++) {
     const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphAfter
                                                : !c->m.nonisothermal && !c->gov_pending;
+    if (c->words_unknown && !captured && !c->gov_pending) {
+      GP_CUDA(gp_f64_tiles_survey(c->m, c->tiles, c->cur, c->pitch, c->plane, (const double*)c->phi[c->cur], c->stream));
+      c->launches++;
+      c->words_unknown = 0;
+    }
     if (graph && !captured && nsteps - t >= kGraphSteps) {
       cudaGraphExec_t ge;
       const int rc = step_graph(c, &ge);
@@ -533,10 +568,9 @@ extern "C" int gp_smooth(gp_ctx* c, int64_t nsteps) {
       c->launches += 2;
       c->cur = nxt;
     }
-    GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
     c->dphi_stale = 0;
     c->have_prev = 0;
-    return GP_OK;
+    return tiles_unknown(c);
   }
   // FP32 context: the pre-steps run in FP64 on a copy of the state
   const size_t cells = (size_t)c->m.mesh_x * c->m.mesh_y;
@@ -665,8 +699,7 @@ extern "C" int gp_shift_y(gp_ctx* c, int64_t d) {
   c->cur = nxt;
   c->have_prev = 0;
   if (c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
-  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
-  return GP_OK;
+  return tiles_unknown(c);
 }
 
 extern "C" int gp_sync(gp_ctx* c) {
@@ -704,8 +737,7 @@ extern "C" int gp_state_changed(gp_ctx* c) {
   if (!c) return GP_E_ARG;
   c->have_prev = 0;
   if (c->f32) GP_CUDA(gp_f32_batch_invalidate(c->f32, c->stream));
-  GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
-  return GP_OK;
+  return tiles_unknown(c);
 }
 extern "C" int64_t gp_launch_count(const gp_ctx* c) { return c ? c->launches : 0; }
 

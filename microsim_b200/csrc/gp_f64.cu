@@ -1093,6 +1093,25 @@ __device__ __forceinline__ void pair_of(int p, int& a, int& b) {  // pairs a < b
 template <int N>
 __device__ __forceinline__ int pair_index(int a, int b) { return a * N - a * (a + 1) / 2 + (b - a - 1); }
 
+// Purity word of a tile (gp_tiles.cuh) from the classes (the phase a cell is the one-hot field of, 0xFF for
+// none) of its corner cells (0, 0), (ex - 1, 0), (0, ey - 1) and the parts in which some cell differs.
+__device__ __forceinline__ uint32_t part_bits(int TXi, int TYj, int ex, int ey, int v, int r0, int rxh, int ryh) {
+  uint32_t bad = 0u;
+  if (v != r0) bad |= (TXi < 2 ? 3u : 1u) | (TYj < 2 ? 8u : 0u);
+  if (TXi >= ex - 2 && v != rxh) bad |= 4u;
+  if (TYj >= ey - 2 && v != ryh) bad |= 16u;
+  return bad;
+}
+__device__ __forceinline__ uint32_t word_of(uint32_t bad, int r0, int rxh, int ryh) {
+  uint32_t w = 0u;
+  if (!(bad & 1u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_CORE;
+  if (!(bad & 2u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_XLO;
+  if (!(bad & 4u) && rxh != 0xFF) w |= (uint32_t)(1 + rxh) << PF_XHI;
+  if (!(bad & 8u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_YLO;
+  if (!(bad & 16u) && ryh != 0xFF) w |= (uint32_t)(1 + ryh) << PF_YHI;
+  return w;
+}
+
 // New mu of a bulk cell of phase b all of whose neighbours hold the one-hot phi of b: what cell_update
 // yields there (no current, face mobility (D + D) / 2).  u: centre, x-, x+, y-, y+.
 template <int N, int K1>
@@ -1117,6 +1136,62 @@ __device__ __forceinline__ void pure_cell(const gp_model& m, const C64& c64, Th 
   }
 #pragma unroll
   for (int k = 0; k < K1; k++) mnew[k] = Mu<K1>(m, th, cnew, b, k);
+}
+
+// Purity words of a state that no step wrote (an upload, a caller's writes, smoothing, a shift), nothing known of
+// the other buffer (its words 0) and both list counts 0: a warp per tile, the lanes' cells as in k_lean64.
+// One read of phi, where a step without words takes every tile through k_step64: a 1024^2 dendrite whose
+// state changes every step takes 33 us per step, 86 without this and 46 through the ring array.
+template <int N, int K1>
+__global__ void __launch_bounds__(256) k_words64(Geo g, const double* __restrict__ phi, uint32_t* __restrict__ words,
+                                                 uint32_t* __restrict__ other, int* __restrict__ cnt, int ntile) {
+  constexpr int TX = T64<N, K1>::TX, TY = T64<N, K1>::TY;
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x < 2) cnt[threadIdx.x] = 0;
+  if (t >= ntile) return;
+  const int nty = (g.my + TY - 1) / TY, x0 = (t / nty) * TX, y0 = (t % nty) * TY;
+  const int ex = min(TX, g.mx - x0), ey = min(TY, g.my - y0), i0 = lane >> 3, j0 = 2 * (lane & 7);
+  double2 v[2][N];
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const int x = min(x0 + i0 + 4 * r, g.mx - 1);  // (a row's padding lies within its pitch)
+#pragma unroll
+    for (int a = 0; a < N; a++)
+      v[r][a] = __ldg(reinterpret_cast<const double2*>(phi + a * g.plane + (int64_t)x * g.pitch + y0 + j0));
+  }
+  int cls[2][2];
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      int hot = -1;
+      bool onehot = true;
+#pragma unroll
+      for (int a = 0; a < N; a++) {
+        const double p = c ? v[r][a].y : v[r][a].x;
+        if (p == 1.0 && hot < 0) hot = a;
+        else if (__double_as_longlong(p) != 0) onehot = false;  // -0 is not the pure field's +0
+      }
+      cls[r][c] = onehot && hot >= 0 ? hot : 0xFF;
+    }
+  constexpr unsigned ALL = 0xffffffffu;
+  const int r0 = __shfl_sync(ALL, cls[0][0], 0);
+  const int xr = ex - 1, xlane = (xr & 3) * 8, h0 = __shfl_sync(ALL, cls[0][0], xlane), h1 = __shfl_sync(ALL, cls[1][0], xlane);
+  const int yc = ey - 1, y_0 = __shfl_sync(ALL, cls[0][0], yc >> 1), y_1 = __shfl_sync(ALL, cls[0][1], yc >> 1);
+  const int rxh = xr >= 4 ? h1 : h0, ryh = yc & 1 ? y_1 : y_0;
+  uint32_t bad = 0u;
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      const int i = i0 + 4 * r, j = j0 + c;
+      if (i < ex && j < ey) bad |= part_bits(i, j, ex, ey, cls[r][c], r0, rxh, ryh);
+    }
+  bad = __reduce_or_sync(ALL, bad);
+  if (lane == 0) {
+    words[t] = word_of(bad, r0, rxh, ryh);
+    other[t] = 0u;
+  }
 }
 
 // The step of the tiles that lean_phase accepts: they hold the one-hot field of one phase on their
@@ -1619,25 +1694,11 @@ __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
       const int ex = min(TX, g.mx - x0), ey = min(TY, g.my - y0);
       const int r0 = s_cls[0], rxh = s_cls[(ex - 1) * TY], ryh = s_cls[ey - 1];
       unsigned bad = 0u;
-      if (ti < ex && tj < ey) {
-        const int v = s_cls[tid];
-        if (v != r0) bad |= (ti < 2 ? 3u : 1u) | (tj < 2 ? 8u : 0u);
-        if (ti >= ex - 2 && v != rxh) bad |= 4u;
-        if (tj >= ey - 2 && v != ryh) bad |= 16u;
-      }
+      if (ti < ex && tj < ey) bad = part_bits(ti, tj, ex, ey, s_cls[tid], r0, rxh, ryh);
       bad = __reduce_or_sync(0xffffffffu, bad);
       if (lane == 0 && bad) atomicOr(&s_bad, (int)bad);
       __syncthreads();
-      if (tid == 0) {
-        const unsigned B = (unsigned)s_bad;
-        uint32_t w = 0u;
-        if (!(B & 1u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_CORE;
-        if (!(B & 2u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_XLO;
-        if (!(B & 4u) && rxh != 0xFF) w |= (uint32_t)(1 + rxh) << PF_XHI;
-        if (!(B & 8u) && r0 != 0xFF) w |= (uint32_t)(1 + r0) << PF_YLO;
-        if (!(B & 16u) && ryh != 0xFF) w |= (uint32_t)(1 + ryh) << PF_YHI;
-        wout[t] = w;
-      }
+      if (tid == 0) wout[t] = word_of((uint32_t)s_bad, r0, rxh, ryh);
     }
   }
 }
@@ -1780,12 +1841,27 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
   return cudaSuccess;
 }
 
-// The buffers' contents changed behind the kernels' back, or a step was taken without them: nothing is
-// known of the tiles, and both list counts start at 0 again (they alternate with the buffers).
+// Nothing is known of the tiles, and both list counts start at 0 again (they alternate with the buffers).
 cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s) {
   if (!t) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(t->words, 0, 2 * sizeof(uint32_t) * (size_t)t->n, s);
   return e == cudaSuccess ? cudaMemsetAsync(t->list + t->n, 0, 2 * sizeof(int), s) : e;
+}
+
+// The tables for the state in buffer parity p, from the state itself.
+cudaError_t gp_f64_tiles_survey(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
+                                cudaStream_t s) {
+  const gp_temp_step none = {};
+  const Geo g = make_geo(m, pitch, plane, 0, 0, &none, nullptr);
+#define GP_CASE(NN, KK)                                                                                       \
+  if (m.N == NN && m.K1 == KK) {                                                                              \
+    k_words64<NN, KK><<<(t->n + 7) / 8, 256, 0, s>>>(g, phi, t->words + (size_t)p * t->n,                     \
+                                                     t->words + (size_t)(p ^ 1) * t->n, t->list + t->n, t->n); \
+    return cudaGetLastError();                                                                                \
+  }
+  GP_ALL_CASES
+#undef GP_CASE
+  return cudaErrorInvalidValue;
 }
 
 // The list of the step from buffer parity p is empty.  A step leaves the next parity's count at 0, which is
