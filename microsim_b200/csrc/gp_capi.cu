@@ -25,6 +25,7 @@ struct gp_f64_tiles;
 cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out);
 void gp_f64_tiles_destroy(gp_f64_tiles* t);
 cudaError_t gp_f64_tiles_invalidate(gp_f64_tiles* t, cudaStream_t s);
+bool gp_f64_tiles_dense(const gp_f64_tiles* t);
 cudaError_t gp_f64_tiles_empty_list(gp_f64_tiles* t, int p, cudaStream_t s);
 cudaError_t gp_f64_tiles_survey(const gp_model& m, gp_f64_tiles* t, int p, int pitch, int64_t plane, const double* phi,
                                 cudaStream_t s);
@@ -134,7 +135,8 @@ struct gp_ctx {
   int64_t launches;
   int64_t tstep = 0;  // steps taken (the frozen gradient's clock)
   int64_t direct = 0; // FP32 form: steps launched directly (kGraphAfter)
-  cudaGraphExec_t graph[2];  // kGraphSteps steps from buffer parity 0 / 1, captured on first use
+  int64_t ring_steps = 0; // FP64 form: steps through the ring array since the tile kernels' last
+  cudaGraphExec_t graph[2][2];  // [FP64 form: through the ring array][buffer parity] kGraphSteps steps, captured on first use
   // running extrema (microsim_gp.c prints running values since t = 0)
   double run_phi_max[GP_MAX_PHASES], run_phi_min[GP_MAX_PHASES];
   double run_mu_max[GP_MAX_K1], run_mu_min[GP_MAX_K1];
@@ -419,22 +421,31 @@ extern "C" int gp_download_dphi(gp_ctx* c, double* dphi) {
   return GP_OK;
 }
 
-// One FP64 step from the current buffer into the other, queued: the tile kernels, or the ring-array
-// path for the step after a moving-frame shift (its explicit ghost rows) and for models the tile
-// kernels do not take.  Returns the launches it took, or a negative error.
-static int f64_launch(gp_ctx* c, int p, const gp_temp_step& ts, const double* gov) {
-  if (c->tiles && !gov) {
-    GP_CUDA(gp_f64_step_tiled(c->m, c->tiles, p, c->pitch, c->plane, (const double*)c->phi[p], (const double*)c->mu[p],
-                              (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream, &ts));
-    c->dphi_stale = 1;
-    return 2;
-  }
-  GP_CUDA(gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, (const double*)c->phi[p], (const double*)c->mu[p],
-                      c->dphi, (double*)c->phi[p ^ 1], (double*)c->mu[p ^ 1], c->stream, false, gov, &ts));
-  const int rc = tiles_unknown(c);
-  if (rc != GP_OK) return rc;
-  c->dphi_stale = 0;
-  return 2;
+// Steps through the ring array after which a tiled step counts the listed tiles anew.
+static const int64_t kLookEvery = 512;
+
+// Whether the next FP64 step goes through the ring array: for models the tile kernels do not take, after a
+// moving-frame shift (its explicit ghost rows), and while most tiles hold an interface (gp_f64_tiles_create).
+static bool ring_step(const gp_ctx* c, bool captured) {
+  if (!c->tiles || c->gov_pending) return true;
+  return !captured && gp_f64_tiles_dense(c->tiles) && c->ring_steps < kLookEvery;
+}
+
+// One FP64 step from buffer p into the other, queued (two launches).
+static cudaError_t f64_launch(gp_ctx* c, int p, const gp_temp_step& ts, bool ring, const double* gov) {
+  const double *phi = (const double*)c->phi[p], *mu = (const double*)c->mu[p];
+  double *phi_out = (double*)c->phi[p ^ 1], *mu_out = (double*)c->mu[p ^ 1];
+  if (!ring) return gp_f64_step_tiled(c->m, c->tiles, p, c->pitch, c->plane, phi, mu, phi_out, mu_out, c->stream, &ts);
+  return gp_f64_step(c->m, c->pitch, c->plane, c->rpitch, c->rplane, phi, mu, c->dphi, phi_out, mu_out, c->stream, false,
+                     gov, &ts);
+}
+
+// n FP64 steps were queued.
+static int f64_stepped(gp_ctx* c, bool ring, int64_t n) {
+  c->launches += 2 * n;
+  c->dphi_stale = !ring;
+  c->ring_steps = ring ? c->ring_steps + n : 0;
+  return ring ? tiles_unknown(c) : GP_OK;
 }
 
 // A step is the same launches every time (the FP32 form counts its temperature's clock on the device;
@@ -449,19 +460,15 @@ static const int kGraphSteps = 8;
 // few dozen steps would pay more than it gains.
 static const int64_t kGraphAfter = 64;
 
-static int step_graph(gp_ctx* c, cudaGraphExec_t* out) {
-  cudaGraphExec_t& ge = c->graph[c->cur];
+static int step_graph(gp_ctx* c, bool ring, cudaGraphExec_t* out) {
+  cudaGraphExec_t& ge = c->graph[ring][c->cur];
   if (!ge) {
     const gp_temp_step ts = gp_temp_after(c->m, 0);  // not read by an isothermal step
     cudaGraph_t g = nullptr;
     GP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = 0;
     cudaError_t e = cudaSuccess;
-    for (int t = 0, p = c->cur; t < kGraphSteps && rc >= 0 && e == cudaSuccess; t++, p ^= 1) {
-      if (c->precision == GP_FP64) rc = f64_launch(c, p, ts, nullptr);
-      else e = gp_f32_batch_launch(c->f32, p, c->stream);
-    }
-    if (rc < 0) e = cudaErrorUnknown;
+    for (int t = 0, p = c->cur; t < kGraphSteps && e == cudaSuccess; t++, p ^= 1)
+      e = c->precision == GP_FP64 ? f64_launch(c, p, ts, ring, nullptr) : gp_f32_batch_launch(c->f32, p, c->stream);
     const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&ge, g, 0);
@@ -474,11 +481,12 @@ static int step_graph(gp_ctx* c, cudaGraphExec_t* out) {
 }
 
 static void drop_graphs(gp_ctx* c) {
-  for (cudaGraphExec_t& ge : c->graph)
-    if (ge) {
-      cudaGraphExecDestroy(ge);
-      ge = nullptr;
-    }
+  for (auto& by_path : c->graph)
+    for (cudaGraphExec_t& ge : by_path)
+      if (ge) {
+        cudaGraphExecDestroy(ge);
+        ge = nullptr;
+      }
 }
 
 extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
@@ -494,18 +502,19 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
   for (int64_t t = 0; t < nsteps; t++) {
     const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphAfter
                                                : !c->m.nonisothermal && !c->gov_pending;
-    if (c->words_unknown && !captured && !c->gov_pending) {
+    const bool ring = c->precision == GP_FP64 && ring_step(c, captured);
+    if (c->words_unknown && !captured && !ring) {
       GP_CUDA(gp_f64_tiles_survey(c->m, c->tiles, c->cur, c->pitch, c->plane, (const double*)c->phi[c->cur], c->stream));
       c->launches++;
       c->words_unknown = 0;
     }
     if (graph && !captured && nsteps - t >= kGraphSteps) {
       cudaGraphExec_t ge;
-      const int rc = step_graph(c, &ge);
+      int rc = step_graph(c, ring, &ge);
       if (rc != GP_OK) return rc;
       GP_CUDA(cudaGraphLaunch(ge, c->stream));
-      c->launches += (c->f32 ? gp_f32_batch_launches_per_step(c->f32) : 2) * kGraphSteps;
-      c->dphi_stale = c->tiles != nullptr;
+      if (c->precision == GP_FP32) c->launches += gp_f32_batch_launches_per_step(c->f32) * kGraphSteps;
+      else if ((rc = f64_stepped(c, ring, kGraphSteps)) != GP_OK) return rc;
       c->have_prev = 1;
       c->tstep += kGraphSteps;
       t += kGraphSteps - 1;
@@ -514,11 +523,11 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
     const int nxt = 1 - c->cur;
     if (c->precision == GP_FP64) {
       const gp_temp_step ts = gp_temp_after(c->m, c->tstep);  // T reset after the previous step
-      if (captured && c->tiles) GP_CUDA(gp_f64_tiles_empty_list(c->tiles, c->cur, c->stream));
-      const int n = f64_launch(c, c->cur, ts, c->gov_pending ? c->gov : nullptr);
-      if (n < 0) return n;
+      if (captured && !ring) GP_CUDA(gp_f64_tiles_empty_list(c->tiles, c->cur, c->stream));
+      GP_CUDA(f64_launch(c, c->cur, ts, ring, c->gov_pending ? c->gov : nullptr));
+      const int rc = f64_stepped(c, ring, 1);
+      if (rc != GP_OK) return rc;
       c->gov_pending = 0;
-      c->launches += n;
       c->last_temp = ts;
     } else {
       GP_CUDA(gp_f32_batch_launch(c->f32, c->cur, c->stream));

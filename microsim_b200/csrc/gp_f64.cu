@@ -1304,7 +1304,7 @@ template <int N, int K1>
 __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
     k_step64(const __grid_constant__ gp_model m, const __grid_constant__ C64 c64, Geo g, uint32_t* wout,
              const double* phi, const double* mu, double* phi_out, double* mu_out, const int* list, const int* cnt,
-             int* next_cnt) {
+             int* next_cnt, int* seen, int* told) {
   using T = T64<N, K1>;
   constexpr int TX = T::TX, TY = T::TY, NT = T::NT, X1 = T::X1, Y1 = T::Y1, X2 = T::X2, Y2 = T::Y2;
   constexpr int R1 = X1 * Y1, R2 = X2 * Y2, FX = T::FX, NF = T::NF, JX = T::JX, NJ = T::NJ, L = N - 1;
@@ -1326,7 +1326,13 @@ __global__ void __launch_bounds__(T64<N, K1>::NT, T64<N, K1>::blocks)
   gp_allow_dependents();
   gp_wait_for_earlier_kernels();
   const int ntile = *cnt;
-  if (blockIdx.x == 0 && tid == 0) *next_cnt = 0;  // the next step's list starts empty (read last by the step before)
+  if (blockIdx.x == 0 && tid == 0) {
+    *next_cnt = 0;  // the next step's list starts empty (read last by the step before)
+    if (seen && *told != ntile) {  // the host's copy of the count (mapped memory), written when it changes
+      *told = ntile;
+      *reinterpret_cast<volatile int*>(seen) = ntile;
+    }
+  }
   {
 #pragma unroll 1
     for (int q = blockIdx.x; q < ntile; q += gridDim.x) {
@@ -1749,8 +1755,11 @@ struct gp_f64_tiles {
   C64 c;
   uint32_t* geo = nullptr;    // [n]
   uint32_t* words = nullptr;  // [2][n]
-  int* list = nullptr;        // [n] tiles of the current step for k_step64, then its two alternating counts
+  int* list = nullptr;        // [n] tiles of the current step for k_step64, its two alternating counts, the count last
+                              // told to the host
+  int* seen = nullptr;        // that count in page-locked memory: read without waiting for the device, so it lags
   int n = 0, grid = 0;
+  int dense_from = INT32_MAX;  // more listed tiles than this: the ring-array kernels are faster
 };
 
 void gp_f64_tiles_destroy(gp_f64_tiles* t) {
@@ -1758,6 +1767,7 @@ void gp_f64_tiles_destroy(gp_f64_tiles* t) {
   cudaFree(t->geo);
   cudaFree(t->words);
   cudaFree(t->list);
+  if (t->seen) cudaFreeHost(t->seen);
   delete t;
 }
 
@@ -1823,6 +1833,15 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
     }
   const int most = sms * (occ > 0 ? occ : 1);
   t->grid = t->n < most ? t->n : most;
+  // Two phases: a listed tile costs more than its share of k_dphi and k_update (its ring is 1.4 times its cells,
+  // and two blocks an SM overlap less than their three), so they win where most tiles are listed, unless one
+  // round of resident blocks takes them all.  us per step, tiles against ring array, listed / all: 200^2 obstacle
+  // 247/325 19.8 and 25.7; 300x280 well 558/684 31.9 and 29.2, 684/684 40.3 and 29.1; 512^2 obstacle 776/2048 44.9
+  // and 52.1, well 1012/2048 54.3 and 49.6, 1544/2048 73.6 and 57.9; 700^2 obstacle 1070/3872 63.3 and 67.5,
+  // 1741/3872 88.5 and 88.0; 1024^2 well 2269/8192 102 and 110, 3474/8192 146 and 143, 5408/8192 219 and 189.
+  // Three and four phases share more between the pairs and win at any density (four phases, all 3,425 of
+  // 3,872 listed: 428 and 695).
+  if (m.N == 2) t->dense_from = most > 2 * t->n / 5 ? most : 2 * t->n / 5;
   std::vector<uint32_t> geo(t->n);
   const gp_bc bc = gp_bc_of(m);
   for (int k = 0; k < t->n; k++) geo[k] = tile_geo((int)m.mesh_x, (int)m.mesh_y, bc, k, TX, TY);
@@ -1830,8 +1849,12 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
   if (e == cudaSuccess) e = cudaMemcpy(t->geo, geo.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&t->words, 2 * sizeof(uint32_t) * n);
   if (e == cudaSuccess) e = cudaMemset(t->words, 0, 2 * sizeof(uint32_t) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&t->list, sizeof(int) * (n + 2));
-  if (e == cudaSuccess) e = cudaMemset(t->list + n, 0, 2 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&t->list, sizeof(int) * (n + 3));
+  if (e == cudaSuccess) e = cudaMemset(t->list + n, 0, 3 * sizeof(int));
+  if (e == cudaSuccess && t->dense_from < t->n) {
+    e = cudaHostAlloc((void**)&t->seen, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) *t->seen = 0;
+  }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     gp_f64_tiles_destroy(t);
@@ -1864,6 +1887,12 @@ cudaError_t gp_f64_tiles_survey(const gp_model& m, gp_f64_tiles* t, int p, int p
   return cudaErrorInvalidValue;
 }
 
+// Whether the last count the host has seen makes the ring-array kernels the faster ones.  Either path gives the
+// same bits, so it does not matter that the count lags.
+bool gp_f64_tiles_dense(const gp_f64_tiles* t) {
+  return t->seen && *reinterpret_cast<volatile int*>(t->seen) > t->dense_from;
+}
+
 // The list of the step from buffer parity p is empty.  A step leaves the next parity's count at 0, which is
 // enough while steps alternate; a caller's captured step may be replayed from one parity again and again, so
 // there this goes first.
@@ -1886,7 +1915,7 @@ cudaError_t gp_f64_step_tiled(const gp_model& m, gp_f64_tiles* t, int p, int pit
                                      t->n, mu, phi_out, mu_out, t->list, cnt);                                       \
     if (e == cudaSuccess)                                                                                            \
       e = gp_launch_dependent(k_step64<NN, KK>, t->grid, T64<NN, KK>::NT, T64<NN, KK>::bytes, s, m, t->c, g, wout, phi, \
-                           mu, phi_out, mu_out, t->list, cnt, next);                                                 \
+                              mu, phi_out, mu_out, t->list, cnt, next, t->seen, t->list + t->n + 2);                 \
     return e;                                                                                                        \
   }
   GP_ALL_CASES

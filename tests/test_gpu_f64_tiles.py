@@ -200,3 +200,61 @@ def test_a_changed_state_costs_a_survey_not_the_bulk():
         best(True)
         plain, changed = best(False), best(True)
     assert changed < 2.5 * plain, (changed / 64, plain / 64)
+
+
+def _dense(mx, my, seed=6):
+    """A well alloy (isotropic: _pair) whose grains leave hardly a tile without an interface."""
+    c = configs.binary_case(mx, my, gap=1.0, supersat=0.5, eps=4.0, dt=0.05, tau=1.7776, function_w=2, seed=(0, 0, 5.0))
+    m, phi, mu = mb.load_case(c)
+    x, y = np.mgrid[0:mx, 0:my]
+    rng = np.random.default_rng(seed)
+    d = np.min([np.hypot(x - a, y - b) for a, b in rng.uniform(0, 1, (mx * my // 1500, 2)) * (mx, my)], 0) - 12.0
+    phi[0] = 0.5 - 0.5 * np.sin(np.pi * np.clip(d / 9.6, -0.5, 0.5))
+    phi[1] = 1.0 - phi[0]
+    return m, phi, mu
+
+
+def test_the_path_follows_the_share_of_listed_tiles_and_the_bits_do_not():
+    """A dense state (through the ring array once the host has seen the count), a sparse one written over it
+    (back to the tiles when the count is taken anew), shifts and smoothing in between, against the ring array
+    throughout."""
+    m, phi, mu = _dense(300, 280)
+    sparse = np.zeros_like(phi)
+    sparse[0, :20, :20] = 1.0
+    sparse[1] = 1.0 - sparse[0]
+    a, b = _pair(m)
+    with a, b:
+        for state in (phi, sparse, phi):
+            for c in (a, b):
+                c.upload(state, mu)
+            for n in (1, 3, 8, 17, 64, 5):
+                for c in (a, b):
+                    c.step(n)
+                _same(a, b, n)
+            for c in (a, b):
+                c.shift_y(3)
+                c.step(9)
+                c.smooth(2)
+                c.step(600)  # past the next count
+                c.step(1)
+            _same(a, b, "long")
+
+
+def test_dense_two_phase_states_are_not_slower_than_the_ring_array():
+    """684 tiles, all listed: 40 us per step through the tile kernels, 29 through the ring array."""
+    import time
+    m, phi, mu = _dense(300, 280)
+    best = []
+    for c in _pair(m):
+        with c:
+            c.upload(phi, mu)
+            c.step(32)
+            c.sync()
+            t = []
+            for _ in range(6):
+                t0 = time.perf_counter()
+                c.step(64)
+                c.sync()
+                t.append(time.perf_counter() - t0)
+            best.append(min(t))
+    assert best[0] < 1.12 * best[1], best
