@@ -195,23 +195,38 @@ static int check_model(const gp_model* m) {
   return GP_OK;
 }
 
-// Tile shape and full-kernel block size of an FP32 context, and of a batch until they are set or tuned.  The full
-// kernel's interface tiles run a chain of barrier-separated phases whose length follows the items per
-// thread, so a grid whose tiles all fit a few rounds of blocks is fastest with the smallest tiles and
-// (binary alloys) the widest blocks, however much of it is interface; beyond that the halo of small
-// tiles costs more than their shorter chain saves when much of the grid is interface.  Measured, us per
-// step, 16x32 tiles / 256 threads against 8x32 / 512: 400x700 planar front (1,100 tiles of 8x32) 18.2
-// and 13.2, 300x280 obstacle grains (342) 19.0 and 13.5, 300x280 well grains (342, 60% interface) 18.5
-// and 14.5; three phases 517x333 (715) at 256 threads 21.1 and 16.7, four 300x280 30.4 and 23.5; but
-// 1024^2 well grains (4,096, 31% interface) 30.8 and 42.1, four phases 2048^2 191 and 228.
+// Tile shape and full-kernel block size of an FP32 context, and of a batch until they are set or tuned.
+//
+// An interface tile runs a chain of barrier-separated phases whose length follows the items per thread, so
+// as long as the tiles that hold an interface (the listed ones) are resident at once, 8x32 tiles are faster than
+// 16x32, and for binary alloys 512 threads than 256; with more of them their halo (1.33 times the cells
+// in Delta-phi, against 1.2) and the fewer wide blocks cost more than the chain saves.  The listed tiles are
+// not known here, so the lines are drawn by the grid's tiles and the potential: the obstacle
+// potential's interfaces are compact and leave most tiles pure, a well's tails list most of them.
+// us per step of one grid, 16x32/256 | 8x32/256 | 8x32/512, listed/all in tiles of 8x32:
+//   obstacle 400x352 174/550 17.5 | 14.8 | 13.9, 370/550 20.0 | 17.0 | 19.5; 592x512 284/1184 17.5 | 15.6 | 14.9,
+//            574/1184 20.8 | 18.2 | 21.7; 800x700 390/2200 19.1 | 16.8 | 19.9, 847/2200 21.7 | 23.7 | 28.3;
+//            1024^2 45/4096 19.0 | 15.9 | 14.8
+//   well     300x280 339/342 20.0 | 17.3 | 19.5; 400x416 572/650 22.6 | 19.0 | 22.6; 512x416 674/832 23.7 | 20.7 | 25.3,
+//            809/832 24.3 | 25.6 | 29.0; 504x512 774/1008 24.1 | 23.7 | 27.6; 592x512 844/1184 23.3 | 24.6 | 28.7
+//   three phases (obstacle lamellae) 400x352 150/550 21.0 | 15.9, 330/550 20.2 | 20.8; 517x333 168/715 20.8 | 16.3,
+//            374/715 20.6 | 23.0; 592x512 266/1184 19.6 | 17.5, 640/1184 29.4 | 29.1; 800x700 540/2200 24.9 | 25.1
+//   four phases 400x352 192/550 28.9 | 24.3, 304/550 38.2 | 30.4, 356/550 31.4 | 34.5; 592x512 305/1184 28.3 | 24.9,
+//            584/1184 36.2 | 39.3, 755/1184 55.4 | 54.4; 1024^2 600/4096 36.2 | 39.5
+// So grids above these lines keep 16x32 although a sparse one would gain, and a grid below them that
+// fills with interfaces loses up to a tenth; gp_batch_autotune measures instead.
 static void default_tiles(const gp_model* models, int n, int* tx, int* ty, int* threads) {
   const gp_model& m = models[0];
   int64_t tiles = 0;
-  for (int i = 0; i < n; i++) tiles += ((models[i].mesh_x + 7) / 8) * ((models[i].mesh_y + 31) / 32);
-  const bool small = m.N <= 4 && tiles <= 1184;  // four rounds of 296 blocks
+  bool well = false;
+  for (int i = 0; i < n; i++) {
+    tiles += ((models[i].mesh_x + 7) / 8) * ((models[i].mesh_y + 31) / 32);
+    well |= !models[i].obstacle;
+  }
+  const bool small = m.N <= 4 && tiles <= (well ? 832 : 1184);
   *tx = small ? 8 : 16;
   *ty = 32;
-  *threads = small && m.N == 2 && m.K1 == 1 ? 512 : 256;
+  *threads = small && m.N == 2 && m.K1 == 1 && (!well || tiles <= 296) ? 512 : 256;  // 296: resident blocks of 512
 }
 
 extern "C" int gp_create(const gp_model* m, int precision, gp_ctx** out) {

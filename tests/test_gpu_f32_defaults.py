@@ -51,3 +51,35 @@ def test_defaults_equal_large_tiles_and_direct_steps(size, kind):
             pb, ub = b.download(0)
             assert np.array_equal(pc, pb) and np.array_equal(uc, ub), (n, comp)
             assert np.array_equal(pd, pb) and np.array_equal(ud, ub), (n, comp)
+
+
+@pytest.mark.parametrize("size", [(300, 280), (400, 416), (512, 416), (592, 512)])
+def test_the_default_shape_does_not_lose_on_well_grains(size):
+    """A well potential's tails leave few pure tiles: the shape a context and a batch choose against 16x32 tiles
+    with 256 threads, which they had everywhere before small tiles existed (8x32/512 on the last grid: 1.2 times
+    their time)."""
+    import time
+    mx, my = size
+    m, phi, mu = mb.load_case(_case("well", mx, my))
+    x, y = np.mgrid[0:mx, 0:my]
+    c = np.random.default_rng(6).uniform(0, 1, (30, 2)) * (mx, my)
+    d = np.min([np.hypot(x - a, y - b) for a, b in c], 0) - 0.15 * min(mx, my)
+    phi[0] = 0.5 - 0.5 * np.sin(np.pi * np.clip(d / 9.6, -0.5, 0.5))
+    phi[1] = 1.0 - phi[0]
+    best = []
+    for given in (False, True):
+        with mb.Batch([m]) as b:
+            if given:
+                b.set_tile(16, 32)
+                b.set_block(256)
+            b.upload(0, phi, mu)
+            b.step(64)
+            b.sync()
+            t = []
+            for _ in range(6):
+                t0 = time.perf_counter()
+                b.step(64)
+                b.sync()
+                t.append(time.perf_counter() - t0)
+            best.append(min(t))
+    assert best[0] < 1.08 * best[1], best
