@@ -469,11 +469,11 @@ static int f64_stepped(gp_ctx* c, bool ring, int64_t n) {
 // of two to seven per step, which is what bounds a small grid, and several small instances stepped from
 // one host thread.  An even count returns the state to the buffer it started in.
 static const int kGraphSteps = 8;
-// Steps an FP32 context takes directly before it captures, unless one call asks for as many: capturing
-// and instantiating its seven nodes a step over two streams takes about 200 us, and a replayed step
-// saves about 3 (1024^2 grid, 19.4 against 16.9 us with the same tiles), so a context that lives for a
-// few dozen steps would pay more than it gains.
-static const int64_t kGraphAfter = 64;
+// Steps an FP32 context takes directly before it captures, and the steps in one call from which it captures
+// at once: capturing and instantiating its seven nodes a step over two streams takes about 200 us, and a
+// replayed step saves 2 to 3 (1024^2 grid, 19.4 against 16.9 us with the same tiles).  A new context's one
+// call, direct and captured: 64 steps 1,237 and 1,369 us, 100 steps 1,913 and 1,944, 200 steps 3,784 and 3,628.
+static const int64_t kGraphAfter = 256, kGraphCall = 128;
 
 static int step_graph(gp_ctx* c, bool ring, cudaGraphExec_t* out) {
   cudaGraphExec_t& ge = c->graph[ring][c->cur];
@@ -515,7 +515,7 @@ extern "C" int gp_step(gp_ctx* c, int64_t nsteps) {
     if (c->words_unknown) GP_CUDA(gp_f64_tiles_invalidate(c->tiles, c->stream));
   }
   for (int64_t t = 0; t < nsteps; t++) {
-    const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphAfter
+    const bool graph = c->precision == GP_FP32 ? c->direct >= kGraphAfter || nsteps >= kGraphCall
                                                : !c->m.nonisothermal && !c->gov_pending;
     const bool ring = c->precision == GP_FP64 && ring_step(c, captured);
     if (c->words_unknown && !captured && !ring) {

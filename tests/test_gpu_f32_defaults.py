@@ -83,3 +83,25 @@ def test_the_default_shape_does_not_lose_on_well_grains(size):
                 t.append(time.perf_counter() - t0)
             best.append(min(t))
     assert best[0] < 1.08 * best[1], best
+
+
+@pytest.mark.parametrize("n", [64, 100])
+def test_a_short_run_does_not_pay_for_a_capture(n):
+    """A new context's only call takes no more than the same steps in calls of twenty, which are direct: less than
+    a third of the 200 us of a capture apart."""
+    import time
+    m, phi, mu = mb.load_case(_case("obstacle", 600, 512))
+    best = []
+    for split in (1, n // 20):
+        t = []
+        for _ in range(9):
+            with mb.Context(m, mb.GP_FP32) as c:
+                c.upload(phi, mu)
+                c.sync()
+                t0 = time.perf_counter()
+                for _ in range(split):
+                    c.step(n // split)
+                c.sync()
+                t.append(time.perf_counter() - t0)
+        best.append(min(t))
+    assert best[0] < best[1] + 60e-6, best
