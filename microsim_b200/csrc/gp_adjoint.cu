@@ -22,13 +22,12 @@
 // Backward: segments of `every` steps, last first: the segment is recomputed
 // from its checkpoint into a buffer of `every` states (each with its Delta-phi
 // and its list), then reversed.
-// Memory: ceil(N / every) + every states (every = ceil(sqrt(N)) by default).
+// Memory: ceil(N / every) + every states (every = ceil(sqrt(N)) by default), and for each state of a segment
+// its Delta-phi and list, about as much as the state, or for one state at a time (Adj::reserve).
 
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
-
-#include <vector>
 
 #include "gp_common.cuh"
 #include "gp_adjoint_cell.cuh"
@@ -775,10 +774,9 @@ struct Adj : AdjBase {
   Geo g;
   cudaStream_t s = nullptr;
   T *cur = nullptr, *nxt = nullptr;
-  // one allocation for what a run keeps (grown when a longer run needs more, kept between calls):
-  // the checkpoints, a segment's states and their slots below
+  // one allocation for what a run keeps (reserve): the checkpoints, a segment's states and their slots below
   char* arena = nullptr;
-  int64_t arena_bytes = 0;
+  int64_t arena_bytes = 0, refused = 0;  // refused: an allocation of that size failed
   T *ckpt = nullptr, *seg = nullptr;
   // Delta-phi, list of the cells that are not flat and its length: of every state of a segment
   // (slots == every), or of one state at a time, recomputed before its reverse, where that
@@ -894,29 +892,50 @@ struct Adj : AdjBase {
     return rc;
   }
 
-  // Room for nc checkpoints, ev segment states and their slots, or one slot where not all fit.
+  // Bytes of nc checkpoints, ev segment states and n slots, and their places in the arena.
+  struct Layout {
+    int64_t states, rings, lists, all;
+  };
+  Layout layout(int64_t nc, int64_t ev, int64_t n) const {
+    Layout y;
+    y.states = sizeof(T) * state() * (nc + ev);
+    y.rings = sizeof(T) * 2 * g.rplane * n;
+    y.lists = sizeof(int) * g.rplane * n;
+    y.all = y.states + y.rings + y.lists + sizeof(int) * n;
+    return y;
+  }
+
+  // Room for nc checkpoints, ev segment states and their slots.  A slot of its own for every state (about as
+  // much again as the states) saves recomputing its Delta-phi; it is taken where that leaves half of
+  // the device's free memory to others, else one slot serves all.  The arena is kept for later runs, but not
+  // at more than four times (and 64 MB) what a run needs.
   bool reserve(int64_t nc, int64_t ev) {
-    for (int64_t n = ev;; n = 1) {
-      const int64_t states = sizeof(T) * state() * (nc + ev), rings = sizeof(T) * 2 * g.rplane * n;
-      const int64_t lists = sizeof(int) * g.rplane * n, need = states + rings + lists + sizeof(int) * n;
-      if (arena_bytes < need) {
+    int64_t n = ev;
+    Layout y = layout(nc, ev, n);
+    if (arena_bytes < y.all && ev > 1) {
+      size_t room = 0, total = 0;
+      if (cudaMemGetInfo(&room, &total) != cudaSuccess) cudaGetLastError();
+      if (y.all > ((int64_t)room + arena_bytes) / 2 || (refused && y.all >= refused)) y = layout(nc, ev, n = 1);
+    }
+    for (;; y = layout(nc, ev, n = 1)) {
+      if (arena_bytes < y.all || arena_bytes > 4 * y.all + (64 << 20)) {
         cudaFree(arena);
         arena = nullptr;
         arena_bytes = 0;
-        if (cudaMalloc(&arena, need) == cudaSuccess) arena_bytes = need;
+        if (cudaMalloc(&arena, y.all) == cudaSuccess) arena_bytes = y.all;
         else cudaGetLastError();
       }
-      if (arena_bytes >= need) {
-        ckpt = reinterpret_cast<T*>(arena);
-        seg = ckpt + state() * nc;
-        ring = reinterpret_cast<T*>(arena + states);
-        list = reinterpret_cast<int*>(arena + states + rings);
-        cnt = reinterpret_cast<int*>(arena + states + rings + lists);
-        slots = n;
-        return true;
-      }
+      if (arena_bytes >= y.all) break;
       if (n == 1) return false;
+      refused = y.all;  // not tried again by this object
     }
+    ckpt = reinterpret_cast<T*>(arena);
+    seg = ckpt + state() * nc;
+    ring = reinterpret_cast<T*>(arena + y.states);
+    list = reinterpret_cast<int*>(arena + y.states + y.rings);
+    cnt = reinterpret_cast<int*>(arena + y.states + y.rings + y.lists);
+    slots = n;
+    return true;
   }
 
   int forward(const double* phi0, const double* mu0, int64_t n, int64_t ev, double* phi_out,

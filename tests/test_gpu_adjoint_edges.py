@@ -108,3 +108,43 @@ def test_a_loss_that_does_not_see_a_nonfinite_cell_has_finite_gradients(bad, pre
     for clean, x in zip(*got):
         assert np.isfinite(x).all()
         np.testing.assert_allclose(x, clean, rtol=rtol, atol=rtol * np.abs(clean).max())
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_a_long_runs_memory_is_given_back_by_a_short_one():
+    m, phi, mu = _case(512, 512, (1, 1, 1, 1), 0)
+    with adjoint.Adjoint(m, mb.GP_FP32) as a:
+        a.forward(phi, mu, 4)
+        short = _free()
+        a.forward(phi, mu, 900)  # 60 states of 3 MB and 30 slots of 3 MB
+        long = _free()
+        a.forward(phi, mu, 4)
+        assert long < short - (200 << 20)
+        assert _free() > short - (80 << 20)
+
+
+def test_slots_leave_memory_to_others_and_one_slot_gives_the_same():
+    """With about 2.4 GB free: 65 states of 12.6 MB fit, a slot for each of a segment's 64 states would take
+    as much again and more than half of what is free."""
+    import torch
+    m, phi, mu = _case(1024, 1024, (1, 1, 1, 1), 0)
+    w = np.random.default_rng(2).standard_normal(phi.shape)
+    got = []
+    for tight in (False, True):
+        hog = None
+        with adjoint.Adjoint(m, mb.GP_FP32) as a:
+            if tight:
+                torch.cuda.empty_cache()
+                hog = torch.empty(_free() - 2400 * (1 << 20), dtype=torch.uint8, device="cuda")
+            a.forward(phi, mu, 64, 64)
+            if tight:
+                assert _free() > 1300 * (1 << 20)
+            got.append(a.backward(w, None, initial=True))
+        del hog
+        torch.cuda.empty_cache()
+    for x, y in zip(*got):
+        np.testing.assert_allclose(x, y, rtol=1e-4, atol=1e-4 * np.abs(x).max())
