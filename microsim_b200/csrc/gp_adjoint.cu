@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(128) k_rev_jat(const __grid_constant__ AM<T, P
   block_add(dl, part + blockIdx.x);
 }
 
-// 3. reverse of Delta-phi (dphi_rev of gp_adjoint_cell.cuh) on the listed ring cells, eight lanes
+// 3. reverse of Delta-phi (the pieces of dphi_rev, gp_adjoint_cell.cuh) on the listed ring cells, eight lanes
 // per cell: lane a * 4 + k reverses face k of phase a's gradient-energy term, the terms at the cell's
 // centre and the projection are evaluated by all eight, and lanes 0 and 1 of each phase scatter the
 // centre's contributions with their faces'.  One thread per cell is a chain of twenty a_c(q)
@@ -515,161 +515,45 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, 
     if (!__any_sync(ALL, on)) continue;
     T P[3][3][2];
     load_P(st, g, x, y, P);
-    const T ph[2] = {P[1][1][0], P[1][1][1]}, mu = ld_mu(st, g, x, y);
-    // the record at the centre and the active phases
-    T cx[2], cy[2];
-    bool act[2];
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      const T gx = m.qx(P[2][1][p] - P[1][1][p]), bgx = m.qx(P[1][1][p] - P[0][1][p]);
-      const T gy = m.qy(P[1][2][p] - P[1][1][p]), lgy = m.qy(P[1][1][p] - P[1][0][p]);
-      cx[p] = (T)0.5 * (gx + bgx);
-      cy[p] = m.qt(P[1][2][p] - P[1][0][p]);
-      act[p] = fabs(m.qx(gx - bgx) + m.qy(gy - lgy)) > (T)0;
-    }
-    on = on && (act[0] || act[1]);  // no active phase: Delta-phi is 0 whatever the inputs
-    // the lane's face: f[n][t] along its normal (n = 0 lower, 1 upper cell) and tangent (t = 0 .. 2)
-    T s[2], gn[2], tg[2];
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      T f[2][3];
-#pragma unroll
-      for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-        for (int t = 0; t < 3; t++)
-          f[nn][t] = dir == 0 ? (k == 0 ? P[1 + nn][t][p] : P[nn][t][p]) : (k == 2 ? P[t][1 + nn][p] : P[t][nn][p]);
-      s[p] = (T)0.5 * (f[1][1] + f[0][1]);
-      gn[p] = m.qd(dir, f[1][1] - f[0][1]);
-      T tt[2];
-#pragma unroll
-      for (int nn = 0; nn < 2; nn++)
-        tt[nn] = dir == 0 ? m.qt(f[nn][2] - f[nn][0])
-                          : (T)0.5 * (m.qx(f[nn][2] - f[nn][1]) + m.qx(f[nn][1] - f[nn][0]));
-      tg[p] = tt[0] + tt[1];
-    }
-    const T sa = a ? s[1] : s[0], sb = a ? s[0] : s[1], ga = a ? gn[1] : gn[0], gb = a ? gn[0] : gn[1];
-    const T ta = a ? tg[1] : tg[0], tb = a ? tg[0] : tg[1];
-    const T pa = a ? ph[1] : ph[0], pb = a ? ph[0] : ph[1], cxa = a ? cx[1] : cx[0], cxb = a ? cx[0] : cx[1];
-    const T cya = a ? cy[1] : cy[0], cyb = a ? cy[0] : cy[1];
-    const bool act_a = a ? act[1] : act[0];
-    const T Qn = sa * gb - sb * ga, Qt = (T)0.5 * (sa * tb - sb * ta);
-    const T Qx = dir ? Qt : Qn, Qy = dir ? Qn : Qt;
-    const T sg = (k & 1) ? (T)-1 : (T)1;
-    T sum4 = sg * m.qd(dir, face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir));
+    const T mu = ld_mu(st, g, x, y);
+    DCell<T> c;
+    dphi_cell(m, P, c);
+    on = on && (c.act[0] || c.act[1]);  // no active phase: Delta-phi is 0 whatever the inputs
+    DLane<T> L;
+    dphi_lane(m, P, c, a, k, L);
+    T sum4 = dphi_face(m, L, a, k);
     sum4 += __shfl_xor_sync(ALL, sum4, 1);
     sum4 += __shfl_xor_sync(ALL, sum4, 2);
-    // the centre term (tterm)
-    const T v0 = pa * cxb - pb * cxa, v1 = pa * cyb - pb * cya;
-    T q0, q1, r0, r1;
-    mv(m.R[a], v0, v1, q0, q1);
-    mv(m.R[a], cxb, cyb, r0, r1);
-    const Aniso<T> A = aniso(m.dab, q0, q1);
-    const T q2 = q0 * q0 + q1 * q1;
-    const T qr = q0 * r0 + q1 * r1, dr = A.d0 * r0 + A.d1 * r1;
-    const T dA = (T)2 * m.gam * (A.ac * A.ac * qr + A.ac * q2 * dr);
-    const T psi = psi_of(m, a, mu);
-    const T lam = act_a ? m.eps * (-dA + (T)2 * m.gam * sum4) - m.inv_eps * wfun(m, ph, act, a) - psi * dhfun(pa) : (T)0;
-    const T lam_o = __shfl_xor_sync(ALL, lam, 4);
-    const T l0 = a ? lam_o : lam, l1 = a ? lam : lam_o;
-    const int na = (act[0] ? 1 : 0) + (act[1] ? 1 : 0);
-    const T nact = (T)(na ? na : 1), mean = (l0 + l1) / nact;
-    const T kk = m.dt * mob_eff(m, ph) / m.eps;
-    T dp[2] = {act[0] ? kk * (l0 - mean) : (T)0, act[1] ? kk * (l1 - mean) : (T)0};
-    Proj pr;
-    T Dsum, sphi;
-    proj_fwd(ph, act, dp, pr, Dsum, sphi);
-    T ld[2] = {ldp[0], ldp[1]}, lph[2] = {(T)0, (T)0};
-    proj_rev(ph, act, pr, Dsum, sphi, ld, lph);
-    const T m0 = act[0] ? kk * ld[0] : (T)0, m1 = act[1] ? kk * ld[1] : (T)0;
-    const T la = act_a && on ? (a ? m1 : m0) - (m0 + m1) / nact : (T)0;
-    if (on && sub == 0)
-      acc[0] += (double)((act[0] ? ld[0] * (l0 - mean) : (T)0) * kk / m.mob +
-                         (act[1] ? ld[1] * (l1 - mean) : (T)0) * kk / m.mob);
-    if (!on || sub != 0) lph[0] = lph[1] = (T)0;  // the projection's own adjoint once per cell
-    T lpa = a ? lph[1] : lph[0], lpb = a ? lph[0] : lph[1];
-    // the face's reverse
-    const T lt = m.eps * la;
-    T lQx = (T)0, lQy = (T)0, lS = (T)0, ldab = (T)0, lgam = (T)0, lmu = (T)0;
-    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, sb, dir, m.qd(dir, (T)2 * m.gam * sg) * lt, lQx, lQy, lS, ldab);
-    const T lQn = dir ? lQy : lQx, lQt = dir ? lQx : lQy;
-    const T lsa = lQn * gb + (T)0.5 * lQt * tb, lsb = -lQn * ga - (T)0.5 * lQt * ta + lS;
-    const T lga = -lQn * sb, lgb = lQn * sa, lta = -(T)0.5 * lQt * sb, ltb = (T)0.5 * lQt * sa;
-    // the centre's reverse (every lane of the phase evaluates it; lanes k = 0 and 1 use it)
-    T lcxa, lcya, lcxb = (T)0, lcyb = (T)0;
-    {
-      const T ldA = -lt, L = (T)2 * m.gam * ldA;
-      const T lac = L * ((T)2 * A.ac * qr + q2 * dr);
-      const T lqr = L * A.ac * A.ac, lq2 = L * A.ac * dr, ldr = L * A.ac * q2;
-      const T ld0 = ldr * r0, ld1 = ldr * r1;
-      const T lr0 = lqr * q0 + ldr * A.d0, lr1 = lqr * q1 + ldr * A.d1;
-      const T c = (T)16 * m.dab;
-      const T lq0 = lqr * r0 + c * (ld0 * A.J[0][0] + ld1 * A.J[1][0]) + lac * A.d0 + (T)2 * q0 * lq2;
-      const T lq1 = lqr * r1 + c * (ld0 * A.J[0][1] + ld1 * A.J[1][1]) + lac * A.d1 + (T)2 * q1 * lq2;
-      T lv0 = (T)0, lv1 = (T)0;
-      mv_rev(m.R[a], lr0, lr1, lcxb, lcyb);
-      mv_rev(m.R[a], lq0, lq1, lv0, lv1);
-      lcxb += lv0 * pa;
-      lcyb += lv1 * pa;
-      lcxa = -lv0 * pb;
-      lcya = -lv1 * pb;
-      if (k == 0) {
-        ldab += (T)16 * (ld0 * A.u0 + ld1 * A.u1) + lac * A.g;
-        lgam += (T)2 * sum4 * lt + (T)2 * (A.ac * A.ac * qr + A.ac * q2 * dr) * ldA;
-        lpa += lv0 * cxb + lv1 * cyb;
-        lpb += -lv0 * cxa - lv1 * cya;
-        const T lw = -m.inv_eps * la;
-        if (a ? act[0] : act[1]) {
-          if (m.obstacle) {
-            const T sgn = (pa * pb >= (T)0) ? (T)1 : (T)-1;
-            lpb += m.wobs * sgn * m.gam * lw;
-            lgam += m.wobs * sgn * pb * lw;
-          } else {
-            lpb += (T)36 * m.gam * pb * pa * lw;
-            lpa += (T)18 * m.gam * pb * pb * lw;
-            lgam += (T)18 * pb * pb * pa * lw;
-          }
-        }
-        lmu = -dpsi_dmu(m, a, mu) * dhfun(pa) * la;
-        lpa -= psi * d2hfun(pa) * la;
-      }
-    }
-    if (!on) {  // the other cells of the warp: nothing (their operands may have overflowed)
-      ldab = lgam = lmu = (T)0;
-      lpa = lpb = (T)0;
-    }
-    acc[1] += (double)ldab;
-    acc[2] += (double)lgam;
+    DTerm<T> t;
+    dphi_term(m, c, L, mu, a, sum4, t);
+    const T lam_o = __shfl_xor_sync(ALL, t.lam, 4);
+    T lph[2], dmob;
+    const T la = dphi_mean_rev(m, c, a ? lam_o : t.lam, a ? t.lam : lam_o, ldp, a, lph, dmob);
+    const bool lane_on = on && L.act_a;  // an inactive phase's operands may have overflowed
+    DAdj<T> o8;
+    dphi_lane_rev(m, L, t, mu, a, k, sum4, lane_on ? la : (T)0, o8);
+    T lmu = lane_on ? o8.lmu : (T)0;
+    acc[1] += lane_on ? (double)o8.ldab : 0.0;
+    acc[2] += lane_on ? (double)o8.lgam : 0.0;
     lmu += __shfl_xor_sync(ALL, lmu, 4);
-    if (on && sub == 0) add_nz(lam_out + ix_mu(g, x, y), lmu);
-    // the six cells of the face, both phases of the pair; the partner lane (the other phase) holds
-    // the same cells' other half, exchanged so that a lane adds one phase's values
-    T mine[2][3], other[2][3];
-#pragma unroll
-    for (int w = 0; w < 2; w++) {
-      const T lg = m.qd(dir, w ? lgb : lga), ls = (T)0.5 * (w ? lsb : lsa), lT = w ? ltb : lta;
-      const T tv = dir == 0 ? m.qt(lT) : m.qx((T)0.5 * lT);
-      T v[2][3] = {{-tv, ls - lg, tv}, {-tv, ls + lg, tv}};
-      const T hx = m.qx((T)0.5 * (w ? lcxb : lcxa)), hy = m.qt(w ? lcyb : lcya);
-      if (k == 0) {  // rows x, x + 1: the centre and its x+, y-, y+ neighbours
-        v[0][1] += w ? lpb : lpa;
-        v[1][1] += hx;
-        v[0][0] -= hy;
-        v[0][2] += hy;
-      } else if (k == 1) {  // row x - 1
-        v[0][1] -= hx;
-      }
-#pragma unroll
-      for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-        for (int t = 0; t < 3; t++) (w ? other : mine)[nn][t] = on ? v[nn][t] : (T)0;
+    if (on && sub == 0) {
+      acc[0] += (double)dmob;
+      add_nz(lam_out + ix_mu(g, x, y), lmu);
     }
+    // the partner lane (the other phase) holds the same cells' other half, exchanged so that a lane adds one
+    // phase's values; the projection's own adjoints go with the first lane's centre
 #pragma unroll
     for (int nn = 0; nn < 2; nn++)
 #pragma unroll
-      for (int t = 0; t < 3; t++) {
-        const T v = mine[nn][t] + __shfl_xor_sync(ALL, other[nn][t], 4);
+      for (int i = 0; i < 3; i++) {
+        T mine = lane_on ? o8.v[0][nn][i] : (T)0, other = lane_on ? o8.v[1][nn][i] : (T)0;
+        if (nn == 0 && i == 1 && sub == 0) {
+          mine += lph[0];
+          other += lph[1];
+        }
+        const T v = mine + __shfl_xor_sync(ALL, other, 4);
         if (!on) continue;
-        const int dn = nn - (k & 1), dt = t - 1;
+        const int dn = nn - (k & 1), dt = i - 1;
         add_nz(lam_out + ix_phi(g, dir ? x + dt : x + dn, dir ? y + dn : y + dt, a), v);
       }
   }

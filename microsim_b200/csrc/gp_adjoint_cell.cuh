@@ -182,33 +182,6 @@ GP_HD void grad_fwd(const AM<T, POW2>& m, const T (&P)[3][3][2], Grad<T>& G) {
   }
 }
 
-// reverse of grad_fwd: LG holds the adjoints of the record, accumulated into LP
-template <typename T, bool POW2>
-GP_HD void grad_rev(const AM<T, POW2>& m, const Grad<T>& LG, T (&LP)[3][3][2]) {
-  for (int a = 0; a < 2; a++) {
-    const T lgx = LG.gx[a] + (T)0.5 * LG.cx[a], lbgx = LG.bgx[a] + (T)0.5 * LG.cx[a];
-    LP[2][1][a] += m.qx(lgx) + (T)0.5 * LG.sx[a];
-    LP[1][1][a] += m.qx(-lgx) + (T)0.5 * LG.sx[a];
-    LP[1][2][a] += m.qy(LG.gy[a]) + (T)0.5 * LG.sy[a];
-    LP[1][1][a] += m.qy(-LG.gy[a]) + (T)0.5 * LG.sy[a];
-    LP[1][2][a] += m.qt(LG.cy[a]);
-    LP[1][0][a] -= m.qt(LG.cy[a]);
-    LP[1][1][a] += m.qx(lbgx) + (T)0.5 * LG.bsx[a];
-    LP[0][1][a] += m.qx(-lbgx) + (T)0.5 * LG.bsx[a];
-    LP[0][2][a] += m.qt(LG.bcy[a]);
-    LP[0][0][a] -= m.qt(LG.bcy[a]);
-    LP[2][2][a] += m.qt(LG.fcy[a]);
-    LP[2][0][a] -= m.qt(LG.fcy[a]);
-    LP[1][1][a] += m.qy(LG.lgy[a]) + (T)0.5 * LG.lsy[a];
-    LP[1][0][a] += m.qy(-LG.lgy[a]) + (T)0.5 * LG.lsy[a];
-    const T hl = m.qx((T)0.5 * LG.lcx[a]), hr = m.qx((T)0.5 * LG.rcx[a]);
-    LP[2][0][a] += hl;
-    LP[0][0][a] -= hl;
-    LP[2][2][a] += hr;
-    LP[0][2][a] -= hr;
-  }
-}
-
 // ------------------------------------------------------------------ gradient energy
 
 // One face term of div(dA/dgrad phi_a) (function_A_01.h:101-219):
@@ -275,48 +248,6 @@ GP_HD void face_ops(const Grad<T>& G, int a, int k, T& Qx, T& Qy, T& S) {
   }
 }
 
-template <typename T>
-GP_HD void face_ops_rev(const Grad<T>& G, int a, int k, T lQx, T lQy, T lS, Grad<T>& L) {
-  const int b = 1 - a;
-  if (k == 0) {
-    L.sx[a] += lQx * G.gx[b] + (T)0.5 * lQy * (G.cy[b] + G.fcy[b]);
-    L.gx[b] += lQx * G.sx[a];
-    L.sx[b] += -lQx * G.gx[a] - (T)0.5 * lQy * (G.cy[a] + G.fcy[a]) + lS;
-    L.gx[a] += -lQx * G.sx[b];
-    L.cy[b] += (T)0.5 * lQy * G.sx[a];
-    L.fcy[b] += (T)0.5 * lQy * G.sx[a];
-    L.cy[a] += -(T)0.5 * lQy * G.sx[b];
-    L.fcy[a] += -(T)0.5 * lQy * G.sx[b];
-  } else if (k == 1) {
-    L.bsx[a] += lQx * G.bgx[b] + (T)0.5 * lQy * (G.bcy[b] + G.cy[b]);
-    L.bgx[b] += lQx * G.bsx[a];
-    L.bsx[b] += -lQx * G.bgx[a] - (T)0.5 * lQy * (G.bcy[a] + G.cy[a]) + lS;
-    L.bgx[a] += -lQx * G.bsx[b];
-    L.bcy[b] += (T)0.5 * lQy * G.bsx[a];
-    L.cy[b] += (T)0.5 * lQy * G.bsx[a];
-    L.bcy[a] += -(T)0.5 * lQy * G.bsx[b];
-    L.cy[a] += -(T)0.5 * lQy * G.bsx[b];
-  } else if (k == 2) {
-    L.sy[a] += (T)0.5 * lQx * (G.cx[b] + G.rcx[b]) + lQy * G.gy[b];
-    L.sy[b] += -(T)0.5 * lQx * (G.cx[a] + G.rcx[a]) - lQy * G.gy[a] + lS;
-    L.cx[b] += (T)0.5 * lQx * G.sy[a];
-    L.rcx[b] += (T)0.5 * lQx * G.sy[a];
-    L.cx[a] += -(T)0.5 * lQx * G.sy[b];
-    L.rcx[a] += -(T)0.5 * lQx * G.sy[b];
-    L.gy[b] += lQy * G.sy[a];
-    L.gy[a] += -lQy * G.sy[b];
-  } else {
-    L.lsy[a] += (T)0.5 * lQx * (G.lcx[b] + G.cx[b]) + lQy * G.lgy[b];
-    L.lsy[b] += -(T)0.5 * lQx * (G.lcx[a] + G.cx[a]) - lQy * G.lgy[a] + lS;
-    L.lcx[b] += (T)0.5 * lQx * G.lsy[a];
-    L.cx[b] += (T)0.5 * lQx * G.lsy[a];
-    L.lcx[a] += -(T)0.5 * lQx * G.lsy[b];
-    L.cx[a] += -(T)0.5 * lQx * G.lsy[b];
-    L.lgy[b] += lQy * G.lsy[a];
-    L.lgy[a] += -lQy * G.lsy[b];
-  }
-}
-
 // t_a = -dA/dphi_a + div dA/dgrad phi_a for the pair (a, 1-a)
 // (function_A_01.h:4-71, 101-219)
 template <typename T, bool POW2>
@@ -339,52 +270,6 @@ GP_HD T tterm(const AM<T, POW2>& m, const Grad<T>& G, const T (&ph)[2], int a) {
     sum += (k & 1) ? -W : W;
   }
   return -dA + (T)2 * m.gam * sum;
-}
-
-template <typename T, bool POW2>
-GP_HD void tterm_rev(const AM<T, POW2>& m, const Grad<T>& G, const T (&ph)[2], int a, T lam, Grad<T>& LG, T (&lph)[2],
-                     T& ldab, T& lgam) {
-  const int b = 1 - a;
-  // divA = 2 gam sum_k sign_k V_k / h_k
-  T sum = (T)0;
-  for (int k = 0; k < 4; k++) {
-    T Qx, Qy, S;
-    face_ops(G, a, k, Qx, Qy, S);
-    const T sg = (k & 1) ? (T)-1 : (T)1;
-    sum += m.qd(k >> 1, sg * face_term(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1));
-    T lQx = 0, lQy = 0, lS = 0;
-    face_term_rev(m.R[a], m.Ri[a], m.dab, Qx, Qy, S, k >> 1, m.qd(k >> 1, (T)2 * m.gam * sg) * lam, lQx, lQy, lS, ldab);
-    face_ops_rev(G, a, k, lQx, lQy, lS, LG);
-  }
-  lgam += (T)2 * sum * lam;
-  // -dA
-  const T v0 = ph[a] * G.cx[b] - ph[b] * G.cx[a], v1 = ph[a] * G.cy[b] - ph[b] * G.cy[a];
-  T q0, q1, r0, r1;
-  mv(m.R[a], v0, v1, q0, q1);
-  mv(m.R[a], G.cx[b], G.cy[b], r0, r1);
-  const Aniso<T> A = aniso(m.dab, q0, q1);
-  const T q2 = q0 * q0 + q1 * q1;
-  const T qr = q0 * r0 + q1 * r1, dr = A.d0 * r0 + A.d1 * r1;
-  const T ldA = -lam;
-  lgam += (T)2 * (A.ac * A.ac * qr + A.ac * q2 * dr) * ldA;
-  const T L = (T)2 * m.gam * ldA;
-  const T lac = L * ((T)2 * A.ac * qr + q2 * dr);
-  const T lqr = L * A.ac * A.ac, lq2 = L * A.ac * dr, ldr = L * A.ac * q2;
-  const T ld0 = ldr * r0, ld1 = ldr * r1;
-  const T lr0 = lqr * q0 + ldr * A.d0, lr1 = lqr * q1 + ldr * A.d1;
-  const T c = (T)16 * m.dab;
-  const T lq0 = lqr * r0 + c * (ld0 * A.J[0][0] + ld1 * A.J[1][0]) + lac * A.d0 + (T)2 * q0 * lq2;
-  const T lq1 = lqr * r1 + c * (ld0 * A.J[0][1] + ld1 * A.J[1][1]) + lac * A.d1 + (T)2 * q1 * lq2;
-  ldab += (T)16 * (ld0 * A.u0 + ld1 * A.u1) + lac * A.g;
-  T lcxb = 0, lcyb = 0, lv0 = 0, lv1 = 0;
-  mv_rev(m.R[a], lr0, lr1, lcxb, lcyb);
-  mv_rev(m.R[a], lq0, lq1, lv0, lv1);
-  lph[a] += lv0 * G.cx[b] + lv1 * G.cy[b];
-  lph[b] += -lv0 * G.cx[a] - lv1 * G.cy[a];
-  LG.cx[b] += lcxb + lv0 * ph[a];
-  LG.cy[b] += lcyb + lv1 * ph[a];
-  LG.cx[a] += -lv0 * ph[b];
-  LG.cy[a] += -lv1 * ph[b];
 }
 
 // ------------------------------------------------------------------ Delta-phi of a cell
@@ -513,72 +398,227 @@ GP_HD void dphi_fwd(const AM<T, POW2>& m, const T (&P)[3][3][2], T mu, T (&dp)[2
   proj_fwd(ph, act, dp, r, Dsum, sphi);
 }
 
+// Reverse of dphi_fwd in pieces for the eight lanes of a cell, a lane per phase a and face k (x+, x-, y+,
+// y-) of its gradient-energy term: the kernel's lanes exchange what they need of each other, dphi_rev below
+// runs the same pieces one after the other.
+template <typename T>
+struct DCell {  // the record at the centre
+  T ph[2], cx[2], cy[2];
+  bool act[2];
+};
+template <typename T, bool POW2>
+GP_HD void dphi_cell(const AM<T, POW2>& m, const T (&P)[3][3][2], DCell<T>& c) {
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    const T gx = m.qx(P[2][1][p] - P[1][1][p]), bgx = m.qx(P[1][1][p] - P[0][1][p]);
+    const T gy = m.qy(P[1][2][p] - P[1][1][p]), lgy = m.qy(P[1][1][p] - P[1][0][p]);
+    c.ph[p] = P[1][1][p];
+    c.cx[p] = (T)0.5 * (gx + bgx);
+    c.cy[p] = m.qt(P[1][2][p] - P[1][0][p]);
+    c.act[p] = fabs(m.qx(gx - bgx) + m.qy(gy - lgy)) > (T)0;
+  }
+}
+
+// Lane (a, k)'s operands, b = 1 - a.  The face: means sa, sb, normal gradients ga, gb and doubled tangential
+// ones ta, tb of the two phases.  The centre: pa, pb, cxa .. cyb.
+template <typename T>
+struct DLane {
+  T sa, sb, ga, gb, ta, tb, Qx, Qy;
+  T pa, pb, cxa, cxb, cya, cyb;
+  bool act_a, act_b;
+};
+template <typename T, bool POW2>
+GP_HD void dphi_lane(const AM<T, POW2>& m, const T (&P)[3][3][2], const DCell<T>& c, int a, int k, DLane<T>& L) {
+  const int dir = k >> 1;
+  T s[2], gn[2], tg[2];
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    T f[2][3];  // the six cells: n = 0 lower, 1 upper cell along the normal, t along the tangent
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+#pragma unroll
+      for (int t = 0; t < 3; t++)
+        f[n][t] = dir == 0 ? (k == 0 ? P[1 + n][t][p] : P[n][t][p]) : (k == 2 ? P[t][1 + n][p] : P[t][n][p]);
+    s[p] = (T)0.5 * (f[1][1] + f[0][1]);
+    gn[p] = m.qd(dir, f[1][1] - f[0][1]);
+    T tt[2];
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+      tt[n] = dir == 0 ? m.qt(f[n][2] - f[n][0]) : (T)0.5 * (m.qx(f[n][2] - f[n][1]) + m.qx(f[n][1] - f[n][0]));
+    tg[p] = tt[0] + tt[1];
+  }
+  L.sa = a ? s[1] : s[0]; L.sb = a ? s[0] : s[1];
+  L.ga = a ? gn[1] : gn[0]; L.gb = a ? gn[0] : gn[1];
+  L.ta = a ? tg[1] : tg[0]; L.tb = a ? tg[0] : tg[1];
+  const T Qn = L.sa * L.gb - L.sb * L.ga, Qt = (T)0.5 * (L.sa * L.tb - L.sb * L.ta);
+  L.Qx = dir ? Qt : Qn;
+  L.Qy = dir ? Qn : Qt;
+  L.pa = a ? c.ph[1] : c.ph[0]; L.pb = a ? c.ph[0] : c.ph[1];
+  L.cxa = a ? c.cx[1] : c.cx[0]; L.cxb = a ? c.cx[0] : c.cx[1];
+  L.cya = a ? c.cy[1] : c.cy[0]; L.cyb = a ? c.cy[0] : c.cy[1];
+  L.act_a = a ? c.act[1] : c.act[0]; L.act_b = a ? c.act[0] : c.act[1];
+}
+
+// the lane's share of sum_k sign_k V_k / h_k
+template <typename T, bool POW2>
+GP_HD T dphi_face(const AM<T, POW2>& m, const DLane<T>& L, int a, int k) {
+  const T sg = (k & 1) ? (T)-1 : (T)1;
+  return sg * m.qd(k >> 1, face_term(m.R[a], m.Ri[a], m.dab, L.Qx, L.Qy, L.sb, k >> 1));
+}
+
+// the terms at the centre and phase a's lambda, from the sum over its four faces
+template <typename T>
+struct DTerm {
+  Aniso<T> A;
+  T q0, q1, r0, r1, q2, qr, dr, psi, lam;
+};
+template <typename T, bool POW2>
+GP_HD void dphi_term(const AM<T, POW2>& m, const DCell<T>& c, const DLane<T>& L, T mu, int a, T sum4, DTerm<T>& t) {
+  const T v0 = L.pa * L.cxb - L.pb * L.cxa, v1 = L.pa * L.cyb - L.pb * L.cya;
+  mv(m.R[a], v0, v1, t.q0, t.q1);
+  mv(m.R[a], L.cxb, L.cyb, t.r0, t.r1);
+  t.A = aniso(m.dab, t.q0, t.q1);
+  t.q2 = t.q0 * t.q0 + t.q1 * t.q1;
+  t.qr = t.q0 * t.r0 + t.q1 * t.r1;
+  t.dr = t.A.d0 * t.r0 + t.A.d1 * t.r1;
+  const T dA = (T)2 * m.gam * (t.A.ac * t.A.ac * t.qr + t.A.ac * t.q2 * t.dr);
+  t.psi = psi_of(m, a, mu);
+  t.lam = L.act_a ? m.eps * (-dA + (T)2 * m.gam * sum4) - m.inv_eps * wfun(m, c.ph, c.act, a) - t.psi * dhfun(L.pa) : (T)0;
+}
+
+// From both phases' lambda and the adjoint of Delta-phi: the adjoint of phase a's lambda, lph what the
+// projection adds to the phases' own adjoints (once per cell), dmob the mobility's gradient.
+template <typename T, bool POW2>
+GP_HD T dphi_mean_rev(const AM<T, POW2>& m, const DCell<T>& c, T l0, T l1, const T (&ldp)[2], int a, T (&lph)[2], T& dmob) {
+  const int na = (c.act[0] ? 1 : 0) + (c.act[1] ? 1 : 0);
+  const T nact = (T)(na ? na : 1), mean = (l0 + l1) / nact;
+  const T kk = m.dt * mob_eff(m, c.ph) / m.eps;
+  T dp[2] = {c.act[0] ? kk * (l0 - mean) : (T)0, c.act[1] ? kk * (l1 - mean) : (T)0};
+  Proj pr;
+  T Dsum, sphi;
+  proj_fwd(c.ph, c.act, dp, pr, Dsum, sphi);
+  T ld[2] = {ldp[0], ldp[1]};
+  lph[0] = lph[1] = (T)0;
+  proj_rev(c.ph, c.act, pr, Dsum, sphi, ld, lph);
+  const T m0 = c.act[0] ? kk * ld[0] : (T)0, m1 = c.act[1] ? kk * ld[1] : (T)0;
+  dmob = (c.act[0] ? ld[0] * (l0 - mean) : (T)0) * kk / m.mob + (c.act[1] ? ld[1] * (l1 - mean) : (T)0) * kk / m.mob;
+  return (a ? m1 : m0) - (m0 + m1) / nact;
+}
+
+// What lane (a, k) adds for the adjoint la of phase a's lambda: v[w][n][t] to the six cells of its face, w = 0
+// its own phase, w = 1 the other; with the centre's terms, in lane k = 0 (and for the back neighbour k = 1).
+template <typename T>
+struct DAdj {
+  T v[2][2][3], lmu, ldab, lgam;
+};
+template <typename T, bool POW2>
+GP_HD void dphi_lane_rev(const AM<T, POW2>& m, const DLane<T>& L, const DTerm<T>& t, T mu, int a, int k, T sum4, T la,
+                         DAdj<T>& o) {
+  const int dir = k >> 1;
+  const T sg = (k & 1) ? (T)-1 : (T)1, lt = m.eps * la;
+  T lQx = (T)0, lQy = (T)0, lS = (T)0, lpa = (T)0, lpb = (T)0;
+  o.lmu = o.ldab = o.lgam = (T)0;
+  face_term_rev(m.R[a], m.Ri[a], m.dab, L.Qx, L.Qy, L.sb, dir, m.qd(dir, (T)2 * m.gam * sg) * lt, lQx, lQy, lS, o.ldab);
+  const T lQn = dir ? lQy : lQx, lQt = dir ? lQx : lQy;
+  const T lsa = lQn * L.gb + (T)0.5 * lQt * L.tb, lsb = -lQn * L.ga - (T)0.5 * lQt * L.ta + lS;
+  const T lga = -lQn * L.sb, lgb = lQn * L.sa, lta = -(T)0.5 * lQt * L.sb, ltb = (T)0.5 * lQt * L.sa;
+  // the centre's terms (lanes k = 0 and 1 use them)
+  const Aniso<T>& A = t.A;
+  const T ldA = -lt, G = (T)2 * m.gam * ldA;
+  const T lac = G * ((T)2 * A.ac * t.qr + t.q2 * t.dr);
+  const T lqr = G * A.ac * A.ac, lq2 = G * A.ac * t.dr, ldr = G * A.ac * t.q2;
+  const T ld0 = ldr * t.r0, ld1 = ldr * t.r1;
+  const T lr0 = lqr * t.q0 + ldr * A.d0, lr1 = lqr * t.q1 + ldr * A.d1;
+  const T c = (T)16 * m.dab;
+  const T lq0 = lqr * t.r0 + c * (ld0 * A.J[0][0] + ld1 * A.J[1][0]) + lac * A.d0 + (T)2 * t.q0 * lq2;
+  const T lq1 = lqr * t.r1 + c * (ld0 * A.J[0][1] + ld1 * A.J[1][1]) + lac * A.d1 + (T)2 * t.q1 * lq2;
+  T lcxb = (T)0, lcyb = (T)0, lv0 = (T)0, lv1 = (T)0;
+  mv_rev(m.R[a], lr0, lr1, lcxb, lcyb);
+  mv_rev(m.R[a], lq0, lq1, lv0, lv1);
+  lcxb += lv0 * L.pa;
+  lcyb += lv1 * L.pa;
+  const T lcxa = -lv0 * L.pb, lcya = -lv1 * L.pb;
+  if (k == 0) {
+    o.ldab += (T)16 * (ld0 * A.u0 + ld1 * A.u1) + lac * A.g;
+    o.lgam += (T)2 * sum4 * lt + (T)2 * (A.ac * A.ac * t.qr + A.ac * t.q2 * t.dr) * ldA;
+    lpa += lv0 * L.cxb + lv1 * L.cyb;
+    lpb += -lv0 * L.cxa - lv1 * L.cya;
+    const T lw = -m.inv_eps * la;
+    if (L.act_b) {
+      if (m.obstacle) {
+        const T sgn = (L.pa * L.pb >= (T)0) ? (T)1 : (T)-1;
+        lpb += m.wobs * sgn * m.gam * lw;
+        o.lgam += m.wobs * sgn * L.pb * lw;
+      } else {
+        lpb += (T)36 * m.gam * L.pb * L.pa * lw;
+        lpa += (T)18 * m.gam * L.pb * L.pb * lw;
+        o.lgam += (T)18 * L.pb * L.pb * L.pa * lw;
+      }
+    }
+    o.lmu = -dpsi_dmu(m, a, mu) * dhfun(L.pa) * la;
+    lpa -= t.psi * d2hfun(L.pa) * la;
+  }
+#pragma unroll
+  for (int w = 0; w < 2; w++) {
+    const T lg = m.qd(dir, w ? lgb : lga), ls = (T)0.5 * (w ? lsb : lsa), lT = w ? ltb : lta;
+    const T tv = dir == 0 ? m.qt(lT) : m.qx((T)0.5 * lT);
+    const T hx = m.qx((T)0.5 * (w ? lcxb : lcxa)), hy = m.qt(w ? lcyb : lcya);
+    o.v[w][0][0] = -tv;
+    o.v[w][0][1] = ls - lg;
+    o.v[w][0][2] = tv;
+    o.v[w][1][0] = -tv;
+    o.v[w][1][1] = ls + lg;
+    o.v[w][1][2] = tv;
+    if (k == 0) {  // rows x, x + 1: the centre and its x+, y-, y+ neighbours
+      o.v[w][0][1] += w ? lpb : lpa;
+      o.v[w][1][1] += hx;
+      o.v[w][0][0] -= hy;
+      o.v[w][0][2] += hy;
+    } else if (k == 1) {  // row x - 1
+      o.v[w][0][1] -= hx;
+    }
+  }
+}
+
 // reverse of dphi_fwd: ldp = adjoint of dp; accumulates LP, lmu, lpar
 template <typename T, bool POW2>
 GP_HD void dphi_rev(const AM<T, POW2>& m, const T (&P)[3][3][2], T mu, const T (&ldp)[2], T (&LP)[3][3][2], T& lmu,
                     T (&lpar)[NPARAM]) {
-  Grad<T> G;
-  grad_fwd(m, P, G);
-  const T ph[2] = {P[1][1][0], P[1][1][1]};
-  bool act[2];
-  T lam[2], sum = (T)0;
-  int cnt = 0;
+  DCell<T> c;
+  dphi_cell(m, P, c);
+  if (!c.act[0] && !c.act[1]) return;  // Delta-phi is 0 whatever the inputs
+  DLane<T> L[2][4];
+  DTerm<T> t[2];
+  T sum4[2], lph[2], dmob;
   for (int a = 0; a < 2; a++) {
-    const T dv = m.qx(G.gx[a] - G.bgx[a]) + m.qy(G.gy[a] - G.lgy[a]);
-    act[a] = fabs(dv) > (T)0;
+    T f[4];
+    for (int k = 0; k < 4; k++) {
+      dphi_lane(m, P, c, a, k, L[a][k]);
+      f[k] = dphi_face(m, L[a][k], a, k);
+    }
+    sum4[a] = (f[0] + f[1]) + (f[2] + f[3]);
+    dphi_term(m, c, L[a][0], mu, a, sum4[a], t[a]);
   }
   for (int a = 0; a < 2; a++) {
-    lam[a] = (T)0;
-    if (act[a]) {
-      lam[a] = m.eps * tterm(m, G, ph, a) - m.inv_eps * wfun(m, ph, act, a) - psi_of(m, a, mu) * dhfun(ph[a]);
-      sum += lam[a];
-      cnt++;
+    const T la = dphi_mean_rev(m, c, t[0].lam, t[1].lam, ldp, a, lph, dmob);
+    if (!c.act[a]) continue;
+    for (int k = 0; k < 4; k++) {
+      DAdj<T> o;
+      dphi_lane_rev(m, L[a][k], t[a], mu, a, k, sum4[a], la, o);
+      for (int w = 0; w < 2; w++)
+        for (int n = 0; n < 2; n++)
+          for (int i = 0; i < 3; i++) {
+            const int dn = n - (k & 1) + 1;
+            LP[k >> 1 ? i : dn][k >> 1 ? dn : i][w ? 1 - a : a] += o.v[w][n][i];
+          }
+      lmu += o.lmu;
+      lpar[P_DELTA] += o.ldab;
+      lpar[P_GAMMA] += o.lgam;
     }
   }
-  if (!cnt) return;  // Delta-phi is 0 whatever the inputs
-  sum /= (T)cnt;
-  const T me = mob_eff(m, ph);
-  const T k = m.dt * me / m.eps;
-  T dp[2];
-  for (int a = 0; a < 2; a++) dp[a] = act[a] ? k * (lam[a] - sum) : (T)0;
-  Proj r;
-  T Dsum, sphi;
-  proj_fwd(ph, act, dp, r, Dsum, sphi);
-  T ld[2] = {ldp[0], ldp[1]}, lph[2] = {(T)0, (T)0};
-  proj_rev(ph, act, r, Dsum, sphi, ld, lph);
-  // dp_a = k (lam_a - mean) on active phases
-  T llam[2] = {(T)0, (T)0}, lmean = (T)0;
-  for (int a = 0; a < 2; a++)
-    if (act[a]) {
-      llam[a] += k * ld[a];
-      lmean -= k * ld[a];
-      lpar[P_MOB] += ld[a] * (lam[a] - sum) * k / m.mob;  // d me / d mob = me / mob
-    }
-  Grad<T> LG = {};
-  for (int a = 0; a < 2; a++)
-    if (act[a]) {
-      const T la = llam[a] + lmean / (T)cnt;
-      // lam_a = eps t_a - w_a / eps - psi_a(mu) h'(phi_a)
-      tterm_rev(m, G, ph, a, m.eps * la, LG, lph, lpar[P_DELTA], lpar[P_GAMMA]);
-      const T lw = -m.inv_eps * la;
-      const int b = 1 - a;
-      if (act[b]) {
-        if (m.obstacle) {
-          const T sg = (ph[a] * ph[b] >= (T)0) ? (T)1 : (T)-1;
-          lph[b] += m.wobs * sg * m.gam * lw;
-          lpar[P_GAMMA] += m.wobs * sg * ph[b] * lw;
-        } else {
-          lph[b] += (T)36 * m.gam * ph[b] * ph[a] * lw;
-          lph[a] += (T)18 * m.gam * ph[b] * ph[b] * lw;
-          lpar[P_GAMMA] += (T)18 * ph[b] * ph[b] * ph[a] * lw;
-        }
-      }
-      lmu -= dpsi_dmu(m, a, mu) * dhfun(ph[a]) * la;
-      lph[a] -= psi_of(m, a, mu) * d2hfun(ph[a]) * la;
-    }
   LP[1][1][0] += lph[0];
   LP[1][1][1] += lph[1];
-  grad_rev(m, LG, LP);
+  lpar[P_MOB] += dmob;
 }
 
 // ------------------------------------------------------------------ faces of the mu update
