@@ -148,3 +148,48 @@ def test_slots_leave_memory_to_others_and_one_slot_gives_the_same():
         torch.cuda.empty_cache()
     for x, y in zip(*got):
         np.testing.assert_allclose(x, y, rtol=1e-4, atol=1e-4 * np.abs(x).max())
+
+
+SPACINGS = [(0.5, 2.0), (0.7, 1.3)]  # products with reciprocals, quotients
+
+
+@pytest.mark.parametrize("well", [0, 1])
+@pytest.mark.parametrize("size", [(9, 33), (33, 47)])
+@pytest.mark.parametrize("spacing", SPACINGS)
+def test_adjoint_at_other_spacings(spacing, size, well):
+    """FP64 against directional differences (as above), FP32 against FP64 for the obstacle potential: its fields and
+    adjoints are rounded at every one of five steps and reverses, a few times 6e-8 each, which the antitrapping
+    term's quotients grow tenfold (2e-6 seen); a wrong or swapped spacing is an error of its own size.  (In a well's
+    tails 1 - phi is below FP32's resolution of phi: which phases are active there is a matter of rounding at
+    any spacing, and random weights see it.)"""
+    m, phi, mu = _case(*size, (1, 1, 1, 1), well)
+    m.dx, m.dy = spacing
+    m.dt *= 0.4
+    with mb.Context(m, mb.GP_FP64) as c:
+        c.upload(phi, mu)
+        c.step(60)
+        phi, mu = c.download()
+        c.step(5)
+        want = c.download()
+    rng = np.random.default_rng(7)
+    wp, wu = rng.standard_normal(phi.shape), rng.standard_normal(mu.shape)
+    dphi = rng.standard_normal(phi.shape) * ((phi > 1e-3) & (phi < 1 - 1e-3))
+    dmu, dp, p = rng.standard_normal(mu.shape), np.array([0.3, 0.0, 0.2, 0.3]), adjoint.params_of(m)
+
+    def forward(h, precision=mb.GP_FP64, back=False):
+        with adjoint.Adjoint(adjoint.with_params(m, p + h * dp), precision) as a:
+            q, u = a.forward(phi + h * dphi, mu + h * dmu, 5)
+            return (a.backward(wp, wu, initial=True), q, u) if back else float((wp * q).sum() + (wu * u).sum())
+
+    (g, lphi, lmu), q, u = forward(0.0, back=True)
+    assert np.abs(q - want[0]).max() <= 1e-10 and np.abs(u - want[1]).max() <= 1e-10
+    an = float((lphi * dphi).sum() + (lmu * dmu).sum() + g @ dp)
+    fd = (forward(1e-6) - forward(-1e-6)) / 2e-6
+    scale = np.abs(lphi * dphi).sum() + np.abs(lmu * dmu).sum() + np.abs(g * dp).sum()
+    assert abs(an - fd) <= 1e-4 * scale, (an, fd, scale)
+    if well:
+        return
+    (g32, lphi32, lmu32), _, _ = forward(0.0, mb.GP_FP32, True)
+    for a, b in ((lphi32, lphi), (lmu32, lmu)):
+        assert np.linalg.norm(a - b) <= 2e-5 * np.linalg.norm(b)
+    assert np.abs(g32 - g).max() <= 2e-5 * np.abs(g).max()

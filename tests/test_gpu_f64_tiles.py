@@ -114,12 +114,15 @@ def test_tiles_equal_the_ring_array_path_on_wild_states(kind):
             _same(a, b, name)
 
 
+@pytest.mark.parametrize("spacing", [(1.0, 1.0), (0.5, 2.0), (4.0, 0.25), (0.7, 1.3)])  # the last: no tiles
 @pytest.mark.parametrize("size", [(33, 47), (64, 64)])
-def test_anisotropic_tiles_equal_the_oracle(size):
+def test_anisotropic_tiles_equal_the_oracle(size, spacing):
     mx, my = size
     c = configs.binary_case(mx, my, gap=1.0, supersat=0.5, eps=3.0, delta=0.04, theta=17.0, dt=0.05, tau=1.3332,
                             seed=(0, 0, 9.0))
     m, phi, mu = mb.load_case(c)
+    m.dx, m.dy = spacing
+    m.dt *= min(1.0, min(spacing) ** 2)
     om = O.OracleModel(
         N=m.N, K1=m.K1, mesh_x=mx, mesh_y=my, dx=m.dx, dy=m.dy, dt=m.dt, epsilon=m.epsilon, tau=m.tau, T=m.T, Teq=m.Teq,
         obstacle=m.obstacle, anisotropy=m.anisotropy, binary=1, ternary=0, dilute=0, bc_phi=tuple(m.bc_phi),
