@@ -359,14 +359,12 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, P
     // the diffusion fluxes: s = +1 where the cell is the face's lower one
     const T k0 = m.Ds * m.cmu[0], k1 = m.Dl * m.cmu[1];
     const T Dme = k0 * ph[0] + k1 * ph[1];
+    T sD = (T)0, sM = (T)0;  // summed apart: one rounding at the scale of the adjoint they are added to
     auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, int dir, bool to_phi, bool to_mu) {
       T lD, lg;
       flux_rev(m.qd(dir, mu_hi - mu_lo), Dsum, m.qd(dir, g_lo - g_hi), lD, lg);
-      if (to_phi) {
-        lph[0] += lD * k0;
-        lph[1] += lD * k1;
-      }
-      if (to_mu) lmu -= s * m.qd(dir, lg);
+      if (to_phi) sD += lD;
+      if (to_mu) sM -= s * m.qd(dir, lg);
       return lD;
     };
     const T gme = sg[i][j];
@@ -401,9 +399,9 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, P
       ghost(false, true);
       ghost(false, false);
     }
-    lam_out[o] = lph[0];
-    lam_out[g.plane + o] = lph[1];
-    lam_out[2 * g.plane + o] = lmu;
+    lam_out[o] = lph[0] + sD * k0;
+    lam_out[g.plane + o] = lph[1] + sD * k1;
+    lam_out[2 * g.plane + o] = lmu + sM;
   }
   block_add(dl, part + blockIdx.x);
 }
@@ -505,7 +503,7 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, 
   begin_dependent();
   constexpr unsigned ALL = 0xffffffffu;
   double acc[3] = {0.0, 0.0, 0.0};  // mobility, delta, gamma
-  const int lane = threadIdx.x & 31, sub = lane & 7, a = sub >> 2, k = sub & 3, dir = k >> 1;
+  const int lane = threadIdx.x & 31, sub = lane & 7, a = sub >> 2, k = sub & 3;
   const int n = *cnt, warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   for (ListWalk four(n, 1, 4 * warp, 4 * warps); four.more(); four.next()) {  // four cells a warp
     const int64_t q = four.at + (lane >> 3);
@@ -540,8 +538,9 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, 
       acc[0] += (double)dmob;
       add_nz(lam_out + ix_mu(g, x, y), lmu);
     }
-    // the partner lane (the other phase) holds the same cells' other half, exchanged so that a lane adds one
-    // phase's values; the projection's own adjoints go with the first lane's centre
+    // The partner lane (the other phase) holds the same cells' other half, exchanged so that a lane has one
+    // phase's values; the projection's own adjoints go with the first lane's centre.
+    T v[2][3];
 #pragma unroll
     for (int nn = 0; nn < 2; nn++)
 #pragma unroll
@@ -551,11 +550,37 @@ __global__ void __launch_bounds__(128) k_rev_dphi(const __grid_constant__ AM<T, 
           mine += lph[0];
           other += lph[1];
         }
-        const T v = mine + __shfl_xor_sync(ALL, other, 4);
-        if (!on) continue;
-        const int dn = nn - (k & 1), dt = i - 1;
-        add_nz(lam_out + ix_phi(g, dir ? x + dt : x + dn, dir ? y + dn : y + dt, a), v);
+        v[nn][i] = mine + __shfl_xor_sync(ALL, other, 4);
       }
+    // The four faces' sums, so that each of the nine cells takes one addition (24 before: each a rounding at
+    // the scale of the adjoint, and an atomic).  The x faces' lanes hold rows (k = 0: 1 and 2, k = 1: 0
+    // and 1), the y faces' columns; the middle row and column go to the even lanes, then each cell's row part
+    // meets its column part.
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const T middle = __shfl_xor_sync(ALL, v[1][i], 1);
+      if (!(k & 1)) v[0][i] += middle;
+    }
+    const T *const lo = v[0], *const up = v[1];
+    const T r0 = __shfl_xor_sync(ALL, k == 0 ? up[1] : k == 1 ? lo[0] : lo[1], 2);
+    const T r1 = __shfl_xor_sync(ALL, k == 0 ? up[2] : up[1], 2);
+    const T r2 = __shfl_xor_sync(ALL, k == 0 ? up[0] : k == 1 ? lo[2] : k == 2 ? lo[0] : lo[1], 3);
+    if (!on) continue;
+    auto add = [&](int dx, int dy, T w) { add_nz(lam_out + ix_phi(g, x + dx, y + dy, a), w); };
+    if (k == 0) {
+      add(0, 0, lo[1] + r0);
+      add(0, 1, lo[2] + r1);
+      add(0, -1, lo[0] + r2);
+    } else if (k == 1) {
+      add(-1, 0, lo[1] + r2);
+    } else if (k == 2) {
+      add(1, 0, lo[2] + r0);
+      add(1, 1, up[2] + r1);
+      add(-1, 1, up[0] + r2);
+    } else {
+      add(1, -1, lo[2] + r2);
+      add(-1, -1, lo[0] + r0);
+    }
   }
 #pragma unroll
   for (int p = 0; p < 3; p++) block_add(acc[p], part + 3 * blockIdx.x + p);
