@@ -1790,7 +1790,8 @@ static bool tile_model(const gp_model& m) {
   return true;
 }
 
-// *out stays nullptr for a model the tile kernel does not take.
+// *out stays nullptr for a model the tile kernel does not take.  The fills run on the legacy stream: the caller waits
+// for them before it uses another one.
 cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
   *out = nullptr;
   if (!tile_model(m)) return cudaSuccess;
@@ -1855,7 +1856,6 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
     e = cudaHostAlloc((void**)&t->seen, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
     if (e == cudaSuccess) *t->seen = 0;
   }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     gp_f64_tiles_destroy(t);
     return e;
