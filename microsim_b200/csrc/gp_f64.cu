@@ -25,6 +25,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <mutex>
 #include <vector>
 
 #include "gp_common.cuh"
@@ -1762,12 +1763,49 @@ struct gp_f64_tiles {
   int dense_from = INT32_MAX;  // more listed tiles than this: the ring-array kernels are faster
 };
 
+// Page-locked words that a kernel writes and the host reads without waiting, one per context that needs one.
+// Allocating page-locked memory takes 1 to 3 ms, longer than the rest of a small context, so the process keeps
+// one page of them from the first such context on; contexts beyond its 1,024 words do without (they stay on
+// the tile kernels).  The page is asked about before it is used again: a device reset takes it away.
+static std::mutex word_lock;
+static int* word_page = nullptr;
+static bool word_used[1024];
+
+static int* word_acquire() {
+  const std::lock_guard<std::mutex> lock(word_lock);
+  cudaPointerAttributes at;
+  if (!word_page || cudaPointerGetAttributes(&at, word_page) != cudaSuccess || at.type != cudaMemoryTypeHost) {
+    cudaGetLastError();
+    word_page = nullptr;
+    memset(word_used, 0, sizeof word_used);
+    if (cudaHostAlloc((void**)&word_page, sizeof word_used / sizeof word_used[0] * sizeof(int),
+                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      word_page = nullptr;
+      return nullptr;
+    }
+  }
+  for (size_t i = 0; i < sizeof word_used / sizeof word_used[0]; i++)
+    if (!word_used[i]) {
+      word_used[i] = true;
+      word_page[i] = 0;
+      return word_page + i;
+    }
+  return nullptr;
+}
+
+static void word_release(int* w) {
+  const std::lock_guard<std::mutex> lock(word_lock);
+  if (w && word_page && w >= word_page && w < word_page + sizeof word_used / sizeof word_used[0]) word_used[w - word_page] = false;
+}
+
+// The caller has waited for the kernels that use the tables.
 void gp_f64_tiles_destroy(gp_f64_tiles* t) {
   if (!t) return;
   cudaFree(t->geo);
   cudaFree(t->words);
   cudaFree(t->list);
-  if (t->seen) cudaFreeHost(t->seen);
+  word_release(t->seen);
   delete t;
 }
 
@@ -1852,10 +1890,7 @@ cudaError_t gp_f64_tiles_create(const gp_model& m, gp_f64_tiles** out) {
   if (e == cudaSuccess) e = cudaMemset(t->words, 0, 2 * sizeof(uint32_t) * n);
   if (e == cudaSuccess) e = cudaMalloc(&t->list, sizeof(int) * (n + 3));
   if (e == cudaSuccess) e = cudaMemset(t->list + n, 0, 3 * sizeof(int));
-  if (e == cudaSuccess && t->dense_from < t->n) {
-    e = cudaHostAlloc((void**)&t->seen, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-    if (e == cudaSuccess) *t->seen = 0;
-  }
+  if (e == cudaSuccess && t->dense_from < t->n) t->seen = word_acquire();
   if (e != cudaSuccess) {
     gp_f64_tiles_destroy(t);
     return e;

@@ -261,3 +261,37 @@ def test_dense_two_phase_states_are_not_slower_than_the_ring_array():
                 t.append(time.perf_counter() - t0)
             best.append(min(t))
     assert best[0] < 1.12 * best[1], best
+
+
+def test_creating_a_context_stays_cheap_and_many_of_them_keep_apart():
+    """A context takes about as long with the host's word for its tile count as without one (a grid that one round
+    of blocks covers has none); page-locked memory of its own took 1 to 3 ms more.  Contexts created and closed
+    in turn, more than the page has words, and dense and sparse ones alive together keep their own counts."""
+    import time
+    dense, phi, mu = _dense(300, 280)
+    sparse, sp, su = mb.load_case(_alloy("obstacle", 300, 280, (1, 1, 1, 1)))
+    small = mb.load_case(_alloy("obstacle", 128, 128, (1, 1, 1, 1)))[0]
+    best = []
+    for m in (small, mb.load_case(_alloy("obstacle", 128, 300, (1, 1, 1, 1)))[0]):
+        t = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            c = mb.Context(m, mb.GP_FP64)
+            t.append(time.perf_counter() - t0)
+            c.close()
+        best.append(sorted(t)[10])
+    assert best[1] < best[0] + 0.6e-3, best
+    for _ in range(1100):
+        mb.Context(dense, mb.GP_FP64).close()
+    a, b = _pair(dense)
+    c, d = _pair(sparse)
+    with a, b, c, d:
+        for x in (a, b):
+            x.upload(phi, mu)
+        for x in (c, d):
+            x.upload(sp, su)
+        for n in (9, 40, 17):
+            for x in (a, c, b, d):
+                x.step(n)
+            _same(a, b, n)
+            _same(c, d, n)
