@@ -197,7 +197,11 @@ int gp_download(gp_ctx *ctx, double *phi, double *mu);
  * or in gp_sync.  Runs of eight steps replay a CUDA graph captured from each of
  * the context's two buffers (the same kernels and arguments as direct launches, one
  * host launch for all of them): isothermal FP64 contexts from the first such run,
- * FP32 contexts once 64 steps were taken, or asked for in one call. */
+ * FP32 contexts in calls of 128 steps or more, or once 256 were taken.  A caller that
+ * is capturing gp_stream(ctx) itself records direct launches; it may replay its graph
+ * as often as it likes, and state changes in between are seen.
+ * A two-phase FP64 context goes through one of two pairs of kernels with the same
+ * results, by the share of its tiles that held an interface in recent steps. */
 int gp_step(gp_ctx *ctx, int64_t nsteps);
 /* The context's step count (the frozen temperature gradient's clock: step t uses the temperature
  * the reference sets after step t - 1).  Starts at 0 on creation; gp_step advances it. */
@@ -244,7 +248,8 @@ void *gp_stream(gp_ctx *ctx);
  * or shift): phi [N][mesh_x][pitch], mu [K1][mesh_x][pitch], plane = elements
  * per plane, esize = 8 (FP64) or 4 (FP32).  For callers that exchange rows
  * between contexts (halo rows of a grid split across GPUs); after writing into
- * them, call gp_state_changed. */
+ * them, call gp_state_changed (the next FP64 step then reads phi once more, the
+ * next FP32 step takes every tile through its full kernel). */
 int gp_state_device(gp_ctx *ctx, void **phi, void **mu, int64_t *pitch, int64_t *plane, int *esize);
 int gp_state_changed(gp_ctx *ctx);
 /* Number of kernel launches this context issued since creation. */
@@ -296,9 +301,10 @@ int gp_batch_get_stats(gp_batch *b, int i, gp_stats *out);
 int gp_batch_get_stats_async(gp_batch *b, int i, double *raw);
 int gp_batch_stats_from_raw(gp_batch *b, int i, const double *raw, gp_stats *out);
 /* Tile shape of the fused kernel (tx along x, ty along y): 16x32, 8x32, 32x32, 16x64.
- * Until it is set or tuned: 8x32 with the widest full-kernel blocks when the batch has
- * at most 1,184 tiles of that shape and four phases or fewer, else 16x32 with 256
- * threads.  The results do not depend on it. */
+ * Until it is set or tuned: 8x32 when the batch has four phases or fewer and at most
+ * 1,184 tiles of that shape (832 when an instance has the well potential), else 16x32;
+ * the full kernel with 512 threads per block for binary alloys with 8x32 tiles (the well
+ * potential: up to 296 of them), else 256.  The results do not depend on it. */
 int gp_batch_set_tile(gp_batch *b, int tx, int ty);
 /* Narrow band (on by default): tiles whose cells and two-cell ring were one
  * pure phase after the previous step (per-tile purity words written by every
@@ -417,7 +423,12 @@ const char *gp_last_error(void);
  *   grad[3]  liquid diffusivity Diff[1][0][0]
  * and, when lam_phi0 / lam_mu0 are not NULL, with respect to the initial state.
  * The segment of checkpoint_every steps is recomputed before it is reversed, so
- * ceil(nsteps / checkpoint_every) + checkpoint_every states are stored. */
+ * ceil(nsteps / checkpoint_every) + checkpoint_every states are stored
+ * (gp_adj_stored_states).  Beside each of a segment's states its Delta-phi and a list
+ * of its interface cells are kept, about as much memory again, where that leaves half
+ * of the device's free memory to others; else they are recomputed state by state.  The
+ * memory is kept for the object's next run and given back when that needs less than a
+ * quarter of it. */
 #define GP_ADJ_NPARAM 4
 typedef struct gp_adj gp_adj;
 int gp_adj_create(const gp_model *m, int precision, gp_adj **out);

@@ -14,10 +14,12 @@
 //               calculate_divergence_concentration.h:4-153), into the other
 //               buffer of a double-buffered state.
 // k_lean64 steps the tiles far from every interface, k_step64 the others, both half
-// steps of a tile in shared memory.  k_dphi and k_update do them one after the other through a ring array in device memory: the smoothing
-// pre-steps, the step after a moving-frame shift (explicit ghost rows), models with
-// spacings that are no powers of two or pair constants that are not symmetric, and the
-// allocation-free entry.
+// steps of a tile in shared memory; k_words64 makes their tile tables for a state that
+// no step wrote.  k_dphi and k_update do the half steps one after the other through a
+// ring array in device memory: the smoothing pre-steps, the step after a moving-frame
+// shift (explicit ghost rows), models with spacings that are no powers of two or pair
+// constants that are not symmetric, two-phase states most of whose tiles hold an
+// interface, and the allocation-free entry.
 // Ghost cells are read through gp_map (boundary copies as index maps).
 //
 // Reference paths are relative to Grand_potential_Finite_difference_2D_serial/.
