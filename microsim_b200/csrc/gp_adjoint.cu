@@ -360,23 +360,25 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, P
     const T k0 = m.Ds * m.cmu[0], k1 = m.Dl * m.cmu[1];
     const T Dme = k0 * ph[0] + k1 * ph[1];
     T sD = (T)0, sM = (T)0;  // summed apart: one rounding at the scale of the adjoint they are added to
-    auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, int dir, bool to_phi, bool to_mu) {
+    // p1: the two cells' phase 1, for the D_liquid gradient that is returned
+    auto gather = [&](T s, T g_lo, T g_hi, T mu_lo, T mu_hi, T Dsum, T p1, int dir, bool to_phi, bool to_mu) {
+      const T lF = m.qd(dir, g_lo - g_hi);
       T lD, lg;
-      flux_rev(m.qd(dir, mu_hi - mu_lo), Dsum, m.qd(dir, g_lo - g_hi), lD, lg);
+      flux_rev(m.qd(dir, mu_hi - mu_lo), Dsum, lF, lD, lg);
       if (to_phi) sD += lD;
       if (to_mu) sM -= s * m.qd(dir, lg);
-      return lD;
+      return lF != (T)0 ? (double)(lD * m.cmu[1] * p1) : 0.0;
     };
     const T gme = sg[i][j];
     auto nb = [&](int a, int ii, int jj) { return sp[a][ii][jj]; };
     auto Dnb = [&](int ii, int jj) { return k0 * nb(0, ii, jj) + k1 * nb(1, ii, jj); };
-    const T a0 = gather((T)1, gme, sg[i + 1][j], M[0], M[2], Dnb(i + 1, j) + Dme, 0, true, true);
-    const T a1 = gather((T)-1, sg[i - 1][j], gme, M[1], M[0], Dme + Dnb(i - 1, j), 0, true, true);
-    const T a2 = gather((T)1, gme, sg[i][j + 1], M[0], M[4], Dnb(i, j + 1) + Dme, 1, true, true);
-    const T a3 = gather((T)-1, sg[i][j - 1], gme, M[3], M[0], Dme + Dnb(i, j - 1), 1, true, true);
-    dl += (double)(a0 * m.cmu[1] * (ph[1] + nb(1, i + 1, j))) + (double)(a2 * m.cmu[1] * (ph[1] + nb(1, i, j + 1)));
-    if (x == 0) dl += (double)(a1 * m.cmu[1] * (nb(1, i - 1, j) + ph[1]));
-    if (y == 0) dl += (double)(a3 * m.cmu[1] * (nb(1, i, j - 1) + ph[1]));
+    const double a0 = gather((T)1, gme, sg[i + 1][j], M[0], M[2], Dnb(i + 1, j) + Dme, ph[1] + nb(1, i + 1, j), 0, true, true);
+    const double a1 = gather((T)-1, sg[i - 1][j], gme, M[1], M[0], Dme + Dnb(i - 1, j), nb(1, i - 1, j) + ph[1], 0, true, true);
+    const double a2 = gather((T)1, gme, sg[i][j + 1], M[0], M[4], Dnb(i, j + 1) + Dme, ph[1] + nb(1, i, j + 1), 1, true, true);
+    const double a3 = gather((T)-1, sg[i][j - 1], gme, M[3], M[0], Dme + Dnb(i, j - 1), nb(1, i, j - 1) + ph[1], 1, true, true);
+    dl += a0 + a2;  // each face by its lower cell; the grid's first ones by their upper
+    if (x == 0) dl += a1;
+    if (y == 0) dl += a3;
     // the ghost cell (ghost row -1 or M, against the grid's first or last row `e`) that maps to this one
     auto ghost = [&](bool along_x, bool low) {
       const int Mg = along_x ? g.mx : g.my, v = low ? -1 : Mg, e = low ? 0 : Mg - 1, own = along_x ? x : y;
@@ -388,8 +390,8 @@ __global__ void __launch_bounds__(NT) k_rev_cell(const __grid_constant__ AM<T, P
       const T ge = cell_ldc(m, e0, e1, lmu_in[(int64_t)ex * g.pitch + ey]) * m.dt;
       const T ue = st[2 * g.plane + (int64_t)ex * g.pitch + ey], uv = ld_mu(st, g, vx, vy);
       const T Ds2 = (k0 * v0 + k1 * v1) + (k0 * e0 + k1 * e1);
-      if (low) gather((T)1, (T)0, ge, uv, ue, Ds2, along_x ? 0 : 1, mp == own, mm == own);
-      else gather((T)-1, ge, (T)0, ue, uv, Ds2, along_x ? 0 : 1, mp == own, mm == own);
+      if (low) gather((T)1, (T)0, ge, uv, ue, Ds2, (T)0, along_x ? 0 : 1, mp == own, mm == own);
+      else gather((T)-1, ge, (T)0, ue, uv, Ds2, (T)0, along_x ? 0 : 1, mp == own, mm == own);
     };
     if (x <= 2 || x >= g.mx - 3) {
       ghost(true, true);

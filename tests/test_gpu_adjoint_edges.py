@@ -216,3 +216,23 @@ def test_fp32_adjoint_sums_are_rounded_at_their_own_scale(spacing):
             a.forward(phi, mu, 5)
             lmu.append(a.backward(wp, wu, initial=True)[2])
     assert np.linalg.norm(lmu[1] - lmu[0]) <= 7.7e-8 * np.linalg.norm(lmu[0])
+
+
+@pytest.mark.parametrize("precision", [mb.GP_FP64, mb.GP_FP32])
+def test_a_face_without_adjoint_leaves_the_diffusivity_gradient_finite(precision):
+    """phi of the liquid is infinite in one bulk cell that the loss does not see.  That cell's own update makes the
+    other gradients NaN (0 times its mobility's terms, whichever kernels run); its faces have a zero adjoint."""
+    m, phi, mu = _case(48, 90, (1, 1, 1, 1), 0)
+    with mb.Context(m, mb.GP_FP64) as c:
+        c.upload(phi, mu)
+        c.step(60)
+        phi, mu = c.download()
+    w = np.random.default_rng(3).standard_normal(phi.shape) * ((phi > 0) & (phi < 1))
+    spoilt = phi.copy()
+    spoilt[1, 42, 80] = np.inf
+    got = []
+    for p in (phi, spoilt):
+        with adjoint.Adjoint(m, precision) as a:
+            a.forward(p, mu, 1)
+            got.append(a.backward(w)[3])
+    np.testing.assert_allclose(got[1], got[0], rtol=1e-9 if precision == mb.GP_FP64 else 1e-4)
