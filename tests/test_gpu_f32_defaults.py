@@ -1,6 +1,6 @@
 """What an FP32 context and a batch choose by themselves against a batch told to use 16x32 tiles, 256
-threads and (by odd step counts) direct launches: bit for bit, on grids either side of the line where
-the small tiles give way (1,184 tiles of 8x32), isothermal and in a frozen gradient, across a switch of
+threads and (by odd step counts) direct launches: bit for bit, on grids either side of the lines where
+the small tiles give way (1,184 tiles of 8x32, 832 with a well) and the wide blocks do (a well, 296), isothermal and in a frozen gradient, across a switch of
 the accumulation mode (which drops the captured steps) and runs split so that both replayed and direct
 steps occur."""
 import numpy as np
@@ -11,7 +11,8 @@ from microsim_b200 import configs
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(4, 4), (8, 32), (9, 33), (70, 90), (592, 512), (600, 512)]  # the last two: 1,184 and 1,200 tiles
+SIZES = [(4, 4), (8, 32), (9, 33), (70, 90), (592, 512), (600, 512),  # the last two: 1,184 and 1,200 tiles
+         (296, 256), (304, 256), (416, 512), (424, 512)]              # 296, 304, 832 and 848
 
 
 def _case(kind, mx, my):
@@ -38,7 +39,7 @@ def test_defaults_equal_large_tiles_and_direct_steps(size, kind):
         c.upload(phi, mu)
         d.upload(0, phi, mu)
         b.upload(0, phi, mu)
-        for n, comp in ((3, False), (64, False), (21, True), (75, True), (9, False)):
+        for n, comp in ((3, False), (64, False), (21, True), (75, True), (9, False), (135, True), (40, False), (17, False)):
             c.set_compensated(comp)
             d.set_compensated(comp)
             b.set_compensated(comp)
@@ -82,7 +83,7 @@ def test_the_default_shape_does_not_lose_on_well_grains(size):
                 b.sync()
                 t.append(time.perf_counter() - t0)
             best.append(min(t))
-    assert best[0] < 1.08 * best[1], best
+    assert best[0] < 1.12 * best[1], best
 
 
 @pytest.mark.parametrize("n", [64, 100])

